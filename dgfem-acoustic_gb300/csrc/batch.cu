@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "bb.cuh"
 #include "ctx.h"
 #include "dg_internal.cuh"
 
@@ -45,6 +46,7 @@ struct dg_batch {
     std::vector<int> inst;            // member instances in order
     std::vector<double> state;        // reference-layout staging [4][E*np]
     bool state_dirty = false, state_valid = false;
+    int own_variant = -2;             // kernel selected before one launch per stage took its layout (-2: none)
     cudaEvent_t join = nullptr;
   };
   std::vector<Group> groups;
@@ -226,6 +228,24 @@ int build_graph(dg_batch* b, int64_t n_steps) {
   return DG_OK;
 }
 
+// One launch per stage works on Bernstein coefficients: a group whose kernel
+// was forced to another layout (DGFEM_STAGE_VARIANT) takes them with it and
+// its own kernel back without it.
+int group_layouts(dg_batch* b) {
+  for (auto& g : b->groups) {
+    int rc = DG_OK;
+    if (b->fused && !g.ctx->bb) {
+      g.own_variant = g.ctx->variant;
+      rc = dg_tune(g.ctx, dgk::kBBVariant);
+    } else if (!b->fused && g.own_variant != -2) {
+      rc = dg_tune(g.ctx, g.own_variant);
+      g.own_variant = -2;
+    }
+    if (rc) return fail(b, rc, dg_last_error(g.ctx));
+  }
+  return DG_OK;
+}
+
 int launch_steps(dg_batch* b, int64_t n_steps, cudaEvent_t* ev) {
   for (auto& g : b->groups) {
     int64_t st[2] = {b->step, b->step};
@@ -335,7 +355,7 @@ int dg_batch_create(int n, const dg_mesh_desc* meshes, const dg_phys* phys, cons
   b->fused_ok = precision == DG_FP32;
   for (size_t k = 0; k < b->groups.size(); ++k) {
     const auto& g = b->groups[k];
-    if (g.dim != 2 || g.order < 2 || g.order > 4 || g.ctx->ncurved > 0)
+    if (g.dim != 2 || g.order < 2 || g.order > 4 || !dgc::bb_mesh(g.ctx))
       b->fused_ok = false;
     else
       b->slot_group[g.order - 2] = (int)k;
@@ -360,6 +380,7 @@ int dg_batch_create(int n, const dg_mesh_desc* meshes, const dg_phys* phys, cons
   // selects one kernel per order
   const char* ev = std::getenv("DGFEM_BATCH_FUSED");
   b->fused = b->fused_ok && !(ev && std::strcmp(ev, "0") == 0);
+  if (group_layouts(b) != DG_OK) return bail(DG_ERR_CUDA, b->err);
   *out = b;
   return DG_OK;
 }
@@ -385,6 +406,7 @@ int dg_batch_set_fused(dg_batch* b, int on) {
   if (b->fused != (on != 0)) {
     b->fused = on != 0;
     if (b->graph) cudaGraphExecDestroy(b->graph), b->graph = nullptr;
+    return group_layouts(b);
   }
   return DG_OK;
 }

@@ -1,0 +1,277 @@
+// Bernstein basis: tables, conversions, source injection, element means
+// (bb.cuh). The nodal values at the element's lattice are V c, the
+// coefficients V^-1 u; both matrices are sparse (a vertex, edge or face of
+// the lattice depends on its own points only), so a conversion is one sparse
+// row per coefficient: 3-D p = 4 has 309 entries of 1225.
+#include <cmath>
+#include <vector>
+
+#include "bb.cuh"
+#include "stage_bb.cuh"
+
+namespace {
+
+constexpr int LW = 32;
+
+// Word strides of a tile's variables, coefficients and elements (BBCfg).
+struct Lay {
+  int sq, sn, se, tw;
+};
+Lay lay(const dg_ctx* c) {
+  const int tw = c->nv * c->np * LW;
+  return c->prec == DG_FP32 && c->dim == 3 ? Lay{1, 4 * LW, 4, tw} : Lay{c->np * LW, LW, 1, tw};
+}
+
+// Reference layout -> tiles. One block per (tile, variable): the tile's
+// nodal values through shared memory (the reference layout is
+// element-major), one warp per coefficient row.
+template <typename T>
+__global__ void __launch_bounds__(128) k_ref_to_bb(const double* __restrict__ ref, T* __restrict__ out,
+                                                   const int* __restrict__ perm, const int* __restrict__ ptr,
+                                                   const int* __restrict__ col, const double* __restrict__ val,
+                                                   int64_t E, int np, Lay l) {
+  __shared__ double x[35 * (LW + 1)];
+  const int64_t tile = blockIdx.x, e0 = tile * LW;
+  const int q = blockIdx.y, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < np * LW; i += blockDim.x) {
+    const int e = i / np, n = i - e * np;
+    x[perm[n] * (LW + 1) + e] = e0 + e < E ? ref[q * E * np + (e0 + e) * np + n] : 0.0;
+  }
+  __syncthreads();
+  T* o = out + tile * l.tw + q * l.sq + lane * l.se;
+  for (int r = threadIdx.x >> 5; r < np; r += blockDim.x >> 5) {
+    double s = 0.0;
+#pragma unroll 4
+    for (int k = ptr[r]; k < ptr[r + 1]; ++k) s += val[k] * x[col[k] * (LW + 1) + lane];
+    o[r * l.sn] = (T)s;
+  }
+}
+
+// Tiles -> reference layout (variables the state does not carry: zero).
+template <typename T>
+__global__ void __launch_bounds__(128) k_bb_to_ref(const T* __restrict__ in, double* __restrict__ ref,
+                                                   const int* __restrict__ perm, const int* __restrict__ ptr,
+                                                   const int* __restrict__ col, const double* __restrict__ val,
+                                                   int64_t E, int np, int nv, Lay l) {
+  __shared__ double x[35 * LW], y[35 * (LW + 1)];
+  const int64_t tile = blockIdx.x, e0 = tile * LW;
+  const int q = blockIdx.y, lane = threadIdx.x & 31;
+  if (q < nv) {
+    const T* p = in + tile * l.tw + q * l.sq;
+    for (int i = threadIdx.x; i < np * LW; i += blockDim.x) x[i] = (double)p[(i / LW) * l.sn + (i % LW) * l.se];
+    __syncthreads();
+    for (int r = threadIdx.x >> 5; r < np; r += blockDim.x >> 5) {
+      double s = 0.0;
+#pragma unroll 4
+      for (int k = ptr[r]; k < ptr[r + 1]; ++k) s += val[k] * x[col[k] * LW + lane];
+      y[r * (LW + 1) + lane] = s;
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < np * LW; i += blockDim.x) {
+    const int e = i / np, n = i - e * np;
+    if (e0 + e < E) ref[q * E * np + (e0 + e) * np + n] = q < nv ? y[perm[n] * (LW + 1) + e] : 0.0;
+  }
+}
+
+// Source overwrite (src/solver.cpp:455-483) of elements given by
+// coefficients: one warp per element that holds source nodes. With S the
+// nodes that an active source covers and v their values, the element's
+// pressure becomes c + V^-1[:, S] (v - V[S, :] c): its nodal values are v at
+// S and unchanged elsewhere.
+template <typename T>
+__global__ void __launch_bounds__(128) k_inject_bb(T* u, const int64_t* __restrict__ elem,
+                                                   const int* __restrict__ eoff, int64_t ne,
+                                                   const int64_t* __restrict__ dof, const int* __restrict__ off,
+                                                   const int* __restrict__ ids, const double* __restrict__ val,
+                                                   int nsrc, int64_t nrows, const int64_t* step, int np, Lay l,
+                                                   const double* __restrict__ Vt, const double* __restrict__ Vit) {
+  __shared__ T sc[4][64], sr[4][64];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t i = blockIdx.x * 4ll + w;
+  if (i >= ne) return;
+  const int64_t s = step[0];
+  if (s < 0 || s >= nrows) return;
+  const double* row = val + s * nsrc;
+  const int64_t e = elem[i];
+  T* c = u + (e >> 5) * l.tw + (e & 31) * l.se;
+  for (int n = lane; n < np; n += 32) sc[w][n] = c[n * l.sn], sr[w][n] = (T)0;
+  __syncwarp();
+  for (int k = eoff[i] + lane; k < eoff[i + 1]; k += 32) {
+    double v = 0.0;
+    bool any = false;
+    for (int t = off[k]; t < off[k + 1]; ++t) {
+      const double x = row[ids[t]];
+      if (!isnan(x)) v = x, any = true;
+    }
+    if (any) {
+      const int n = (int)(dof[k] - e * np);
+      T r0 = (T)v, r1 = (T)0;
+#pragma unroll 4
+      for (int j = 0; j < np; ++j) {
+        const T p = (T)Vt[j * np + n] * sc[w][j];
+        if (j & 1)
+          r1 -= p;
+        else
+          r0 -= p;
+      }
+      sr[w][n] = r0 + r1;
+    }
+  }
+  __syncwarp();
+  for (int n = lane; n < np; n += 32) {
+    T a0 = (T)0, a1 = (T)0;
+#pragma unroll 4
+    for (int j = 0; j < np; ++j) {
+      const T p = (T)Vit[j * np + n] * sr[w][j];
+      if (j & 1)
+        a1 += p;
+      else
+        a0 += p;
+    }
+    c[n * l.sn] = sc[w][n] + (a0 + a1);
+  }
+}
+
+// Element means of p, p/c0^2 and v (src/Mesh.cpp:1196-1212) from the
+// coefficients: w holds the mean of each basis function over the nodes.
+template <typename T>
+__global__ void k_cell_means_bb(const T* __restrict__ u, const double* __restrict__ w, int64_t E, int np, int nv,
+                                double c0sq, double* __restrict__ out, int soa, Lay l) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= E) return;
+  const T* c = u + (e >> 5) * l.tw + (e & 31) * l.se;
+  double m[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int q = 0; q < nv; ++q) {
+    double s = 0.0;
+    for (int n = 0; n < np; ++n) s += w[n] * (double)c[q * l.sq + n * l.sn];
+    m[q] = s;
+  }
+  if (soa) {
+    out[e] = m[0], out[E + e] = m[0] / c0sq;
+    for (int d = 0; d < 3; ++d) out[2 * E + 3 * e + d] = m[1 + d];
+  } else {
+    out[e * 5] = m[0], out[e * 5 + 1] = m[0] / c0sq;
+    for (int d = 0; d < 3; ++d) out[e * 5 + 2 + d] = m[1 + d];
+  }
+}
+
+}  // namespace
+
+namespace dgc {
+
+int64_t bb_slot(const dg_ctx* c, int64_t e, int n) {
+  const Lay l = lay(c);
+  return (e >> 5) * l.tw + n * l.sn + (e & 31) * l.se;
+}
+
+int64_t bb_var_stride(const dg_ctx* c) { return lay(c).sq; }
+
+int bb_setup_basis(dg_ctx* c) {
+  const int np = c->np, D = c->dim, P = c->order;
+  std::vector<double>& V = c->bb_V;
+  std::vector<double>& Vi = c->bb_Vinv;
+  V.assign((size_t)np * np, 0.0), Vi.assign((size_t)np * np, 0.0);
+  std::vector<long double> A((size_t)np * 2 * np, 0.0L);
+  for (int i = 0; i < np; ++i) {
+    for (int j = 0; j < np; ++j) V[i * np + j] = dgk::bb_value(D, P, i, j), A[(size_t)i * 2 * np + j] = V[i * np + j];
+    A[(size_t)i * 2 * np + np + i] = 1.0L;
+  }
+  // Gauss-Jordan elimination with partial pivoting
+  for (int k = 0; k < np; ++k) {
+    int piv = k;
+    for (int i = k + 1; i < np; ++i)
+      if (std::fabs((double)A[(size_t)i * 2 * np + k]) > std::fabs((double)A[(size_t)piv * 2 * np + k])) piv = i;
+    for (int j = 0; j < 2 * np; ++j) std::swap(A[(size_t)k * 2 * np + j], A[(size_t)piv * 2 * np + j]);
+    const long double d = A[(size_t)k * 2 * np + k];
+    for (int j = 0; j < 2 * np; ++j) A[(size_t)k * 2 * np + j] /= d;
+    for (int i = 0; i < np; ++i) {
+      const long double f = A[(size_t)i * 2 * np + k];
+      if (i == k || f == 0.0L) continue;
+      for (int j = 0; j < 2 * np; ++j) A[(size_t)i * 2 * np + j] -= f * A[(size_t)k * 2 * np + j];
+    }
+  }
+  // the inverse has V's sparsity: what elimination leaves elsewhere is rounding
+  for (int i = 0; i < np; ++i)
+    for (int j = 0; j < np; ++j) Vi[i * np + j] = V[i * np + j] != 0.0 ? (double)A[(size_t)i * 2 * np + np + j] : 0.0;
+  // device: [0] V, [1] V^-1 as rows, the transposes dense, the means
+  std::vector<int> idx;
+  std::vector<double> val;
+  for (int m = 0; m < 2; ++m) {
+    const std::vector<double>& M = m ? Vi : V;
+    std::vector<int> ptr(1, 0), col;
+    std::vector<double> v;
+    for (int i = 0; i < np; ++i) {
+      for (int j = 0; j < np; ++j)
+        if (M[i * np + j] != 0.0) col.push_back(j), v.push_back(M[i * np + j]);
+      ptr.push_back((int)col.size());
+    }
+    c->bb_iptr[m] = (int)idx.size(), idx.insert(idx.end(), ptr.begin(), ptr.end());
+    c->bb_icol[m] = (int)idx.size(), idx.insert(idx.end(), col.begin(), col.end());
+    c->bb_ival[m] = (int)val.size(), val.insert(val.end(), v.begin(), v.end());
+    c->bb_iden[m] = (int)val.size();
+    for (int j = 0; j < np; ++j)
+      for (int i = 0; i < np; ++i) val.push_back(M[i * np + j]);
+  }
+  c->bb_imean = (int)val.size();
+  for (int j = 0; j < np; ++j) {
+    double s = 0.0;
+    for (int i = 0; i < np; ++i) s += V[i * np + j];
+    val.push_back(s / np);
+  }
+  cudaError_t e = dev_alloc(c, (void**)&c->bb_int, idx.size() * sizeof(int));
+  if (e == cudaSuccess) e = dev_alloc(c, (void**)&c->bb_dbl, val.size() * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemcpyAsync(c->bb_int, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(c->bb_dbl, val.data(), val.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  return e == cudaSuccess ? DG_OK : DG_ERR_CUDA;
+}
+
+cudaError_t bb_from_ref(dg_ctx* c, const double* ref, void* out) {
+  const dim3 grid((unsigned)(c->Epad / LW), c->nv);
+  const int *p = c->bb_int + c->bb_iptr[1], *k = c->bb_int + c->bb_icol[1];
+  const double* v = c->bb_dbl + c->bb_ival[1];
+  if (c->prec == DG_FP32)
+    k_ref_to_bb<float><<<grid, 128, 0, c->stream>>>(ref, (float*)out, c->d_perm, p, k, v, c->E, c->np, lay(c));
+  else
+    k_ref_to_bb<double><<<grid, 128, 0, c->stream>>>(ref, (double*)out, c->d_perm, p, k, v, c->E, c->np, lay(c));
+  return cudaGetLastError();
+}
+
+cudaError_t bb_to_ref(dg_ctx* c, const void* in, double* ref) {
+  const dim3 grid((unsigned)((c->E + LW - 1) / LW), 4);
+  const int *p = c->bb_int + c->bb_iptr[0], *k = c->bb_int + c->bb_icol[0];
+  const double* v = c->bb_dbl + c->bb_ival[0];
+  if (c->prec == DG_FP32)
+    k_bb_to_ref<float><<<grid, 128, 0, c->stream>>>((const float*)in, ref, c->d_perm, p, k, v, c->E, c->np, c->nv, lay(c));
+  else
+    k_bb_to_ref<double><<<grid, 128, 0, c->stream>>>((const double*)in, ref, c->d_perm, p, k, v, c->E, c->np, c->nv, lay(c));
+  return cudaGetLastError();
+}
+
+cudaError_t bb_inject(dg_ctx* c) {
+  if (c->n_src_elems == 0) return cudaSuccess;
+  const unsigned nb = (unsigned)((c->n_src_elems + 3) / 4);
+  const double *vt = c->bb_dbl + c->bb_iden[0], *vit = c->bb_dbl + c->bb_iden[1];
+  if (c->prec == DG_FP32)
+    k_inject_bb<float><<<nb, 128, 0, c->stream>>>((float*)c->u, c->d_src_elem, c->d_src_eoff, c->n_src_elems,
+                                                  c->d_src_dof, c->d_src_off, c->d_src_ids, c->d_srcval, c->n_src,
+                                                  c->srcval_steps, c->d_step, c->np, lay(c), vt, vit);
+  else
+    k_inject_bb<double><<<nb, 128, 0, c->stream>>>((double*)c->u, c->d_src_elem, c->d_src_eoff, c->n_src_elems,
+                                                   c->d_src_dof, c->d_src_off, c->d_src_ids, c->d_srcval, c->n_src,
+                                                   c->srcval_steps, c->d_step, c->np, lay(c), vt, vit);
+  return cudaGetLastError();
+}
+
+cudaError_t bb_cell_means(dg_ctx* c, double* out, bool soa) {
+  const unsigned nb = (unsigned)((c->E + 127) / 128);
+  const double* w = c->bb_dbl + c->bb_imean;
+  if (c->prec == DG_FP32)
+    k_cell_means_bb<float><<<nb, 128, 0, c->stream>>>((const float*)c->u, w, c->E, c->np, c->nv, c->c0sq, out, soa, lay(c));
+  else
+    k_cell_means_bb<double><<<nb, 128, 0, c->stream>>>((const double*)c->u, w, c->E, c->np, c->nv, c->c0sq, out, soa, lay(c));
+  return cudaGetLastError();
+}
+
+}  // namespace dgc

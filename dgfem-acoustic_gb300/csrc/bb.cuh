@@ -1,0 +1,24 @@
+// Host side of the Bernstein-basis kernels (stage_bb.cuh): basis tables,
+// conversions between the reference layout (nodal values) and the tiles of
+// Bernstein coefficients, source injection and element means.
+#pragma once
+#include "ctx.h"
+
+namespace dgc {
+// Whether the Bernstein-basis kernels take this context's mesh (straight-sided
+// triangles or tetrahedra).
+inline bool bb_mesh(const dg_ctx* c) { return c->dim >= 2 && c->ncurved == 0; }
+// Index of coefficient n of element e's first variable in a state array, and
+// the distance of the next variable's.
+int64_t bb_slot(const dg_ctx* c, int64_t e, int n);
+int64_t bb_var_stride(const dg_ctx* c);
+// Basis tables (c->bb_V, bb_Vinv and their device copies).
+int bb_setup_basis(dg_ctx* c);
+// reference layout [4][E*np] (c->d_ref or another device array) -> tiles, every lane of the padding cleared; and back
+cudaError_t bb_from_ref(dg_ctx* c, const double* ref, void* out);
+cudaError_t bb_to_ref(dg_ctx* c, const void* in, double* ref);
+// Hard overwrite of the pressure at source nodes, for elements' coefficients.
+cudaError_t bb_inject(dg_ctx* c);
+// Element means into out: AoS [E][5] (p, rho, v) or SoA (p [E], rho [E], v [E][3]).
+cudaError_t bb_cell_means(dg_ctx* c, double* out, bool soa);
+}  // namespace dgc

@@ -90,6 +90,24 @@ struct dg_ctx {
   void* cqD = nullptr;       // [dim][ng][np]
   void* cfB = nullptr;       // [nf][ngf][nfp]
   void* crhs = nullptr;      // [nv][ncurved][np]
+  // Bernstein basis (bb.cuh): bb is the layout that u and snap are in (tiles
+  // of coefficients, or nodal planes); the geometry of stage_bb.cuh; the
+  // basis tables ([0] V, [1] its inverse) on the host and the device
+  bool bb = false;
+  void* bbF = nullptr;
+  int* bbI = nullptr;
+  void* bbM = nullptr;
+  std::vector<double> bb_V, bb_Vinv;  // [np][np], V[i][j] = B_j(node i)
+  int* bb_int = nullptr;
+  double* bb_dbl = nullptr;
+  int bb_iptr[2] = {0, 0}, bb_icol[2] = {0, 0}, bb_ival[2] = {0, 0}, bb_iden[2] = {0, 0}, bb_imean = 0;
+  // elements holding source nodes, with their ranges of d_src_dof
+  int64_t n_src_elems = 0;
+  int64_t* d_src_elem = nullptr;
+  int* d_src_eoff = nullptr;
+  // observers as given (internal node slots): the device lists depend on bb
+  std::vector<int64_t> obs_off, obs_dof;
+  std::vector<double> obs_w;
   // per-step graph
   cudaGraphExec_t graph = nullptr;
   double graph_dt = 0.0;

@@ -134,6 +134,12 @@ struct StageArgs {
   const T* geoF;
   const int* geoI;
   const T* bmat;
+  // Bernstein-basis kernels (stage_bb.cuh): element geometry [tile][GW][32],
+  // neighbours and face codes [tile][2 NF][32], boundary matrices
+  // sJ (A_n - B) [n_bfaces][NV*NV]
+  const T* bbF;
+  const int* bbI;
+  const T* bbM;
   const T* Dt;     // [D][NP(j)][NP(i)]
   const T* LIFT;   // [NF*NFP(k)][NP(i)]
   const short* fmask;   // [NF*NFP]
@@ -247,6 +253,18 @@ inline bool is_wide_variant(int v) { return v >= kWideVariant && v < kWideVarian
 cudaError_t launch_stage4(int dim, int order, int variant, const StageArgs<float>& a, int grid, int* err,
                           cudaStream_t s);
 Stage2Info stage4_info(int dim, int order, int variant);
+// Bernstein-basis stage kernel (stage_bb.cuh): variant ids kBBVariant + k;
+// the state is in tiles of 32 elements' coefficients.
+constexpr int kBBVariant = 64;
+inline bool is_bb_variant(int v) { return v >= kBBVariant && v < kBBVariant + 16; }
+cudaError_t launch_stage_bb(int dim, int order, int variant, const StageArgs<float>& a, int grid, int* err,
+                            cudaStream_t s);
+cudaError_t launch_stage_bb(int dim, int order, int variant, const StageArgs<double>& a, int grid, int* err,
+                            cudaStream_t s);
+Stage2Info stage_bb_info_f32(int dim, int order, int variant);
+Stage2Info stage_bb_info_f64(int dim, int order, int variant);
+// geometry words of one element (floating-point) in the kernel's record
+inline int bb_geo_words(int dim) { return (dim + 1) * (dim + 1) + dim + dim * dim + 1; }
 // Mixed-order stage kernel of the batched ensemble (stage_multi.cuh): 2-D,
 // FP32, orders 2-4, one launch per RK stage over every order's tiles.
 // Per-launch description: one StageArgs per order slot (slot k holds order

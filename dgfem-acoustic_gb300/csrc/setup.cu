@@ -23,6 +23,7 @@
 #include <cstring>
 #include <stdexcept>
 
+#include "bb.cuh"
 #include "ctx.h"
 #include "curved.cuh"
 
@@ -379,6 +380,55 @@ __global__ void k_penalty_hist(const int* geoI, int reci, int nf, int64_t E, uns
   atomicAdd(&hist[(code & dgk::kCodeNegPenalty) ? 0 : 1], 1ull);
 }
 
+// Geometry records of the Bernstein-basis kernels (stage_bb.cuh), tiles of 32
+// elements: per face N = sJ n / 2 and A = sJ (v0.n - s c0) / 2 (the factors
+// of its jump flux), then G v0, G and the time-step scale; per face the
+// neighbour and code; per boundary face sJ (A_n - B). One thread per element
+// face of the padded mesh (padding elements: zero records).
+template <typename T>
+__global__ void k_bb_geo(const double* geo64, int recf, const int* geoI, int reci, const double* bm64, int D,
+                         int64_t E, int64_t Epad, double rho0, double c0, int gw, T* outF, int* outI, T* outM) {
+  const int nf = D + 1, NV = D + 1;
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= Epad * nf) return;
+  const int64_t e = i / nf;
+  const int f = (int)(i - e * nf);
+  T* rf = outF + (e >> 5) * gw * 32 + (e & 31);
+  int* ri = outI + (e >> 5) * 2 * nf * 32 + (e & 31);
+  const double* g = geo64 + e * recf;
+  const double* gf = g + D * D + f * (D + 1);
+  const double* v0 = g + D * D + nf * (D + 1);
+  const int nbr = geoI[e * reci + f], code = geoI[e * reci + nf + f];
+  ri[f * 32] = nbr, ri[(nf + f) * 32] = code;
+  const double sJ = gf[D];
+  double vn = 0.0;
+  for (int d = 0; d < D; ++d) vn += v0[d] * gf[d];
+  for (int d = 0; d < D; ++d) rf[(f * (D + 1) + d) * 32] = (T)(0.5 * sJ * gf[d]);
+  rf[(f * (D + 1) + D) * 32] = (T)(0.5 * sJ * (vn - ((code & dgk::kCodeNegPenalty) ? -c0 : c0)));
+  if (f == 0) {
+    const int o = nf * (D + 1);
+    for (int r = 0; r < D; ++r) {
+      double s = 0.0;
+      for (int d = 0; d < D; ++d) {
+        s += g[r * D + d] * v0[d];
+        rf[(o + D + r * D + d) * 32] = (T)g[r * D + d];
+      }
+      rf[(o + r) * 32] = (T)s;
+    }
+    rf[(o + D + D * D) * 32] = (T)v0[D];
+  }
+  if (e < E && (code & dgk::kCodeBoundary)) {
+    const double rc2 = rho0 * c0 * c0;
+    for (int a = 0; a < NV; ++a)
+      for (int b = 0; b < NV; ++b) {
+        double an = a == b ? vn : 0.0;
+        if (a == 0 && b > 0) an = rc2 * gf[b - 1];
+        if (a > 0 && b == 0) an = gf[a - 1] / rho0;
+        outM[(int64_t)nbr * NV * NV + a * NV + b] = (T)(sJ * (an - bm64[(int64_t)nbr * NV * NV + a * NV + b]));
+      }
+  }
+}
+
 struct Scratch {
   std::vector<void*> p;
   ~Scratch() {
@@ -558,6 +608,25 @@ int run_setup(dg_ctx* c, const dg_mesh_desc* mesh, const double* elem_v0, const 
     // ---- curved elements: per-element quadrature data ----
     int rc = setup_curved(c, xyz, en, perm, det, curved, st);
     if (rc != DG_OK) return rc;
+    if (bb_mesh(c)) {
+      const int gw = dgk::bb_geo_words(D);
+      const size_t ts = c->prec == DG_FP32 ? 4 : 8;
+      SETUP_CK(dev_alloc(c, &c->bbF, Epad * gw * ts));
+      SETUP_CK(dev_alloc(c, (void**)&c->bbI, Epad * 2 * nf * sizeof(int)));
+      SETUP_CK(dev_alloc(c, &c->bbM, nbm * ts));
+      if (c->prec == DG_FP32)
+        k_bb_geo<float><<<blocks(Epad * nf, 128), 128, 0, st>>>(geo64, recf64, c->geoI, reci, bm64, D, E, Epad,
+                                                                c->ph.rho0, c->ph.c0, gw, (float*)c->bbF, c->bbI,
+                                                                (float*)c->bbM);
+      else
+        k_bb_geo<double><<<blocks(Epad * nf, 128), 128, 0, st>>>(geo64, recf64, c->geoI, reci, bm64, D, E, Epad,
+                                                                 c->ph.rho0, c->ph.c0, gw, (double*)c->bbF, c->bbI,
+                                                                 (double*)c->bbM);
+      SETUP_CK(cudaGetLastError());
+      SETUP_CK(cudaStreamSynchronize(st));
+      rc = bb_setup_basis(c);
+      if (rc != DG_OK) throw std::runtime_error("basis tables");
+    }
     return DG_OK;
   } catch (const std::exception& ex) {
     c->err = ex.what();

@@ -1,0 +1,779 @@
+// Bernstein-basis RK4 stage kernel (sm_103a, FP32 and FP64 state, triangles
+// and tetrahedra of orders 1..4).
+//
+// Same semi-discrete equations as the reference's per-stage work
+// (src/Mesh.cpp:734-975, src/solver.cpp:38-57, :488-516). The state is held
+// as Bernstein coefficients on the element's lattice in place of nodal
+// values. On straight-sided elements every operator of the scheme is then
+// sparse with small constants (Chan and Warburton, "GPU-accelerated
+// Bernstein-Bezier discontinuous Galerkin methods for wave problems", SIAM J.
+// Sci. Comput. 39, 2017):
+//   * derivative: d/dxi_r of degree P has the degree P-1 coefficients
+//     P (c[b+e_r] - c[b+e_0]);
+//   * degree elevation P-1 -> P: c[a] = sum_k (a_k / P) g[a-e_k];
+//   * lift of a face flux f: layer 0 (the coefficients on the face) is
+//     sJ L0 f, L0 the integer stencil E^T E (E: degree elevation P -> P+1 on
+//     the face, times P+1), and layer j, at lattice distance j from the face,
+//     is -1/(j+1) sum_k (g_k+1) (layer j-1)[g+e_k].
+// The volume term is taken in strong form, so that a face's flux is
+//   f = n.F(y-) - h = 1/2 n.F(d) - 1/2 s c0 d,  d = y- - y+   (interior)
+//   f = (A_n - B) y-                                          (boundary).
+// Per variable and element 3-D p = 3 takes about 700 multiply-adds against
+// 2000 with the dense nodal operators, p = 4 about 1150 against 5800; FP64
+// runs at 2 multiply-adds per clock and SM on GB300, so FP64 stages are bound
+// by that count, and the FP32 stages were bound by the shared-memory loads of
+// the dense operators' entries, which are compile-time constants here.
+//
+// Layout: arrays of tiles of 32 elements, [tile][variable][coefficient][32]:
+// a warp's lanes are the tile's elements, every load and store of a
+// coefficient is one coalesced line or conflict-free shared row (FP32
+// tetrahedra: the Q4 layout of BBCfg and bb_tile_q4).
+// One block per tile with D+1 warps; warp w is face w in the flux phase and
+// variable w in the volume, lift and update phases:
+//   1. the tile's stage input and geometry arrive by TMA bulk copies;
+//   2. each thread issues the loads of its face's neighbour trace (from the
+//      tile itself where the neighbour is in it, else from global memory),
+//      then computes its variable's volume term while they are in flight;
+//   3. it forms its face's flux, applies L0 and stores it to shared memory;
+//   4. it adds its variable's lift of all faces and updates the RK arrays.
+// Every mbarrier wait is bounded; on timeout the block records an error,
+// drains its own copies (bounded) and stops.
+#pragma once
+#include <cstdint>
+#include <utility>
+
+#include "stage2.cuh"
+
+namespace dgk {
+
+// ---- compile-time lattice arithmetic ----------------------------------------
+
+template <class F, int... I>
+__device__ __forceinline__ void bb_for_impl(F&& f, std::integer_sequence<int, I...>) {
+  (f(std::integral_constant<int, I>{}), ...);
+}
+// f(integral_constant<int, 0>) ... f(integral_constant<int, N-1>)
+template <int N, class F>
+__device__ __forceinline__ void bb_for(F&& f) {
+  bb_for_impl(f, std::make_integer_sequence<int, N>{});
+}
+
+struct Bary {
+  int a[4];  // barycentric lattice coordinates, sum p
+};
+
+__host__ __device__ constexpr int bb_np(int d, int p) {
+  return d == 0 ? 1 : d == 1 ? p + 1 : d == 2 ? (p + 1) * (p + 2) / 2 : (p + 1) * (p + 2) * (p + 3) / 6;
+}
+// Index of lattice point (a[1], a[2], a[3]) of degree p, a[1] fastest (the
+// internal node order of refelem.h; a face's lattice is the same in d - 1).
+__host__ __device__ constexpr int bb_index(int d, int p, const Bary& b) {
+  int idx = 0;
+  if (d == 3)
+    for (int k = 0; k < b.a[3]; ++k) idx += bb_np(2, p - k);
+  const int pj = d == 3 ? p - b.a[3] : p;
+  if (d >= 2)
+    for (int j = 0; j < b.a[2]; ++j) idx += pj - j + 1;
+  return d == 0 ? 0 : idx + b.a[1];
+}
+__host__ __device__ constexpr Bary bb_lattice(int d, int p, int n) {
+  Bary b{};
+  int r = n;
+  if (d == 3)
+    while (r >= bb_np(2, p - b.a[3])) r -= bb_np(2, p - b.a[3]), ++b.a[3];
+  const int pj = p - b.a[3];
+  if (d >= 2)
+    while (r >= pj - b.a[2] + 1) r -= pj - b.a[2] + 1, ++b.a[2];
+  if (d >= 1) b.a[1] = r;
+  b.a[0] = p - b.a[1] - b.a[2] - b.a[3];
+  return b;
+}
+// The same as a type (its members are constants inside nested lambdas too).
+template <int DD, int PP, int N>
+struct BLat {
+  static constexpr Bary b = bb_lattice(DD, PP, N);
+};
+__host__ __device__ constexpr Bary bb_add(Bary b, int k, int s) {
+  b.a[k] += s;
+  return b;
+}
+// Local faces' corners (Gmsh's local face tables, as refelem.cpp) and the
+// vertex opposite each face.
+__host__ __device__ constexpr int bb_corner(int d, int f, int k) {
+  if (d == 2) return k == 0 ? f : (f + 1) % 3;
+  const int t[4][3] = {{0, 2, 1}, {0, 1, 3}, {0, 3, 2}, {3, 1, 2}};
+  return t[f][k];
+}
+__host__ __device__ constexpr int bb_opposite(int d, int f) {
+  return d == 2 ? (f + 2) % 3 : f == 0 ? 3 : f == 1 ? 2 : f == 2 ? 1 : 0;
+}
+// Element lattice index of face lattice point g (degree p - j) at distance j
+// from face f.
+__host__ __device__ constexpr int bb_layer_index(int d, int p, int f, int j, const Bary& g) {
+  Bary b{};
+  b.a[bb_opposite(d, f)] = j;
+  for (int k = 0; k < d; ++k) b.a[bb_corner(d, f, k)] = g.a[k];
+  return bb_index(d, p, b);
+}
+// Bernstein polynomial j of degree p at lattice point i.
+__host__ __device__ constexpr double bb_value(int d, int p, int i, int j) {
+  const Bary x = bb_lattice(d, p, i), al = bb_lattice(d, p, j);
+  double v = 1.0;
+  int left = p;
+  for (int k = 0; k <= d; ++k) {
+    for (int t = 1; t <= al.a[k]; ++t) v = v * (double)(left - al.a[k] + t) / (double)t * (double)x.a[k] / (double)p;
+    left -= al.a[k];
+  }
+  return v;
+}
+
+// ---- configuration ------------------------------------------------------------
+
+// NBUF_: stage-input buffers (2: the next tile arrives while this one
+// computes; 1: after its flux phase), MINB: blocks per SM that the register
+// budget allows for.
+template <typename T_, int D_, int P_, int NBUF_, int MINB_, int GA_>
+struct BBCfg {
+  using T = T_;
+  static constexpr int D = D_, P = P_, NBUF = NBUF_, MINB = MINB_;
+  static constexpr bool ASYNC = GA_ != 0;  // neighbour traces by cp.async into sN, else into registers
+  using S = Shape<D_, P_>;
+  static constexpr int NP = S::NP, NF = S::NF, NFP = S::NFP, NV = S::NV, NPERM = S::NPERM;
+  static constexpr int LW = 32;                 // elements per tile
+  static constexpr int NT = LW * NV;            // threads per block
+  static constexpr int TW = NV * NP * LW;       // state words of a tile
+  // Q4 (FP32, 3-D): the four variables of a coefficient side by side,
+  // [tile][coefficient][32][4], else one plane each, [tile][variable][coefficient][32]
+  static constexpr bool Q4 = sizeof(T) == 4 && D == 3;
+  static constexpr int SQ = Q4 ? 1 : NP * LW, SN = Q4 ? 4 * LW : LW, SE = Q4 ? 4 : 1;  // word strides
+  static constexpr int oGV = NF * (D + 1), oG = oGV + D, oS = oG + D * D, GW = oS + 1;  // geometry words
+  static constexpr int GI = 2 * NF;             // neighbour, code
+  static constexpr int CH = sizeof(T) == 8 ? 6 : 10;  // coefficients whose RK operands are in flight together
+  static constexpr uint32_t YB = TW * sizeof(T), GB = GW * LW * sizeof(T), IB = GI * LW * 4;
+  static constexpr size_t oBar = 0;                                     // NBUF mbarriers
+  static constexpr size_t oFm = 64;                                     // int [NF][16]: element word offset of a face node
+  static constexpr size_t oNb = oFm + NF * 16 * 4;                      // uchar [NF*NPERM][16]: neighbour node of a face node
+  static constexpr size_t oY = RoundUp<oNb + NF * NPERM * 16, 128>::v;  // NBUF x [NV][NP][32]
+  static constexpr size_t oGF = oY + (size_t)NBUF * YB;
+  static constexpr size_t oGI = oGF + (size_t)NBUF * GB;
+  static constexpr size_t oN = oGI + (size_t)NBUF * IB;                 // [NF][NV][NFP][32]
+  static constexpr size_t oR = oN + (size_t)NF * NV * NFP * LW * sizeof(T);
+  static constexpr size_t bytes = oR + NV * NV * sizeof(double);
+  static_assert(NF == NV, "a block's warps are faces and variables in turn");
+  static_assert(NFP <= 16 && NP <= 64, "tables hold 16 nodes per face");
+};
+
+// g . (c[b+e_r] - c[b+e_0]) summed over r. FP32 takes the differences first
+// (an error relative to the difference); FP64, whose rate bounds its kernels,
+// one multiply-add per coefficient with g_0 = -sum g_r.
+template <typename T, int D>
+struct BBGrad {
+  T g[D], g0;
+  __device__ __forceinline__ void done() {
+    g0 = -g[0];
+#pragma unroll
+    for (int r = 1; r < D; ++r) g0 -= g[r];
+  }
+  // y: one variable's coefficients; n: index of b + e_0, .., b + e_D
+  template <int N0, int N1, int N2, int N3, int LW>
+  __device__ __forceinline__ T add(T t, const T* y) const {
+    const T c0 = y[N0 * LW];
+    if constexpr (sizeof(T) == 8) {
+      t += g0 * c0;
+      t += g[0] * y[N1 * LW];
+      t += g[1] * y[N2 * LW];
+      if constexpr (D == 3) t += g[2] * y[N3 * LW];
+    } else {
+      t += g[0] * (y[N1 * LW] - c0);
+      t += g[1] * (y[N2 * LW] - c0);
+      if constexpr (D == 3) t += g[2] * (y[N3 * LW] - c0);
+    }
+    return t;
+  }
+};
+
+// Volume term of variable q into out (strong form, see the file comment).
+// y: the tile's stage input at this lane, g: its geometry at this lane.
+template <class C, typename T>
+__device__ __forceinline__ void bb_volume(const T* y, const T* g, int q, T rhoc2, T inv_rho0, T (&out)[C::NP]) {
+  constexpr int D = C::D, P = C::P, NP = C::NP, LW = C::LW;
+  BBGrad<T, D> gv;
+#pragma unroll
+  for (int r = 0; r < D; ++r) gv.g[r] = g[(C::oGV + r) * LW];
+  gv.done();
+#pragma unroll
+  for (int n = 0; n < NP; ++n) out[n] = (T)0;
+  auto scatter = [&](auto b_, T t) {
+    using L = BLat<D, P - 1, decltype(b_)::value>;
+    bb_for<D + 1>([&](auto k_) {
+      constexpr int k = decltype(k_)::value;
+      constexpr int a = bb_index(D, P, bb_add(L::b, k, 1));
+      constexpr int w = L::b.a[k] + 1;
+      out[a] -= (T)w * t;
+    });
+  };
+  if (q == 0) {
+    BBGrad<T, D> gm[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+#pragma unroll
+      for (int r = 0; r < D; ++r) gm[d].g[r] = rhoc2 * g[(C::oG + r * D + d) * LW];
+      gm[d].done();
+    }
+    bb_for<bb_np(D, P - 1)>([&](auto b_) {
+      using L = BLat<D, P - 1, decltype(b_)::value>;
+      constexpr int n0 = bb_index(D, P, bb_add(L::b, 0, 1)), n1 = bb_index(D, P, bb_add(L::b, 1, 1)),
+                    n2 = bb_index(D, P, bb_add(L::b, 2, 1)), n3 = D == 3 ? bb_index(D, P, bb_add(L::b, 3, 1)) : 0;
+      T t = gv.template add<n0, n1, n2, n3, LW>((T)0, y);
+#pragma unroll
+      for (int d = 0; d < D; ++d) t = gm[d].template add<n0, n1, n2, n3, LW>(t, y + (1 + d) * NP * LW);
+      scatter(b_, t);
+    });
+  } else {
+    BBGrad<T, D> gd;
+#pragma unroll
+    for (int r = 0; r < D; ++r) gd.g[r] = inv_rho0 * g[(C::oG + r * D + q - 1) * LW];
+    gd.done();
+    const T* yq = y + q * NP * LW;
+    bb_for<bb_np(D, P - 1)>([&](auto b_) {
+      using L = BLat<D, P - 1, decltype(b_)::value>;
+      constexpr int n0 = bb_index(D, P, bb_add(L::b, 0, 1)), n1 = bb_index(D, P, bb_add(L::b, 1, 1)),
+                    n2 = bb_index(D, P, bb_add(L::b, 2, 1)), n3 = D == 3 ? bb_index(D, P, bb_add(L::b, 3, 1)) : 0;
+      scatter(b_, gd.template add<n0, n1, n2, n3, LW>(gv.template add<n0, n1, n2, n3, LW>((T)0, yq), y));
+    });
+  }
+}
+
+// Value at face node M of the integer stencil L0 = E^T E of a face flux.
+template <class C, int M, typename T>
+__device__ __forceinline__ T bb_stencil_at(const T (&f)[C::NFP]) {
+  constexpr int D = C::D, P = C::P;
+  using L = BLat<D - 1, P, M>;
+  constexpr int w0 = (L::b.a[0] + 1) * (L::b.a[0] + 1) + (L::b.a[1] + 1) * (L::b.a[1] + 1) +
+                     (D == 3 ? (L::b.a[2] + 1) * (L::b.a[2] + 1) : 0);
+  T s = (T)w0 * f[M];
+  bb_for<D * D>([&](auto ij_) {
+    constexpr int i = decltype(ij_)::value / D, j = decltype(ij_)::value % D;
+    if constexpr (i != j && L::b.a[j] > 0) {
+      constexpr int n = bb_index(D - 1, P, bb_add(bb_add(L::b, i, 1), j, -1));
+      constexpr int w = (L::b.a[i] + 1) * L::b.a[j];
+      s += (T)w * f[n];
+    }
+  });
+  return s;
+}
+template <class C, typename T>
+__device__ __forceinline__ void bb_face_stencil(const T (&f)[C::NFP], T* dst) {
+  bb_for<C::NFP>([&](auto m_) { dst[decltype(m_)::value * C::LW] = bb_stencil_at<C, decltype(m_)::value>(f); });
+}
+
+// Adds layers J .. P of face F's lift to out; prev holds layer J-1's values.
+template <class C, int F, int J, typename T>
+__device__ __forceinline__ void bb_layers(const T (&prev)[bb_np(C::D - 1, C::P - J + 1)], T (&out)[C::NP]) {
+  constexpr int D = C::D, P = C::P;
+  if constexpr (J <= P) {
+    T cur[bb_np(D - 1, P - J)];
+    bb_for<bb_np(D - 1, P - J)>([&](auto g_) {
+      using L = BLat<D - 1, P - J, decltype(g_)::value>;
+      constexpr int a = bb_layer_index(D, P, F, J, L::b);
+      T s = J < P ? (T)0 : out[a];
+      bb_for<D>([&](auto k_) {
+        constexpr int k = decltype(k_)::value;
+        constexpr int n = bb_index(D - 1, P - J + 1, bb_add(L::b, k, 1));
+        constexpr double w = -(double)(L::b.a[k] + 1) / (double)(J + 1);
+        s += (T)w * prev[n];
+      });
+      cur[decltype(g_)::value] = s;
+      out[a] = J < P ? out[a] + s : s;
+    });
+    if constexpr (J < P) bb_layers<C, F, J + 1>(cur, out);
+  }
+}
+
+// Adds the lift of all faces for one variable of one element; sN: its face
+// data (node m of face f at f * SF + m * SM).
+template <class C, int SF, int SM, typename T>
+__device__ __forceinline__ void bb_lift(const T* sN, T (&out)[C::NP]) {
+  constexpr int D = C::D, P = C::P;
+  bb_for<C::NF>([&](auto f_) {
+    constexpr int f = decltype(f_)::value;
+    T l0[C::NFP];
+#pragma unroll
+    for (int m = 0; m < C::NFP; ++m) l0[m] = sN[f * SF + m * SM];
+    bb_for<C::NFP>([&](auto m_) {
+      constexpr int a = bb_layer_index(D, P, f, 0, bb_lattice(D - 1, P, decltype(m_)::value));
+      out[a] += l0[decltype(m_)::value];
+    });
+    bb_layers<C, f, 1>(l0, out);
+  });
+}
+
+// Sum over the element's nodes of the squared nodal values of coefficients d.
+template <class C, typename T>
+__device__ __forceinline__ T bb_nodal_square(const T (&d)[C::NP]) {
+  constexpr int D = C::D, P = C::P;
+  T sum = (T)0;
+  bb_for<C::NP>([&](auto i_) {
+    constexpr int i = decltype(i_)::value;
+    T v = (T)0;
+    bb_for<C::NP>([&](auto j_) {
+      constexpr int j = decltype(j_)::value;
+      constexpr double w = bb_value(D, P, i, j);
+      if constexpr (w != 0.0) v += (T)w * d[j];
+    });
+    sum += v * v;
+  });
+  return sum;
+}
+
+// RK operands of CH coefficients of this thread: loaded together (the first
+// group before the lift, so that its latency overlaps it), then combined with
+// dt*L and stored. In stages 4 and 5 out becomes the residual's difference.
+template <class C, typename T>
+struct BBOps {
+  static constexpr int CH = C::CH, SN = C::SN, NP = C::NP;
+  T x0[CH], x1[CH], x2[CH];
+  __device__ __forceinline__ void load(const StageArgs<T>& a, int64_t base, int n0) {
+    const int stage = a.stage;
+    if (stage == 0) return;
+    const T* u = a.u + base;
+    const T* ac = a.acc + base;
+    const T* sn = a.snap + base;
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+      if (n0 + i < NP) x0[i] = u[(n0 + i) * SN];
+    if (stage >= 2 && stage <= 4) {
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) x1[i] = ac[(n0 + i) * SN];
+    }
+    if (stage >= 4) {
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) x2[i] = sn[(n0 + i) * SN];
+    }
+  }
+  __device__ __forceinline__ void update(const StageArgs<T>& a, int64_t base, int n0, T dte, T (&out)[NP]) {
+    const int stage = a.stage;
+    T* ac = a.acc + base;
+    T* yo = a.y_out + base;
+    if (stage == 0) {
+      T* ko = a.k_out + base;
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) ko[(n0 + i) * SN] = dte * out[n0 + i];
+    } else if (stage == 1) {
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) {
+          ac[(n0 + i) * SN] = dte * out[n0 + i];
+          yo[(n0 + i) * SN] = x0[i] + ((T)0.5 * dte) * out[n0 + i];
+        }
+    } else if (stage <= 3) {
+      const T c = stage == 3 ? dte : (T)0.5 * dte, c2 = (T)2 * dte;
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) {
+          ac[(n0 + i) * SN] = x1[i] + c2 * out[n0 + i];
+          yo[(n0 + i) * SN] = x0[i] + c * out[n0 + i];
+        }
+    } else {
+      T* un_ = stage == 4 ? a.u + base : yo;
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) {
+          const T un = stage == 4 ? x0[i] + (x1[i] + dte * out[n0 + i]) * (T)(1.0 / 6.0) : x0[i] + dte * out[n0 + i];
+          un_[(n0 + i) * SN] = un;
+          out[n0 + i] = x2[i] - un;
+        }
+    }
+  }
+};
+
+// constants in the working precision (FP32: rounded on the host, a conversion
+// per thread and tile runs at the FP64 rate)
+template <typename T>
+__device__ __forceinline__ T bb_rhoc2(const StageArgs<T>& a) {
+  if constexpr (sizeof(T) == 4) return a.f_rhoc2; else return a.ph.rhoc2;
+}
+template <typename T>
+__device__ __forceinline__ T bb_inv_rho0(const StageArgs<T>& a) {
+  if constexpr (sizeof(T) == 4) return a.f_inv_rho0; else return a.ph.inv_rho0;
+}
+template <typename T>
+__device__ __forceinline__ T bb_dt(const StageArgs<T>& a) {
+  if constexpr (sizeof(T) == 4) return a.f_dt; else return a.dt;
+}
+
+// One tile: y, g, gi at this lane in shared memory. free_inputs() is called
+// by every thread once the tile's stage input is no longer read.
+template <class C, typename T, class Free>
+__device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, const T* y, const T* g, const int* gi,
+                                        const int* sFm, const unsigned char* sNb, T* sN, int lane, int role, T& racc,
+                                        Free&& free_inputs) {
+  constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, NV = C::NV, LW = C::LW, D = C::D;
+  const T rhoc2 = bb_rhoc2<T>(a), inv_rho0 = bb_inv_rho0<T>(a);
+  // ---- this face's neighbour trace ----
+  const int nbr = gi[role * LW], code = gi[(NF + role) * LW];
+  const bool boundary = code & kCodeBoundary;
+  const bool in_tile = boundary || (nbr >> 5) == tile;
+  const T* nb = in_tile ? y - lane + (boundary ? lane : (nbr & 31)) : a.y_in + (int64_t)(nbr >> 5) * C::TW + (nbr & 31);
+  T up[NV][NFP];
+  uint32_t w[4];
+  T* sf = sN + role * NV * NFP * LW + lane;  // this thread's face data
+  {
+    const int slot = (code & kCodeLfMask) * C::NPERM + ((code >> kCodePermShift) & kCodePermMask);
+    *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(sNb + (boundary ? 0 : slot) * 16);
+    if constexpr (C::ASYNC) {
+      if (!in_tile) {
+#pragma unroll
+        for (int m = 0; m < NFP; ++m) {
+          const T* p = nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * LW;
+#pragma unroll
+          for (int q = 0; q < NV; ++q) {
+            if constexpr (sizeof(T) == 4)
+              cp_async4(sf + (q * NFP + m) * LW, p + q * NP * LW);
+            else
+              cp_async8(sf + (q * NFP + m) * LW, p + q * NP * LW);
+          }
+        }
+      }
+      cp_async_commit();
+    } else {
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        const T* p = nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * LW;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) up[q][m] = p[q * NP * LW];
+      }
+    }
+  }
+  // ---- this variable's volume term ----
+  T out[NP];
+  bb_volume<C>(y, g, role, rhoc2, inv_rho0, out);
+  // ---- this face's flux ----
+  if constexpr (C::ASYNC) cp_async_wait_all();
+  {
+    const T* gf = g + role * (D + 1) * LW;
+    T np_[D], nu_[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) np_[d] = rhoc2 * gf[d * LW], nu_[d] = inv_rho0 * gf[d * LW];
+    const T A = gf[D * LW];
+    const int* fm = sFm + role * 16;
+    if (boundary) {
+      const T* Bg = a.bbM + (int64_t)nbr * NV * NV;
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        T um[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) um[q] = y[q * NP * LW + fm[m]];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          T s = (T)0;
+#pragma unroll
+          for (int qq = 0; qq < NV; ++qq) s += __ldg(Bg + q * NV + qq) * um[qq];
+          up[q][m] = s;
+        }
+      }
+    } else {
+      const T* pb = in_tile ? nb : sf;
+      const int qs = in_tile ? NP * LW : NFP * LW;
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        T d[NV];
+        if constexpr (C::ASYNC) {
+          const T* p = pb + (in_tile ? (int)((w[m / 4] >> (8 * (m % 4))) & 0xffu) : m) * LW;
+#pragma unroll
+          for (int q = 0; q < NV; ++q) up[q][m] = p[q * qs];
+        }
+#pragma unroll
+        for (int q = 0; q < NV; ++q) d[q] = y[q * NP * LW + fm[m]] - up[q][m];
+        T s = A * d[0];
+#pragma unroll
+        for (int k = 0; k < D; ++k) s += np_[k] * d[1 + k];
+        up[0][m] = s;
+#pragma unroll
+        for (int k = 0; k < D; ++k) up[1 + k][m] = A * d[1 + k] + nu_[k] * d[0];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NV; ++q) bb_face_stencil<C>(up[q], sf + q * NFP * LW);
+  }
+  const T dte = bb_dt<T>(a) * g[C::oS * LW];
+  __syncthreads();
+  free_inputs();
+  // ---- this variable's lift and RK update ----
+  const int64_t base = tile * C::TW + role * NP * LW + lane;
+  BBOps<C, T> ops;
+  ops.load(a, base, 0);
+  bb_lift<C, NV * NFP * LW, LW>(sN + role * NFP * LW + lane, out);
+#pragma unroll
+  for (int n0 = 0; n0 < NP; n0 += C::CH) {
+    if (n0 > 0) ops.load(a, base, n0);
+    ops.update(a, base, n0, dte, out);
+  }
+  if (a.stage >= 4) racc += bb_nodal_square<C>(out);
+}
+
+// One tile in the Q4 layout (FP32, 3-D). The flux phase is bb_tile's (a warp
+// per face, a lane per element) with all variables of a node in one 16-byte
+// load: the neighbour trace touches two elements' values per sector instead
+// of one value of eight, and takes a quarter of the load instructions. In the
+// volume, lift and update phases thread t is variable t & 3 of element t >> 2,
+// so that a coefficient of the tile is one contiguous row of the block; the
+// coupling of the variables goes through shuffles within an element's four
+// lanes (every lane forms t_j = H_j . D u with H_j the metric column that its
+// neighbour lane ^ (j+1) needs, zero where it needs none).
+template <class C, class Free>
+__device__ __forceinline__ void bb_tile_q4(const StageArgs<float>& a, int64_t tile, const float* y, const float* g,
+                                           const int* gi, const int* sFm, const unsigned char* sNb, float* sN, int tid,
+                                           int role, float& racc, Free&& free_inputs) {
+  constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, LW = C::LW, D = C::D, P = C::P, SN = C::SN;
+  const float rhoc2 = a.f_rhoc2, inv_rho0 = a.f_inv_rho0;
+  const int lane = tid & 31;
+  // ---- this face's neighbour trace ----
+  const int nbr = gi[role * LW + lane], code = gi[(NF + role) * LW + lane];
+  const bool boundary = code & kCodeBoundary;
+  const bool in_tile = boundary || (nbr >> 5) == tile;
+  float4 up[NFP];
+  {
+    const float* nb = in_tile ? y + 4 * (boundary ? lane : (nbr & 31))
+                              : a.y_in + (int64_t)(nbr >> 5) * C::TW + 4 * (nbr & 31);
+    const int slot = (code & kCodeLfMask) * C::NPERM + ((code >> kCodePermShift) & kCodePermMask);
+    uint32_t w[4];
+    *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(sNb + (boundary ? 0 : slot) * 16);
+#pragma unroll
+    for (int m = 0; m < NFP; ++m)
+      up[m] = *reinterpret_cast<const float4*>(nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * SN);
+  }
+  // ---- volume term of this thread's variable q of element el ----
+  const int q = tid & 3, el = tid >> 2;
+  float out[NP];
+  {
+    float gv[3], H[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) gv[r] = g[(C::oGV + r) * LW + el];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const float x = g[(C::oG + r * D + j) * LW + el];
+        H[j][r] = q == 0 ? inv_rho0 * x : q == j + 1 ? rhoc2 * x : 0.f;
+      }
+#pragma unroll
+    for (int n = 0; n < NP; ++n) out[n] = 0.f;
+    const float* yq = y + tid;
+    bb_for<bb_np(D, P - 1)>([&](auto b_) {
+      using L = BLat<D, P - 1, decltype(b_)::value>;
+      constexpr int n0 = bb_index(D, P, bb_add(L::b, 0, 1)), n1 = bb_index(D, P, bb_add(L::b, 1, 1)),
+                    n2 = bb_index(D, P, bb_add(L::b, 2, 1)), n3 = bb_index(D, P, bb_add(L::b, 3, 1));
+      const float c0 = yq[n0 * SN], d1 = yq[n1 * SN] - c0, d2 = yq[n2 * SN] - c0, d3 = yq[n3 * SN] - c0;
+      float t = gv[0] * d1 + gv[1] * d2 + gv[2] * d3;
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        t += __shfl_xor_sync(0xffffffffu, H[j][0] * d1 + H[j][1] * d2 + H[j][2] * d3, j + 1);
+      bb_for<D + 1>([&](auto k_) {
+        constexpr int k = decltype(k_)::value;
+        constexpr int n = bb_index(D, P, bb_add(L::b, k, 1));
+        constexpr int w = L::b.a[k] + 1;
+        out[n] -= (float)w * t;
+      });
+    });
+  }
+  // ---- this face's flux ----
+  {
+    const float* gf = g + role * (D + 1) * LW + lane;
+    const int* fm = sFm + role * 16;
+    float f[4][NFP];
+    const float* yl = y + 4 * lane;
+    if (boundary) {
+      const float* Bg = a.bbM + (int64_t)nbr * 16;
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          f[v][m] = __ldg(Bg + v * 4) * um.x + __ldg(Bg + v * 4 + 1) * um.y + __ldg(Bg + v * 4 + 2) * um.z +
+                    __ldg(Bg + v * 4 + 3) * um.w;
+      }
+    } else {
+      const float A = gf[D * LW], n0 = gf[0], n1 = gf[LW], n2 = gf[2 * LW];
+      const float p0 = rhoc2 * n0, p1 = rhoc2 * n1, p2 = rhoc2 * n2;
+      const float u0 = inv_rho0 * n0, u1 = inv_rho0 * n1, u2 = inv_rho0 * n2;
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
+        const float dp = um.x - up[m].x, dx = um.y - up[m].y, dy = um.z - up[m].z, dz = um.w - up[m].w;
+        f[0][m] = A * dp + p0 * dx + p1 * dy + p2 * dz;
+        f[1][m] = A * dx + u0 * dp;
+        f[2][m] = A * dy + u1 * dp;
+        f[3][m] = A * dz + u2 * dp;
+      }
+    }
+    float* sf = sN + role * NFP * SN + 4 * lane;
+    bb_for<NFP>([&](auto m_) {
+      constexpr int m = decltype(m_)::value;
+      *reinterpret_cast<float4*>(sf + m * SN) =
+          make_float4(bb_stencil_at<C, m>(f[0]), bb_stencil_at<C, m>(f[1]), bb_stencil_at<C, m>(f[2]),
+                      bb_stencil_at<C, m>(f[3]));
+    });
+  }
+  const float dte = a.f_dt * g[C::oS * LW + el];
+  __syncthreads();
+  free_inputs();
+  // ---- this variable's lift and RK update ----
+  const int64_t base = tile * C::TW + tid;
+  BBOps<C, float> ops;
+  ops.load(a, base, 0);
+  bb_lift<C, NFP * SN, SN>(sN + tid, out);
+#pragma unroll
+  for (int n0 = 0; n0 < NP; n0 += C::CH) {
+    if (n0 > 0) ops.load(a, base, n0);
+    ops.update(a, base, n0, dte, out);
+  }
+  if (a.stage >= 4) racc += bb_nodal_square<C>(out);
+}
+
+// Face tables in shared memory: element word offset of each face node, and
+// the neighbour's node for each (its local face, corner permutation).
+template <class C, typename T>
+__device__ __forceinline__ void bb_load_tables(const StageArgs<T>& a, int* sFm, unsigned char* sNb, int tid, int nt) {
+  for (int i = tid; i < C::NF * 16; i += nt)
+    sFm[i] = i % 16 < C::NFP ? (int)a.fmask[i / 16 * C::NFP + i % 16] * C::SN : 0;
+  for (int i = tid; i < C::NF * C::NPERM * 16; i += nt)
+    sNb[i] = i % 16 < C::NFP ? (unsigned char)a.nbrnode[i / 16 * C::NFP + i % 16] : (unsigned char)0;
+}
+
+template <typename T, int D, int P, int NBUF, int MINB, int GA>
+__global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB, GA>::NT, MINB) stage_bb_kernel(const StageArgs<T> a, int* err) {
+  using C = BBCfg<T, D, P, NBUF, MINB, GA>;
+  extern __shared__ __align__(128) unsigned char sm[];
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + C::oBar);
+  int* sFm = reinterpret_cast<int*>(sm + C::oFm);
+  unsigned char* sNb = sm + C::oNb;
+  T* sY = reinterpret_cast<T*>(sm + C::oY);
+  T* sGF = reinterpret_cast<T*>(sm + C::oGF);
+  int* sGI = reinterpret_cast<int*>(sm + C::oGI);
+  T* sN = reinterpret_cast<T*>(sm + C::oN);
+  double* sRed = reinterpret_cast<double*>(sm + C::oR);
+  const int tid = threadIdx.x, lane = tid & 31;
+  // the pressure's volume term is the longest: its warp is another scheduler's
+  // in each block that shares an SM
+  const int role = ((tid >> 5) + blockIdx.x) % C::NV;
+  const int nepi = a.stage == 1 || a.stage == 5 ? 1 : a.stage == 2 || a.stage == 3 ? 2 : a.stage == 4 ? 3 : 0;
+
+  auto issue = [&](int64_t tile, int b) {
+    mbar_expect_tx(&bar[b], C::YB + C::GB + C::IB);
+    tma_load_1d(sY + (size_t)b * C::TW, a.y_in + tile * C::TW, C::YB, &bar[b]);
+    tma_load_1d(sGF + (size_t)b * C::GW * C::LW, a.bbF + tile * C::GW * C::LW, C::GB, &bar[b]);
+    tma_load_1d(sGI + (size_t)b * C::GI * C::LW, a.bbI + tile * C::GI * C::LW, C::IB, &bar[b]);
+    // the tile's RK operands towards L2
+    if (nepi >= 1 && a.u != a.y_in) prefetch_l2(a.u + tile * C::TW, C::YB);
+    if (nepi >= 2) prefetch_l2(a.acc + tile * C::TW, C::YB);
+    if (nepi >= 3) prefetch_l2(a.snap + tile * C::TW, C::YB);
+  };
+
+  if (tid == 0) {
+#pragma unroll
+    for (int b = 0; b < NBUF; ++b) mbar_init(&bar[b], 1);
+    fence_mbar_init();
+  }
+  bb_load_tables<C>(a, sFm, sNb, tid, C::NT);
+  __syncthreads();
+  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue(blockIdx.x, 0);
+
+  T racc = (T)0;
+  bool ok = true;
+  int it = 0;
+  for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ++it) {
+    const int b = NBUF == 2 ? it & 1 : 0;
+    const bool got = mbar_wait(&bar[b], (NBUF == 2 ? it >> 1 : it) & 1, a.wait_limit);
+    if (__syncthreads_or(!got)) {  // also: every thread is done with the previous tile
+      ok = false;
+      if (tid == 0) mbar_wait(&bar[b], (NBUF == 2 ? it >> 1 : it) & 1);  // drained (full limit)
+      break;
+    }
+    const int next = tile + gridDim.x;
+    auto issue_next = [&]() {
+      if (tid == 0 && next < a.ntiles) {
+        fence_proxy_async();
+        issue(next, NBUF == 2 ? b ^ 1 : 0);
+      }
+    };
+    if constexpr (NBUF == 2) issue_next();
+    const T* y = sY + (size_t)b * C::TW;
+    const T* g = sGF + (size_t)b * C::GW * C::LW;
+    const int* gi = sGI + (size_t)b * C::GI * C::LW;
+    auto free_inputs = [&]() {
+      if constexpr (NBUF == 1) issue_next();
+    };
+    if constexpr (C::Q4)
+      bb_tile_q4<C>(a, tile, y, g, gi, sFm, sNb, sN, tid, role, racc, free_inputs);
+    else
+      bb_tile<C, T>(a, tile, y + lane, g + lane, gi + lane, sFm, sNb, sN, lane, role, racc, free_inputs);
+  }
+  if (!ok && tid == 0) atomicOr(err, 1);
+
+  if (a.stage >= 4) {
+    // block sums per variable: a warp's lanes are one variable's (Q4: each
+    // variable's are every fourth lane)
+    double v = (double)racc;
+#pragma unroll
+    for (int off = 16; off >= (C::Q4 ? 4 : 1); off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if constexpr (C::Q4) {
+      if (lane < 4) sRed[lane * 4 + (tid >> 5)] = v;
+    } else {
+      if (lane == 0) sRed[role] = v;
+    }
+    __syncthreads();
+    if (tid < 5) {
+      // p, p / c0^2, vx, vy, vz
+      const int q = tid < 2 ? 0 : tid - 1;
+      double s = 0.0;
+      if (q < C::NV) {
+        if constexpr (C::Q4)
+          s = (sRed[q * 4] + sRed[q * 4 + 1]) + (sRed[q * 4 + 2] + sRed[q * 4 + 3]);
+        else
+          s = sRed[q];
+      }
+      a.partials[blockIdx.x * 5 + tid] = tid == 1 ? s / (a.c0sq * a.c0sq) : s;
+    }
+  }
+}
+
+template <typename T, int D, int P, int NBUF, int MINB, int GA>
+struct StageBB {
+  using C = BBCfg<T, D, P, NBUF, MINB, GA>;
+  static cudaError_t set_attrs() {
+    auto kfn = stage_bb_kernel<T, D, P, NBUF, MINB, GA>;
+    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::bytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e;
+  }
+  static cudaError_t launch(const StageArgs<T>& a, int grid, int* err, cudaStream_t s) {
+    static bool configured = false;
+    if (!configured) {
+      cudaError_t e = set_attrs();
+      if (e != cudaSuccess) return e;
+      configured = true;
+    }
+    stage_bb_kernel<T, D, P, NBUF, MINB, GA><<<grid, C::NT, C::bytes, s>>>(a, err);
+    return cudaGetLastError();
+  }
+  static int blocks_per_sm() {
+    if (set_attrs() != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stage_bb_kernel<T, D, P, NBUF, MINB, GA>, C::NT, C::bytes) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return nb;
+  }
+};
+
+}  // namespace dgk

@@ -15,9 +15,7 @@ cudaError_t multi_attrs() {
 }
 }  // namespace
 
-int stage_multi_elems_per_tile(int order) {
-  return order == 2 ? MultiC2::ET : order == 3 ? MultiC3::ET : order == 4 ? MultiC4::ET : 0;
-}
+int stage_multi_elems_per_tile(int order) { return order >= 2 && order <= 4 ? MultiC4::LW : 0; }
 
 int stage_multi_blocks_per_sm() {
   if (multi_attrs() != cudaSuccess) {

@@ -32,6 +32,7 @@
 #include <thread>
 #include <vector>
 
+#include "bb.cuh"
 #include "ctx.h"
 
 namespace {
@@ -326,9 +327,14 @@ int dg_vtu_write_async(dg_vtu_writer* w, const char* path) {
     return vfail(w, DG_ERR_CUDA, std::string("CUDA (snapshot): ") + cudaGetErrorString(e));
   };
   const int64_t E = c->E;
-  k_vtu_cells<<<(unsigned)((E + 127) / 128), 128, 0, c->stream>>>(c->u, c->prec == DG_FP32 ? 1 : 0, c->d_perm, E,
-                                                                  c->np, c->nv, c->Epad * c->np, c->c0sq, s.d);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e;
+  if (c->bb) {
+    e = dgc::bb_cell_means(c, s.d, true);
+  } else {
+    k_vtu_cells<<<(unsigned)((E + 127) / 128), 128, 0, c->stream>>>(c->u, c->prec == DG_FP32 ? 1 : 0, c->d_perm, E,
+                                                                    c->np, c->nv, c->Epad * c->np, c->c0sq, s.d);
+    e = cudaGetLastError();
+  }
   if (e == cudaSuccess) e = cudaEventRecord(s.computed, c->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(w->copy, s.computed, 0);
   if (e == cudaSuccess) e = cudaMemcpyAsync(s.h, s.d, (size_t)E * 5 * sizeof(double), cudaMemcpyDeviceToHost, w->copy);

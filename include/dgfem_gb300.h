@@ -90,8 +90,9 @@ typedef struct {
   int64_t penalty_sign_hist[2]; /* interior faces with s_f = -1, +1 */
   int64_t device_bytes;
   double setup_ms;
-  int kernel_variant; /* stage kernel in use: -1 baseline, 0..15 pipelined variant k, 16..18 tensor-core
-                         kernel, 32.. constant-operator variant */
+  int kernel_variant; /* stage kernel in use: 64 + k Bernstein-basis variant k (straight-sided triangles and
+                         tetrahedra), else -1 baseline, 0..15 pipelined variant k, 16..22 tensor-core kernel,
+                         32.. constant-operator variant, 48.. wide-chunk variant */
   int kernel_grid;    /* blocks of each stage-kernel launch (persistent blocks for variants >= 0) */
   int64_t n_curved;   /* curved elements (high-order nodes off the straight-sided lattice), integrated
                          element by element with the reference's quadrature formulation */
@@ -167,7 +168,12 @@ int dg_vtu_writer_stats(const dg_vtu_writer* w, int64_t* files_written, int* com
  * head/tail-split operands, FP32-level results); 19, 20: the two-chunk
  * tensor-core kernel (K applied in at most two chunks so that two blocks
  * share an SM) with 256 or 512 threads per block (FP32 only); 32 + k: constant-operator variant k (FP32
- * contexts only: operators in constant memory). Returns
+ * contexts only: operators in constant memory); 48 + k: wide-chunk variant k
+ * (FP32 contexts only); 64 + k: Bernstein-basis variant k (straight-sided
+ * triangles and tetrahedra, both precisions; there the only ones that are
+ * timed). The Bernstein-basis kernels hold the state as Bernstein
+ * coefficients: a change to or from them converts state and snapshot, to
+ * rounding. Returns
  * DG_ERR_ARG for a variant that does not exist for this element type or
  * precision. */
 int dg_tune(dg_ctx* ctx, int variant);
