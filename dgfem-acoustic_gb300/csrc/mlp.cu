@@ -9,18 +9,20 @@
 // (FP32 master copies for the optimiser), activations and gradients in FP32,
 // every sum accumulated in FP32.
 //
-// Kernels: one GEMM serves the three products of a layer: Z = X W^T
-// (forward), dX = dZ W (input gradient) and dW = dZ^T X (weight gradient),
-// on the CUDA cores (k_gemm: 64 x 64 output tile, 16-deep K slices staged in
-// shared memory, 4 x 4 outputs per thread; the default) or on the tensor
-// cores (k_gemm_tc, tcgen05 kind::tf32; dg_mlp_set_tensor_cores). At this
-// network's sizes (layers of at most 512, 256-2000 rows) the CUDA-core GEMM
-// is the faster: the tensor-core one stages and splits each K slice and waits
-// for its MMAs before the next (GB300, the 6-256-256-256-256-512 network:
-// forward of 2000 rows 0.31 against 0.63 ms, a training step of 256 rows
-// 0.68 against 0.87 ms, host arrays);
-// element-wise GELU and its derivative, the MSE gradient, bias reductions
-// and an Adam step complete the training loop.
+// Networks whose widths are all at most 1024 run the fused passes of
+// mlp_fused.cuh: one launch for the forward pass, one for the chain of input
+// gradients, one for all weight gradients and the loss, one for the optimiser
+// step with every weight copy. Measured against one GEMM per layer (GB300, the
+// 6-256-256-256-256-512 network): forward of 2000 rows on the device 95 -> 29
+// us, a training step of 256 rows 680 -> 79 us.
+// Wider networks, and dg_mlp_set_tensor_cores, use per-layer kernels: one GEMM
+// serves the three products of a layer, Z = X W^T (forward), dX = dZ W (input
+// gradient) and dW = dZ^T X (weight gradient), on the CUDA cores (k_gemm: 64 x
+// 64 output tile, 16-deep K slices staged in shared memory, 4 x 4 outputs per
+// thread) or on the tensor cores (k_gemm_tc, tcgen05 kind::tf32, which stages
+// and splits each K slice and waits for its MMAs before the next: at this
+// network's sizes the slower one); element-wise GELU and its derivative, the
+// MSE gradient, bias reductions and an Adam step complete the loop.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -33,6 +35,7 @@
 #include <vector>
 
 #include "../../include/dgfem_gb300.h"
+#include "mlp_fused.cuh"
 #include "stage_tc.cuh"  // tcgen05, mbarrier and shared-memory descriptor helpers
 
 namespace dgc {
@@ -362,6 +365,16 @@ struct dg_mlp {
   int* bidx = nullptr;
   int64_t n_data = 0, bcap = 0;
   int64_t step = 0;  // Adam steps taken
+  // fused passes (mlp_fused.cuh; every width within kMaxWidth): the weights in
+  // the order the forward and the backward pass read them, the loss's ticket
+  bool fused = false;
+  mlpf::Net net{};
+  __nv_bfloat16 *wt = nullptr, *wb = nullptr;
+  int fwd_chunks = 0, bwd_chunks = 0;
+  int fwd_ka = 1, fwd_kb = 1, bwd_ka = 1, bwd_kb = 1;  // widths of the two activation buffers
+  mlpf::DwPlan plan{};
+  unsigned* ticket = nullptr;
+  int num_sms = 0;
   int tc = 0;             // GEMMs on the tensor cores (k_gemm_tc), else k_gemm
   int* d_err = nullptr;   // set by a tensor-core GEMM whose wait gave up
   std::string err;
@@ -401,7 +414,18 @@ int ensure_cap(dg_mlp* m, int64_t n) {
   }
   MCK(m, cudaMalloc(&m->dA, n * max_width(m) * sizeof(float)));
   MCK(m, cudaMalloc(&m->dB, n * max_width(m) * sizeof(float)));
+  for (int l = 0; l <= L; ++l) m->net.X[l] = m->X[l], m->net.Z[l] = m->Z[l];
   m->cap = n;
+  return DG_OK;
+}
+
+// Room for the targets of a batch of n rows.
+int ensure_targets(dg_mlp* m, int64_t n) {
+  if (n <= m->bcap) return DG_OK;
+  cudaFree(m->by);
+  m->by = nullptr, m->bcap = 0;
+  MCK(m, cudaMalloc(&m->by, n * m->w.back() * sizeof(float)));
+  m->bcap = n;
   return DG_OK;
 }
 
@@ -438,7 +462,135 @@ int check_gemm_waits(dg_mlp* m) {
   return fail(m, DG_ERR_TIMEOUT, "dg_mlp: a tensor-core GEMM timed out waiting for its MMAs");
 }
 
+constexpr size_t mlpf_max_smem = 227 * 1024;
+
+bool use_fused(const dg_mlp* m) { return m->fused && !m->tc; }
+
+// Groups of 8 rows per tile (1, 2 or 4) of a fused pass over n rows: the one
+// with the least time over its waves of tiles, by what a tile of each takes
+// (mlp_fused.cuh; at 8 rows the weight stream bounds it).
+int pick_groups(const dg_mlp* m, int64_t n, int ka, int kb, bool bwd) {
+  int best = 1;
+  double best_cost = 1e300;
+  const int groups[3] = {1, 2, 4};
+  const double cost[3] = {10, 13, 21};
+  for (int k = 0; k < 3; ++k) {
+    if (mlpf::pass_smem(8 * groups[k], mlpf::stages(groups[k], bwd), ka, kb) > mlpf_max_smem) break;
+    const int64_t tiles = (n + 8 * groups[k] - 1) / (8 * groups[k]);
+    const double c = (double)((tiles + m->num_sms - 1) / m->num_sms) * cost[k];
+    if (c < best_cost) best_cost = c, best = groups[k];
+  }
+  return best;
+}
+
+template <typename F>
+cudaError_t pass_attr(F kfn) {
+  return cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlpf_max_smem);
+}
+
+unsigned pass_grid(const dg_mlp* m, int64_t n, int rows) {
+  return (unsigned)std::min<int64_t>((n + rows - 1) / rows, m->num_sms);
+}
+
+// The whole forward pass in one launch: x (device; row idx[r] when given) to
+// y (device).
+template <bool TRAIN>
+int fused_forward(dg_mlp* m, const float* x, const int* idx, int64_t n, float* y) {
+  const int k = pick_groups(m, n, m->fwd_ka, m->fwd_kb, false), rows = 8 * k;
+  auto go = [&](auto kfn) {
+    kfn<<<pass_grid(m, n, rows), mlpf::kThreads, mlpf::pass_smem(rows, mlpf::stages(k, false), m->fwd_ka, m->fwd_kb), m->stream>>>(
+        m->net, m->wt, m->fwd_chunks, x, idx, n, y, m->fwd_ka, m->d_err);
+  };
+  if (k == 1)
+    go(mlpf::k_forward<1, TRAIN>);
+  else if (k == 2)
+    go(mlpf::k_forward<2, TRAIN>);
+  else
+    go(mlpf::k_forward<4, TRAIN>);
+  MCK(m, cudaGetLastError());
+  return DG_OK;
+}
+
+// Gradients of all parameters into m->g and the loss into *loss (device),
+// after fused_forward<true> of the same rows.
+int fused_backward(dg_mlp* m, const float* t, const int* idx, int64_t n, double* loss) {
+  const int k = pick_groups(m, n, m->bwd_ka, m->bwd_kb, true), rows = 8 * k, L = (int)m->w.size() - 1;
+  auto go = [&](auto kfn) {
+    kfn<<<pass_grid(m, n, rows), mlpf::kThreads, mlpf::pass_smem(rows, mlpf::stages(k, true), m->bwd_ka, m->bwd_kb), m->stream>>>(
+        m->net, m->wb, m->bwd_chunks, m->X[L], t, idx, n, m->bwd_ka, m->d_err);
+  };
+  if (k == 1)
+    go(mlpf::k_backward<1>);
+  else if (k == 2)
+    go(mlpf::k_backward<2>);
+  else
+    go(mlpf::k_backward<4>);
+  MCK(m, cudaGetLastError());
+  mlpf::k_weight_grads<<<m->plan.tiles + mlpf::kLossBlocks, mlpf::kDwThreads, 0, m->stream>>>(
+      m->net, m->plan, n, m->g, m->X[L], t, idx, m->part, m->ticket, loss);
+  MCK(m, cudaGetLastError());
+  return DG_OK;
+}
+
+// Layer table, weight streams and gradient tiles of the fused passes.
+cudaError_t fused_setup(dg_mlp* m) {
+  const int L = (int)m->w.size() - 1;
+  for (int v : m->w)
+    if (v > mlpf::kMaxWidth) return cudaSuccess;  // (the per-layer GEMMs)
+  int64_t to = 0, go = 0;
+  mlpf::Net& net = m->net;
+  net.L = L;
+  for (int l = 0; l <= L; ++l) net.w[l] = m->w[l];
+  int tiles = 0;
+  for (int l = 0; l < L; ++l) {
+    const int K = m->w[l], N = m->w[l + 1];
+    net.b[l] = m->p + m->boff[l];
+    net.woff[l] = m->woff[l], net.boff[l] = m->boff[l], net.hoff[l] = m->hoff[l];
+    net.toff[l] = to;
+    to += (int64_t)((N + mlpf::kNC - 1) / mlpf::kNC) * mlpf::up(K, mlpf::kKC) * mlpf::kNC;
+    // layer l's input alternates between the two buffers, from the first on;
+    // so do the backward pass's gradients, from the outputs down
+    int& f = l % 2 == 0 ? m->fwd_ka : m->fwd_kb;
+    f = std::max(f, K);
+    int& g = (L - 1 - l) % 2 == 0 ? m->bwd_ka : m->bwd_kb;
+    g = std::max(g, N);
+    m->plan.first[l] = tiles;
+    tiles += ((N + mlpf::kDwN - 1) / mlpf::kDwN) * ((K + mlpf::kDwK - 1) / mlpf::kDwK);
+  }
+  m->plan.tiles = tiles;
+  for (int l = L - 1; l >= 1; --l) {  // in the order the backward pass reads them
+    const int K = m->w[l], N = m->w[l + 1];
+    net.goff[l] = go;
+    go += (int64_t)((K + mlpf::kNC - 1) / mlpf::kNC) * mlpf::up(N, mlpf::kKC) * mlpf::kNC;
+  }
+  const int64_t cw = mlpf::kKC * mlpf::kNC;
+  m->fwd_chunks = (int)(to / cw), m->bwd_chunks = (int)(go / cw);
+  cudaError_t e = cudaMalloc(&m->wt, to * sizeof(__nv_bfloat16));
+  if (e == cudaSuccess) e = cudaMalloc(&m->wb, std::max<int64_t>(go, cw) * sizeof(__nv_bfloat16));
+  if (e == cudaSuccess) e = cudaMalloc(&m->ticket, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->wt, 0, to * sizeof(__nv_bfloat16), m->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->wb, 0, std::max<int64_t>(go, cw) * sizeof(__nv_bfloat16), m->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->ticket, 0, sizeof(unsigned), m->stream);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, m->device);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_forward<1, false>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_forward<2, false>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_forward<4, false>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_forward<1, true>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_forward<2, true>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_forward<4, true>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_backward<1>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_backward<2>);
+  if (e == cudaSuccess) e = pass_attr(mlpf::k_backward<4>);
+  m->fused = e == cudaSuccess;
+  return e;
+}
+
 int refresh_bf16(dg_mlp* m) {
+  if (m->fused) {
+    mlpf::k_refresh<<<nblk(m->n_params, 256), 256, 0, m->stream>>>(m->net, m->p, m->n_params, m->wh, m->wt, m->wb);
+    MCK(m, cudaGetLastError());
+    return DG_OK;
+  }
   const int L = (int)m->w.size() - 1;
   for (int l = 0; l < L; ++l) {
     const int64_t nw = (int64_t)m->w[l + 1] * m->w[l];
@@ -451,6 +603,7 @@ int refresh_bf16(dg_mlp* m) {
 // Forward pass of n rows already in X[0]; output in X[L].
 int forward(dg_mlp* m, int64_t n) {
   const int L = (int)m->w.size() - 1;
+  if (use_fused(m)) return fused_forward<false>(m, m->X[0], nullptr, n, m->X[L]);
   for (int l = 0; l < L; ++l) {
     const int K = m->w[l], N = m->w[l + 1];
     const bool last = l == L - 1;
@@ -534,6 +687,7 @@ int dg_mlp_create(int n_layers, const int* widths, int device, dg_mlp** out) {
   // not be ordered with the uploads that follow
   for (float* q : {m->p, m->g, m->m1, m->m2})
     if (e == cudaSuccess) e = cudaMemsetAsync(q, 0, m->n_params * sizeof(float), m->stream);
+  if (e == cudaSuccess) e = fused_setup(m);
   if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
   if (e != cudaSuccess) {
     std::string msg = std::string("dg_mlp_create: CUDA: ") + cudaGetErrorString(e);
@@ -551,7 +705,7 @@ int dg_mlp_destroy(dg_mlp* m) {
   for (float* q : m->Z) cudaFree(q);
   for (void* q : {(void*)m->p, (void*)m->g, (void*)m->m1, (void*)m->m2, (void*)m->wh, (void*)m->dA, (void*)m->dB,
                   (void*)m->part, (void*)m->loss, (void*)m->tx, (void*)m->ty, (void*)m->bx, (void*)m->by,
-                  (void*)m->bidx, (void*)m->d_err})
+                  (void*)m->bidx, (void*)m->d_err, (void*)m->wt, (void*)m->wb, (void*)m->ticket})
     cudaFree(q);
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
@@ -586,6 +740,17 @@ int dg_mlp_get_params(dg_mlp* m, float* params) {
 int dg_mlp_forward_device(dg_mlp* m, const float* x, int64_t n, float* y, void* stream) {
   if (!m || !x || !y || n < 1) return fail(m, DG_ERR_ARG, "dg_mlp_forward_device: invalid argument");
   cudaSetDevice(m->device);
+  // a block reads its rows of x before it writes its rows of y, but not before
+  // other blocks write theirs: arrays that overlap go through a copy of x
+  const uintptr_t xb = (uintptr_t)x, xe = (uintptr_t)(x + n * m->w.front());
+  const uintptr_t yb = (uintptr_t)y, ye = (uintptr_t)(y + n * m->w.back());
+  if (use_fused(m) && (xe <= yb || ye <= xb)) {
+    cudaStream_t keep = m->stream;
+    if (stream) m->stream = (cudaStream_t)stream;
+    const int rc = fused_forward<false>(m, x, nullptr, n, y);
+    m->stream = keep;
+    return rc;
+  }
   int rc = ensure_cap(m, n);
   if (rc != DG_OK) return rc;
   cudaStream_t s = stream ? (cudaStream_t)stream : m->stream;
@@ -611,7 +776,6 @@ int dg_mlp_forward(dg_mlp* m, const float* x, int64_t n, float* y) {
   rc = forward(m, n);
   if (rc != DG_OK) return rc;
   MCK(m, cudaMemcpyAsync(y, m->X[L], n * m->w[L] * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-  MCK(m, cudaStreamSynchronize(m->stream));
   return check_gemm_waits(m);
 }
 
@@ -619,25 +783,23 @@ int dg_mlp_gradient(dg_mlp* m, const float* x, const float* t, int64_t n, float*
   if (!m || !x || !t || !grad || n < 1) return fail(m, DG_ERR_ARG, "dg_mlp_gradient: invalid argument");
   cudaSetDevice(m->device);
   int rc = ensure_cap(m, n);
+  if (rc == DG_OK) rc = ensure_targets(m, n);
   if (rc != DG_OK) return rc;
   const int L = (int)m->w.size() - 1;
-  float* dt = nullptr;
-  MCK(m, cudaMalloc(&dt, n * m->w[L] * sizeof(float)));
-  cudaError_t e = cudaMemcpyAsync(m->X[0], x, n * m->w[0] * sizeof(float), cudaMemcpyHostToDevice, m->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, n * m->w[L] * sizeof(float), cudaMemcpyHostToDevice, m->stream);
-  if (e == cudaSuccess) {
+  MCK(m, cudaMemcpyAsync(m->X[0], x, n * m->w[0] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+  if (use_fused(m)) rc = fused_forward<true>(m, m->X[0], nullptr, n, m->X[L]);
+  MCK(m, cudaMemcpyAsync(m->by, t, n * m->w[L] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+  if (use_fused(m)) {
+    if (rc == DG_OK) rc = fused_backward(m, m->by, nullptr, n, m->loss);
+  } else {
     rc = forward(m, n);
-    if (rc == DG_OK) rc = mse(m, dt, n);
+    if (rc == DG_OK) rc = mse(m, m->by, n);
     if (rc == DG_OK) rc = backward(m, n);
-    if (rc == DG_OK) e = cudaMemcpyAsync(grad, m->g, m->n_params * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
-    if (rc == DG_OK && e == cudaSuccess && loss)
-      e = cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
   }
-  cudaFree(dt);
-  if (e != cudaSuccess) return fail(m, DG_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e));
-  if (rc == DG_OK) rc = check_gemm_waits(m);
-  return rc;
+  if (rc != DG_OK) return rc;
+  MCK(m, cudaMemcpyAsync(grad, m->g, m->n_params * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+  if (loss) MCK(m, cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
+  return check_gemm_waits(m);
 }
 
 int dg_mlp_set_data(dg_mlp* m, const float* x, const float* t, int64_t n) {
@@ -664,12 +826,8 @@ int dg_mlp_train(dg_mlp* m, int64_t n_steps, int batch, double lr, double lr_fin
   int rc = ensure_cap(m, batch);
   if (rc != DG_OK) return rc;
   const int L = (int)m->w.size() - 1;
-  if (m->bcap < batch) {
-    cudaFree(m->by), cudaFree(m->bidx);
-    m->by = nullptr, m->bidx = nullptr;
-    MCK(m, cudaMalloc(&m->by, (int64_t)batch * m->w[L] * sizeof(float)));
-    m->bcap = batch;
-  }
+  if (!use_fused(m)) rc = ensure_targets(m, batch);
+  if (rc != DG_OK) return rc;
   // one permutation of the training rows per epoch, drawn on the host
   const int64_t nd = m->n_data, steps_per_epoch = nd / batch;
   std::vector<int> perm(nd);
@@ -689,26 +847,38 @@ int dg_mlp_train(dg_mlp* m, int64_t n_steps, int batch, double lr, double lr_fin
       if (e != cudaSuccess) break;
     }
     const int* idx = m->bidx + within * batch;
-    k_gather_rows<<<nblk((int64_t)batch * m->w[0], 256), 256, 0, m->stream>>>(m->tx, idx, batch, m->w[0], m->X[0]);
-    k_gather_rows<<<nblk((int64_t)batch * m->w[L], 256), 256, 0, m->stream>>>(m->ty, idx, batch, m->w[L], m->by);
-    rc = forward(m, batch);
-    if (rc == DG_OK) rc = mse(m, m->by, batch);
-    if (rc == DG_OK) e = cudaMemcpyAsync(d_losses + s, m->loss, sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
-    if (rc == DG_OK && e == cudaSuccess) rc = backward(m, batch);
+    if (use_fused(m)) {
+      rc = fused_forward<true>(m, m->tx, idx, batch, m->X[L]);
+      if (rc == DG_OK) rc = fused_backward(m, m->ty, idx, batch, d_losses + s);
+    } else {
+      k_gather_rows<<<nblk((int64_t)batch * m->w[0], 256), 256, 0, m->stream>>>(m->tx, idx, batch, m->w[0], m->X[0]);
+      k_gather_rows<<<nblk((int64_t)batch * m->w[L], 256), 256, 0, m->stream>>>(m->ty, idx, batch, m->w[L], m->by);
+      rc = forward(m, batch);
+      if (rc == DG_OK) rc = mse(m, m->by, batch);
+      if (rc == DG_OK) e = cudaMemcpyAsync(d_losses + s, m->loss, sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
+      if (rc == DG_OK && e == cudaSuccess) rc = backward(m, batch);
+    }
     if (rc != DG_OK || e != cudaSuccess) break;
     // cosine decay from lr to lr_final
     const double frac = n_steps > 1 ? (double)s / (double)(n_steps - 1) : 1.0;
     const double lrs = lr_final + 0.5 * (lr - lr_final) * (1.0 + std::cos(3.14159265358979323846 * frac));
     m->step += 1;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    k_adam<<<nblk(m->n_params, 256), 256, 0, m->stream>>>(m->p, m->g, m->m1, m->m2, m->n_params, (float)lrs, b1, b2,
-                                                          eps, c1, c2, (float)weight_decay);
-    rc = refresh_bf16(m);
+    if (m->fused) {
+      mlpf::k_adam_refresh<<<nblk(m->n_params, 256), 256, 0, m->stream>>>(
+          m->net, m->p, m->g, m->m1, m->m2, m->n_params, (float)lrs, b1, b2, eps, c1, c2, (float)weight_decay, m->wh,
+          m->wt, m->wb);
+    } else {
+      k_adam<<<nblk(m->n_params, 256), 256, 0, m->stream>>>(m->p, m->g, m->m1, m->m2, m->n_params, (float)lrs, b1, b2,
+                                                            eps, c1, c2, (float)weight_decay);
+      rc = refresh_bf16(m);
+    }
     if (e == cudaSuccess) e = cudaGetLastError();
   }
   if (e == cudaSuccess && rc == DG_OK && losses && n_steps > 0)
     e = cudaMemcpyAsync(losses, d_losses, n_steps * sizeof(double), cudaMemcpyDeviceToHost, m->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+  const cudaError_t es = cudaStreamSynchronize(m->stream);
+  if (e == cudaSuccess) e = es;
   cudaFree(d_losses);
   cudaFree(m->bidx);
   m->bidx = nullptr;

@@ -571,7 +571,7 @@ class Network:
         self._ck(_mlp_lib().dg_mlp_set_data(self.h, _fp(self._x), _fp(self._t), self._x.shape[0]), "dg_mlp_set_data")
 
     def set_tensor_cores(self, on):
-        """GEMMs on the tensor cores or on the CUDA cores (the default)."""
+        """The layers as single tcgen05 GEMMs, or the fused passes (the default)."""
         self._ck(_mlp_lib().dg_mlp_set_tensor_cores(self.h, 1 if on else 0), "dg_mlp_set_tensor_cores")
 
     @property
