@@ -248,7 +248,7 @@ int group_layouts(dg_batch* b) {
 
 int launch_steps(dg_batch* b, int64_t n_steps, cudaEvent_t* ev) {
   for (auto& g : b->groups) {
-    int64_t st[2] = {b->step, b->step};
+    int64_t st[3] = {b->step, b->step, b->step + n_steps};
     BCK(b, cudaMemcpyAsync(g.ctx->d_step, st, sizeof(st), cudaMemcpyHostToDevice, b->main));
   }
   for (int64_t i = 0; i < n_steps; ++i) {

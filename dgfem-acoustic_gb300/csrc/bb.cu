@@ -7,16 +7,15 @@
 #include <vector>
 
 #include "bb.cuh"
+#include "bb_inject.cuh"
 #include "stage_bb.cuh"
 
 namespace {
 
+using namespace dgk;
+
 constexpr int LW = 32;
 
-// Word strides of a tile's variables, coefficients and elements (BBCfg).
-struct Lay {
-  int sq, sn, se, tw;
-};
 Lay lay(const dg_ctx* c) {
   const int tw = c->nv * c->np * LW;
   return c->prec == DG_FP32 && c->dim == 3 ? Lay{1, 4 * LW, 4, tw} : Lay{c->np * LW, LW, 1, tw};
@@ -74,63 +73,10 @@ __global__ void __launch_bounds__(128) k_bb_to_ref(const T* __restrict__ in, dou
   }
 }
 
-// Source overwrite (src/solver.cpp:455-483) of elements given by
-// coefficients: one warp per element that holds source nodes. With S the
-// nodes that an active source covers and v their values, the element's
-// pressure becomes c + V^-1[:, S] (v - V[S, :] c): its nodal values are v at
-// S and unchanged elsewhere.
+// Source overwrite at the start of a run's step (bb_inject_block).
 template <typename T>
-__global__ void __launch_bounds__(128) k_inject_bb(T* u, const int64_t* __restrict__ elem,
-                                                   const int* __restrict__ eoff, int64_t ne,
-                                                   const int64_t* __restrict__ dof, const int* __restrict__ off,
-                                                   const int* __restrict__ ids, const double* __restrict__ val,
-                                                   int nsrc, int64_t nrows, const int64_t* step, int np, Lay l,
-                                                   const double* __restrict__ Vt, const double* __restrict__ Vit) {
-  __shared__ T sc[4][64], sr[4][64];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t i = blockIdx.x * 4ll + w;
-  if (i >= ne) return;
-  const int64_t s = step[0];
-  if (s < 0 || s >= nrows) return;
-  const double* row = val + s * nsrc;
-  const int64_t e = elem[i];
-  T* c = u + (e >> 5) * l.tw + (e & 31) * l.se;
-  for (int n = lane; n < np; n += 32) sc[w][n] = c[n * l.sn], sr[w][n] = (T)0;
-  __syncwarp();
-  for (int k = eoff[i] + lane; k < eoff[i + 1]; k += 32) {
-    double v = 0.0;
-    bool any = false;
-    for (int t = off[k]; t < off[k + 1]; ++t) {
-      const double x = row[ids[t]];
-      if (!isnan(x)) v = x, any = true;
-    }
-    if (any) {
-      const int n = (int)(dof[k] - e * np);
-      T r0 = (T)v, r1 = (T)0;
-#pragma unroll 4
-      for (int j = 0; j < np; ++j) {
-        const T p = (T)Vt[j * np + n] * sc[w][j];
-        if (j & 1)
-          r1 -= p;
-        else
-          r0 -= p;
-      }
-      sr[w][n] = r0 + r1;
-    }
-  }
-  __syncwarp();
-  for (int n = lane; n < np; n += 32) {
-    T a0 = (T)0, a1 = (T)0;
-#pragma unroll 4
-    for (int j = 0; j < np; ++j) {
-      const T p = (T)Vit[j * np + n] * sr[w][j];
-      if (j & 1)
-        a1 += p;
-      else
-        a0 += p;
-    }
-    c[n * l.sn] = sc[w][n] + (a0 + a1);
-  }
+__global__ void __launch_bounds__(kInjectThreads) k_inject_bb(const InjectArgs<T> a, const int64_t* step) {
+  bb_inject_block<T>(a, blockIdx.x, step[0]);
 }
 
 // Element means of p, p/c0^2 and v (src/Mesh.cpp:1196-1212) from the
@@ -249,18 +195,25 @@ cudaError_t bb_to_ref(dg_ctx* c, const void* in, double* ref) {
   return cudaGetLastError();
 }
 
+template <typename T>
+InjectArgs<T> bb_inject_args(const dg_ctx* c) {
+  InjectArgs<T> a{};
+  a.u = (T*)c->u, a.elem = c->d_src_elem, a.eoff = c->d_src_eoff, a.ne = c->n_src_elems;
+  a.dof = c->d_src_dof, a.off = c->d_src_off, a.ids = c->d_src_ids, a.val = c->d_srcval;
+  a.nsrc = c->n_src, a.nrows = c->srcval_steps, a.np = c->np, a.l = lay(c);
+  a.Vt = c->bb_dbl + c->bb_iden[0], a.Vit = c->bb_dbl + c->bb_iden[1];
+  return a;
+}
+template InjectArgs<float> bb_inject_args<float>(const dg_ctx*);
+template InjectArgs<double> bb_inject_args<double>(const dg_ctx*);
+
 cudaError_t bb_inject(dg_ctx* c) {
   if (c->n_src_elems == 0) return cudaSuccess;
-  const unsigned nb = (unsigned)((c->n_src_elems + 3) / 4);
-  const double *vt = c->bb_dbl + c->bb_iden[0], *vit = c->bb_dbl + c->bb_iden[1];
+  const unsigned nb = (unsigned)bb_inject_blocks(c->n_src_elems);
   if (c->prec == DG_FP32)
-    k_inject_bb<float><<<nb, 128, 0, c->stream>>>((float*)c->u, c->d_src_elem, c->d_src_eoff, c->n_src_elems,
-                                                  c->d_src_dof, c->d_src_off, c->d_src_ids, c->d_srcval, c->n_src,
-                                                  c->srcval_steps, c->d_step, c->np, lay(c), vt, vit);
+    k_inject_bb<float><<<nb, kInjectThreads, 0, c->stream>>>(bb_inject_args<float>(c), c->d_step);
   else
-    k_inject_bb<double><<<nb, 128, 0, c->stream>>>((double*)c->u, c->d_src_elem, c->d_src_eoff, c->n_src_elems,
-                                                   c->d_src_dof, c->d_src_off, c->d_src_ids, c->d_srcval, c->n_src,
-                                                   c->srcval_steps, c->d_step, c->np, lay(c), vt, vit);
+    k_inject_bb<double><<<nb, kInjectThreads, 0, c->stream>>>(bb_inject_args<double>(c), c->d_step);
   return cudaGetLastError();
 }
 

@@ -14,8 +14,10 @@
 #include <vector>
 
 #include "bb.cuh"
+#include "bb_inject.cuh"
 #include "ctx.h"
 #include "curved.cuh"
+#include "stage2.cuh"
 
 namespace {
 
@@ -78,6 +80,7 @@ __global__ void k_inject(T* up, const int64_t* dof, const int* off, const int* i
 // Block sizes of the finalize kernel: 256 threads when an observer holds
 // more node slots than the small block (one slot per thread), else 64.
 constexpr int kFinalizeThreads = 256, kFinalizeThreadsSmall = 64;
+static_assert(kFinalizeThreadsSmall >= dgk::kInjectThreads, "the source blocks' warps");
 
 // Block sums of five FP64 values per thread by a halving tree in shared
 // memory, each level with only the warps it needs (GB300's FP64 rate makes
@@ -98,86 +101,121 @@ __device__ __forceinline__ void block_sum5(double (&red)[5][NT], const double (&
   }
 }
 
-// Residuals (block 0) and observer IDW samples (then, per observer o, the
-// blocks bfirst[o] .. bfirst[o+1]-1 of the observer blocks, bmap giving each
-// block's observer; each block sums a strided share of the observer's node
-// slots) of the step just completed (src/solver.cpp:518-573). With more than
-// one block per observer, the blocks store partial sums and the observer's
-// last block to finish (counted with an atomic per observer) combines them in
-// block order: the result does not depend on the blocks' timing. Without
-// bmap every observer has one block.
+// What follows a step's last stage, in one launch: the residuals (block 0),
+// the observers' IDW samples of the step just completed (src/solver.cpp:518-573;
+// per observer o the blocks bfirst[o] .. bfirst[o+1]-1 of the observer blocks,
+// bmap giving each block's observer; each block sums a strided share of the
+// observer's slots), the source overwrite of the run's next step (the last
+// blocks, when inj.ne > 0), and the step counter, which the last block to have
+// read it increments. With more than one block per observer, the blocks store
+// partial sums and the observer's last block to finish (counted with an atomic
+// per observer) combines them in block order: the result does not depend on
+// the blocks' timing. Without bmap every observer has one block. The overwrite
+// shares a launch only with observers that read none of its elements.
+struct EndArgs {
+  const double* partials;
+  int nparts;
+  double inv_count;
+  double* res;
+  int64_t stride;
+  int nv;
+  const int64_t *odof, *ooff;
+  const double* ow;
+  double* obs;
+  int n_obs, obs_blocks;
+  const int *bmap, *bfirst;
+  double* obs_part;
+  unsigned* obs_cnt;
+  int64_t* step;  // [0] global step, [1] first step of the run, [2] one past its last step
+  unsigned* ticket;
+  int64_t cap;
+};
+
 template <typename T, int NT>
-__global__ void __launch_bounds__(NT)
-    k_finalize(const double* partials, int nparts, double inv_count, double* res, const T* u, int64_t stride, int nv,
-               const int64_t* odof, const int64_t* ooff, const double* ow, double* obs, int n_obs, const int* bmap,
-               const int* bfirst, double* obs_part, unsigned* obs_cnt, const int64_t* step, int64_t cap) {
+__global__ void __launch_bounds__(NT) k_step_end(const EndArgs a, const T* u, const dgk::InjectArgs<T> inj) {
   __shared__ double red[5][NT];
   __shared__ bool last;
-  int64_t slot = step[0] - step[1];
-  if (slot < 0 || slot >= cap) return;
+  dgk::grid_dependency_wait();
+  const int64_t s = a.step[0], slot = s - a.step[1], end = a.step[2];
   const int tid = threadIdx.x;
+  __syncthreads();  // the whole block has read the step
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(a.ticket, 1u) == gridDim.x - 1) {
+      *a.ticket = 0u;
+      a.step[0] = s + 1;
+    }
+  }
+  const bool in_cap = slot >= 0 && slot < a.cap;
   if (blockIdx.x == 0) {
+    if (!in_cap) return;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (int b = tid; b < nparts; b += NT)
-      for (int c = 0; c < 5; ++c) acc[c] += partials[b * 5 + c];
+    for (int b = tid; b < a.nparts; b += NT)
+      for (int c = 0; c < 5; ++c) acc[c] += a.partials[b * 5 + c];
     block_sum5<NT>(red, acc, tid);
-    if (tid < 5) res[slot * 5 + tid] = red[tid][0] * inv_count;
+    if (tid < 5) a.res[slot * 5 + tid] = red[tid][0] * a.inv_count;
     return;
   }
   const int ob = blockIdx.x - 1;
-  const int o = bmap ? bmap[ob] : ob;
-  if (o >= n_obs) return;
-  const int first = bmap ? bfirst[o] : ob, nb = bmap ? bfirst[o + 1] - first : 1, part = ob - first;
+  if (ob >= a.obs_blocks) {
+    if (s + 1 < end) dgk::bb_inject_block<T>(inj, ob - a.obs_blocks, s + 1);
+    return;
+  }
+  if (!in_cap) return;
+  const int o = a.bmap ? a.bmap[ob] : ob;
+  if (o >= a.n_obs) return;
+  const int first = a.bmap ? a.bfirst[o] : ob, nb = a.bmap ? a.bfirst[o + 1] - first : 1, part = ob - first;
   double acc[5] = {0, 0, 0, 0, 0};  // p, vx, vy, vz, w
   const int64_t step_k = (int64_t)NT * nb;
 #pragma unroll 4
-  for (int64_t k = ooff[o] + (int64_t)part * NT + tid; k < ooff[o + 1]; k += step_k) {
-    double w = ow[k];
-    int64_t d = odof[k];
+  for (int64_t k = a.ooff[o] + (int64_t)part * NT + tid; k < a.ooff[o + 1]; k += step_k) {
+    double w = a.ow[k];
+    int64_t d = a.odof[k];
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (q < nv) acc[q] += (double)u[q * stride + d] * w;
+      if (q < a.nv) acc[q] += (double)u[q * a.stride + d] * w;
     acc[4] += w;
   }
   block_sum5<NT>(red, acc, tid);
   if (nb == 1) {
-    if (tid < 4) obs[(slot * n_obs + o) * 4 + tid] = red[tid][0] / red[4][0];
+    if (tid < 4) a.obs[(slot * a.n_obs + o) * 4 + tid] = red[tid][0] / red[4][0];
     return;
   }
   if (tid < 5) {
-    obs_part[(int64_t)ob * 5 + tid] = red[tid][0];
+    a.obs_part[(int64_t)ob * 5 + tid] = red[tid][0];
     __threadfence();
   }
   __syncthreads();
-  if (tid == 0) last = atomicAdd(obs_cnt + o, 1u) == (unsigned)(nb - 1);
+  if (tid == 0) last = atomicAdd(a.obs_cnt + o, 1u) == (unsigned)(nb - 1);
   __syncthreads();
   if (!last) return;
   __threadfence();
   if (tid < 4) {
     double v = 0.0, w = 0.0;
     for (int b = first; b < first + nb; ++b) {
-      v += __ldcg(obs_part + (int64_t)b * 5 + tid);
-      w += __ldcg(obs_part + (int64_t)b * 5 + 4);
+      v += __ldcg(a.obs_part + (int64_t)b * 5 + tid);
+      w += __ldcg(a.obs_part + (int64_t)b * 5 + 4);
     }
-    obs[(slot * n_obs + o) * 4 + tid] = v / w;
+    a.obs[(slot * a.n_obs + o) * 4 + tid] = v / w;
   }
-  if (tid == 0) obs_cnt[o] = 0u;  // for the next step
+  if (tid == 0) a.obs_cnt[o] = 0u;  // for the next step
 }
 
-__global__ void k_advance(int64_t* step) { step[0] += 1; }
-
-template <typename T, int NT>
-void launch_finalize_nt(dg_ctx* c, int nparts, double inv_count, int64_t stride) {
-  k_finalize<T, NT><<<1 + c->obs_blocks, NT, 0, c->stream>>>(
-      c->partials, nparts, inv_count, c->d_res, (const T*)c->u, stride, c->nv, c->d_obs_dof, c->d_obs_off, c->d_obs_w,
-      c->d_obs, c->n_obs, c->d_obs_bmap, c->d_obs_bfirst, c->d_obs_part, c->d_obs_cnt, c->d_step, c->out_cap);
-}
 template <typename T>
-void launch_finalize(dg_ctx* c, int nparts, double inv_count, int64_t stride) {
+cudaError_t launch_step_end(dg_ctx* c, int nparts, double inv_count, int64_t stride, bool inject, bool pdl) {
+  EndArgs a{};
+  a.partials = c->partials, a.nparts = nparts, a.inv_count = inv_count, a.res = c->d_res, a.stride = stride, a.nv = c->nv;
+  a.odof = c->d_obs_dof, a.ooff = c->d_obs_off, a.ow = c->d_obs_w, a.obs = c->d_obs, a.n_obs = c->n_obs;
+  a.obs_blocks = c->obs_blocks, a.bmap = c->d_obs_bmap, a.bfirst = c->d_obs_bfirst, a.obs_part = c->d_obs_part;
+  a.obs_cnt = c->d_obs_cnt, a.step = c->d_step, a.ticket = c->d_ticket, a.cap = c->out_cap;
+  dgk::InjectArgs<T> inj{};
+  if (inject) inj = dgc::bb_inject_args<T>(c);
+  const dim3 grid((unsigned)(1 + c->obs_blocks + (inject ? dgk::bb_inject_blocks(inj.ne) : 0)));
   if (c->obs_small)
-    launch_finalize_nt<T, kFinalizeThreadsSmall>(c, nparts, inv_count, stride);
-  else
-    launch_finalize_nt<T, kFinalizeThreads>(c, nparts, inv_count, stride);
+    return dgk::launch_kernel(k_step_end<T, kFinalizeThreadsSmall>, grid, kFinalizeThreadsSmall, 0, c->stream, pdl, a,
+                              (const T*)c->u, inj);
+  return dgk::launch_kernel(k_step_end<T, kFinalizeThreads>, grid, kFinalizeThreads, 0, c->stream, pdl, a,
+                            (const T*)c->u, inj);
 }
 
 // Euler1 commit: u = y (computed as u + k by the stage kernel) with residuals.
@@ -245,6 +283,14 @@ int fail(dg_ctx* c, int code, const std::string& msg) {
     if (e_ != cudaSuccess) return fail((c), DG_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e_)); \
   } while (0)
 
+// Steps of the longer step graph.
+constexpr int kGraphSteps = 8;
+
+void drop_graphs(dg_ctx* c) {
+  if (c->graph) cudaGraphExecDestroy(c->graph), c->graph = nullptr;
+  if (c->graph_n) cudaGraphExecDestroy(c->graph_n), c->graph_n = nullptr;
+}
+
 template <typename T>
 dgk::StageArgs<T> stage_args(dg_ctx* c, int stage, const T* y_in, T* y_out, T* k_out, double dt) {
   dgk::StageArgs<T> a{};
@@ -272,6 +318,7 @@ dgk::StageArgs<T> stage_args(dg_ctx* c, int stage, const T* y_in, T* y_out, T* k
   a.ntiles = c->variant >= 0 ? (int)(c->Epad / c->s2.et) : (int)c->ntiles;
   a.stage = stage;
   a.wait_limit = c->wait_limit;
+  a.pdl = c->pdl ? 1 : 0;
   a.dt = dt;
   a.c0sq = c->c0sq;
   a.ph = c->ph;
@@ -351,36 +398,48 @@ cudaError_t enqueue_inject(dg_ctx* c) {
   return cudaSuccess;
 }
 
-// Residual means (from nparts rows of stage-4 partial sums) and observer
-// samples after a step, then the step counter (on c->stream).
-cudaError_t enqueue_finalize(dg_ctx* c, int nparts) {
+// Residual means (from nparts rows of stage-4 partial sums), observer samples
+// and the step counter after a step, with inject also the next step's source
+// overwrite (on c->stream; pdl: directly after a kernel).
+cudaError_t enqueue_finalize(dg_ctx* c, int nparts, bool inject = false, bool pdl = false) {
   const int64_t stride = c->bb ? dgc::bb_var_stride(c) : c->Epad * c->np;
   double inv_count = 1.0 / (double)(c->E * c->np);
   // an observer with thousands of node slots is summed by several blocks:
   // the sums are FP64, whose rate per SM on GB300 bounds a single block
-  if (c->prec == DG_FP32)
-    launch_finalize<float>(c, nparts, inv_count, stride);
-  else
-    launch_finalize<double>(c, nparts, inv_count, stride);
-  cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
-  k_advance<<<1, 1, 0, c->stream>>>(c->d_step);
-  return cudaGetLastError();
+  return c->prec == DG_FP32 ? launch_step_end<float>(c, nparts, inv_count, stride, inject, pdl)
+                            : launch_step_end<double>(c, nparts, inv_count, stride, inject, pdl);
 }
 
+// Whether a step's end can also overwrite the next step's sources: the state
+// is in coefficients and no observer reads an element that holds source nodes.
+bool chained(const dg_ctx* c) { return c->bb && c->n_src_elems > 0 && c->src_obs_apart; }
+
 // One time step on c->stream. kind 0: RK4, 1: Euler1. ev (optional, 8
-// events) brackets the stage launches for kernel timing.
-cudaError_t enqueue_step(dg_ctx* c, int kind, double dt, cudaEvent_t* ev) {
+// events) brackets the stage launches for kernel timing. chain: the step's
+// sources are in place already (see chained) and its end places the next
+// step's; follows: the kernel before it on the stream is another step's end.
+cudaError_t enqueue_step(dg_ctx* c, int kind, double dt, cudaEvent_t* ev, bool chain = false, bool follows = false) {
   cudaError_t err;
   const int64_t stride = c->Epad * c->np;
-  if ((err = enqueue_inject(c)) != cudaSuccess) return err;
+  if (!chain && (err = enqueue_inject(c)) != cudaSuccess) return err;
+  // Programmatic dependents (only the kernels of stage_bb.cuh wait for their
+  // predecessor themselves): the step's end always, a stage only while its
+  // tiles have an SM each. Blocks that start while the stage before drains fill
+  // the SMs as those come free, consecutive ones on one SM, and with more tiles
+  // than SMs the blocks that take one tile more meet there: 196,608 tetrahedra
+  // of order 3, FP32, 0.36 against 0.33 ms per step; 4050 triangles of order 3,
+  // FP64, 57 against 61 us.
+  const bool pdl = c->bb && !ev, pdl_stage = pdl && c->Epad / 32 <= c->num_sms;
   int nparts = c->variant >= 0 ? c->grid2 : c->grid;
   if (kind == 0) {
     const void* in[4] = {c->u, c->y0, c->y1, c->y0};
     void* out[4] = {c->y0, c->y1, c->y0, nullptr};
     for (int s = 0; s < 4; ++s) {
       if (ev) cudaEventRecord(ev[2 * s], c->stream);
-      if ((err = launch_stage(c, s + 1, in[s], out[s], nullptr, dt)) != cudaSuccess) return err;
+      c->pdl = pdl_stage && (s > 0 || (chain && follows));
+      err = launch_stage(c, s + 1, in[s], out[s], nullptr, dt);
+      c->pdl = false;
+      if (err != cudaSuccess) return err;
       if (ev) cudaEventRecord(ev[2 * s + 1], c->stream);
     }
   } else {
@@ -390,7 +449,7 @@ cudaError_t enqueue_step(dg_ctx* c, int kind, double dt, cudaEvent_t* ev) {
     if (c->bb) {
       // the stage kernel summed the residuals
       err = cudaMemcpyAsync(c->u, c->y0, (size_t)c->nv * stride * c->tsize, cudaMemcpyDeviceToDevice, c->stream);
-      return err != cudaSuccess ? err : enqueue_finalize(c, nparts);
+      return err != cudaSuccess ? err : enqueue_finalize(c, nparts, chain);
     }
     const int cb = 2 * c->num_sms;
     nparts = cb;
@@ -403,7 +462,7 @@ cudaError_t enqueue_step(dg_ctx* c, int kind, double dt, cudaEvent_t* ev) {
                                                         n, stride, c->nv, c->c0sq, c->partials);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
   }
-  return enqueue_finalize(c, nparts);
+  return enqueue_finalize(c, nparts, chain, pdl && kind == 0);
 }
 
 int ensure_out_cap(dg_ctx* c, int64_t n) {
@@ -415,30 +474,43 @@ int ensure_out_cap(dg_ctx* c, int64_t n) {
   CK(c, cudaMalloc(&c->d_res, cap * 5 * sizeof(double)));
   CK(c, cudaMalloc(&c->d_obs, cap * std::max(1, c->n_obs) * 4 * sizeof(double)));
   c->out_cap = cap;
-  if (c->graph) {
-    cudaGraphExecDestroy(c->graph);
-    c->graph = nullptr;
-  }
+  drop_graphs(c);
   return DG_OK;
 }
 
-int build_graph(dg_ctx* c, int kind, double dt) {
-  if (c->graph && c->graph_dt == dt && c->graph_kind == kind) return DG_OK;
-  if (c->graph) {
-    cudaGraphExecDestroy(c->graph);
-    c->graph = nullptr;
-  }
+// The step graphs of (kind, dt): one step, and kGraphSteps of them where the
+// run is that long (fewer graph launches, and the kernels of one step follow
+// those of the step before it as programmatic dependents).
+int build_graph(dg_ctx* c, int kind, double dt, int steps) {
+  if (c->graph_dt != dt || c->graph_kind != kind) drop_graphs(c);
+  cudaGraphExec_t& exec = steps == 1 ? c->graph : c->graph_n;
+  if (exec) return DG_OK;
   cudaGraph_t g = nullptr;
+  const bool chain = chained(c);
   CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  cudaError_t err = enqueue_step(c, kind, dt, nullptr);
+  cudaError_t err = cudaSuccess;
+  for (int i = 0; i < steps && err == cudaSuccess; ++i) err = enqueue_step(c, kind, dt, nullptr, chain, i > 0);
   cudaError_t err2 = cudaStreamEndCapture(c->stream, &g);
-  if (err != cudaSuccess) return fail(c, DG_ERR_CUDA, std::string("CUDA (capture): ") + cudaGetErrorString(err));
+  if (err != cudaSuccess) {
+    if (g) cudaGraphDestroy(g);
+    return fail(c, DG_ERR_CUDA, std::string("CUDA (capture): ") + cudaGetErrorString(err));
+  }
   CK(c, err2);
-  err = cudaGraphInstantiate(&c->graph, g, 0);
+  err = cudaGraphInstantiate(&exec, g, 0);
   cudaGraphDestroy(g);
+  if (err != cudaSuccess) exec = nullptr;
   CK(c, err);
   c->graph_dt = dt;
   c->graph_kind = kind;
+  return DG_OK;
+}
+
+// Step counters of a run of n_steps on the device, and its first step's
+// sources where the steps' ends place the others.
+int begin_run(dg_ctx* c, int64_t n_steps) {
+  int64_t st[3] = {c->step, c->step, c->step + n_steps};
+  CK(c, cudaMemcpyAsync(c->d_step, st, sizeof(st), cudaMemcpyHostToDevice, c->stream));
+  if (chained(c)) CK(c, enqueue_inject(c));
   return DG_OK;
 }
 
@@ -448,11 +520,13 @@ int run_steps(dg_ctx* c, int kind, int64_t n_steps, double dt, double* residuals
   if (n_steps == 0) return DG_OK;
   int rc = ensure_out_cap(c, n_steps);
   if (rc) return rc;
-  rc = build_graph(c, kind, dt);
+  const int64_t many = n_steps / kGraphSteps, rest = n_steps % kGraphSteps;
+  if (many > 0) rc = build_graph(c, kind, dt, kGraphSteps);
+  if (!rc && rest > 0) rc = build_graph(c, kind, dt, 1);
+  if (!rc) rc = begin_run(c, n_steps);
   if (rc) return rc;
-  int64_t st[2] = {c->step, c->step};
-  CK(c, cudaMemcpyAsync(c->d_step, st, sizeof(st), cudaMemcpyHostToDevice, c->stream));
-  for (int64_t i = 0; i < n_steps; ++i) CK(c, cudaGraphLaunch(c->graph, c->stream));
+  for (int64_t i = 0; i < many; ++i) CK(c, cudaGraphLaunch(c->graph_n, c->stream));
+  for (int64_t i = 0; i < rest; ++i) CK(c, cudaGraphLaunch(c->graph, c->stream));
   std::vector<double> res(n_steps * 5);
   CK(c, cudaMemcpyAsync(res.data(), c->d_res, n_steps * 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   if (obs && c->n_obs > 0)
@@ -547,7 +621,7 @@ bool set_variant(dg_ctx* c, int v) {
   c->variant = v;
   c->s2 = si;
   c->grid2 = (int)std::min<int64_t>(c->Epad / si.et, (int64_t)si.blocks_per_sm * c->num_sms);
-  if (c->graph) cudaGraphExecDestroy(c->graph), c->graph = nullptr;
+  drop_graphs(c);
   return true;
 }
 
@@ -565,7 +639,7 @@ int upload_observers(dg_ctx* c) {
   const int n_obs = c->n_obs;
   c->obs_blocks = n_obs;
   c->obs_small = true;
-  if (c->graph) cudaGraphExecDestroy(c->graph), c->graph = nullptr;
+  drop_graphs(c);
   if (n_obs == 0) return DG_OK;
   std::vector<int64_t> off, dof;
   std::vector<double> w;
@@ -1078,8 +1152,10 @@ int dgc::create_ctx(const dg_mesh_desc* mesh, const dg_phys* phys, int precision
   if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->partials, c->max_grid * 5 * sizeof(double));
   if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-  if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_step, 2 * sizeof(int64_t));
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_step, 0, 2 * sizeof(int64_t), c->stream);
+  if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_step, 3 * sizeof(int64_t));
+  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_step, 0, 3 * sizeof(int64_t), c->stream);
+  if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_ticket, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_ticket, 0, sizeof(unsigned), c->stream);
   cudaEventRecord(t1, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
@@ -1122,7 +1198,7 @@ extern "C" {
 
 int dg_destroy(dg_ctx* c) {
   if (!c) return DG_OK;
-  if (c->graph) cudaGraphExecDestroy(c->graph);
+  drop_graphs(c);
   for (void* p : c->allocs) cudaFree(p);
   void* extra[] = {c->d_res, c->d_obs, c->d_src_dof, c->d_src_off, c->d_src_ids, c->d_srcval, c->d_src_elem, c->d_src_eoff,
                    c->d_obs_dof, c->d_obs_off, c->d_obs_w, c->d_obs_part, c->d_obs_cnt, c->d_obs_bmap,
@@ -1171,6 +1247,16 @@ int dg_get_state(dg_ctx* c, double* u) {
   return DG_OK;
 }
 
+// Whether no observer reads an element that holds source nodes.
+static void note_overlap(dg_ctx* c) {
+  c->src_obs_apart = true;
+  for (int64_t d : c->obs_dof)
+    if (std::binary_search(c->src_elems.begin(), c->src_elems.end(), d / c->np)) {
+      c->src_obs_apart = false;
+      return;
+    }
+}
+
 int dg_set_sources(dg_ctx* c, int n_src, const int64_t* offsets, const int64_t* dofs) {
   if (!c || n_src < 0 || (n_src > 0 && !offsets)) return DG_ERR_ARG;
   // sources may cover no dof at all (a radius with no node inside): then
@@ -1201,9 +1287,10 @@ int dg_set_sources(dg_ctx* c, int n_src, const int64_t* offsets, const int64_t* 
     if (p) cudaFree(p);
   c->d_src_dof = nullptr, c->d_src_off = nullptr, c->d_src_ids = nullptr;
   c->d_src_elem = nullptr, c->d_src_eoff = nullptr, c->n_src_elems = 0;
+  c->src_elems.clear();
   c->n_src = n_src;
   c->n_src_dofs = (int64_t)hd.size();
-  if (c->graph) cudaGraphExecDestroy(c->graph), c->graph = nullptr;
+  drop_graphs(c);
   if (hd.empty()) return DG_OK;
   CK(c, cudaMalloc(&c->d_src_dof, hd.size() * sizeof(int64_t)));
   CK(c, cudaMalloc(&c->d_src_off, ho.size() * sizeof(int)));
@@ -1226,6 +1313,8 @@ int dg_set_sources(dg_ctx* c, int n_src, const int64_t* offsets, const int64_t* 
   CK(c, cudaMemcpyAsync(c->d_src_eoff, heo.data(), heo.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
   c->n_src_elems = (int64_t)he.size();
+  c->src_elems.swap(he);
+  note_overlap(c);
   return DG_OK;
 }
 
@@ -1233,7 +1322,7 @@ int dg_set_source_values(dg_ctx* c, int64_t n_steps, const double* values) {
   if (!c || n_steps < 0 || (n_steps > 0 && c->n_src > 0 && !values)) return DG_ERR_ARG;
   if (c->d_srcval) cudaFree(c->d_srcval), c->d_srcval = nullptr;
   c->srcval_steps = 0;
-  if (c->graph) cudaGraphExecDestroy(c->graph), c->graph = nullptr;
+  drop_graphs(c);
   if (n_steps == 0 || c->n_src == 0) return DG_OK;
   CK(c, cudaMalloc(&c->d_srcval, n_steps * c->n_src * sizeof(double)));
   CK(c, cudaMemcpyAsync(c->d_srcval, values, n_steps * c->n_src * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -1261,6 +1350,7 @@ int dg_set_observers(dg_ctx* c, int n_obs, const int64_t* offsets, const int64_t
   if (c->d_obs) cudaFree(c->d_obs), c->d_obs = nullptr;
   if (c->d_res) cudaFree(c->d_res), c->d_res = nullptr;
   c->out_cap = 0;
+  note_overlap(c);
   return upload_observers(c);
 }
 
@@ -1409,10 +1499,7 @@ int dg_set_wait_limit(dg_ctx* c, int rounds) {
   c->wait_limit = rounds;
   // the per-step graph holds the kernel arguments: captured again on the
   // next run
-  if (c->graph) {
-    cudaGraphExecDestroy(c->graph);
-    c->graph = nullptr;
-  }
+  drop_graphs(c);
   return DG_OK;
 }
 
@@ -1420,13 +1507,16 @@ int dg_bench_steps(dg_ctx* c, int64_t n_steps, double dt, int64_t flush_bytes, d
   if (!c || n_steps <= 0 || !(dt > 0)) return DG_ERR_ARG;
   int rc = ensure_out_cap(c, n_steps);
   if (rc) return rc;
-  rc = build_graph(c, 0, dt);
+  rc = build_graph(c, 0, dt, 1);
   if (rc) return rc;
   unsigned* flush = nullptr;
   int64_t nflush = flush_bytes / 4;
   if (nflush > 0) CK(c, cudaMalloc(&flush, nflush * 4));
-  int64_t st[2] = {c->step, c->step};
-  CK(c, cudaMemcpyAsync(c->d_step, st, sizeof(st), cudaMemcpyHostToDevice, c->stream));
+  rc = begin_run(c, n_steps);
+  if (rc) {
+    if (flush) cudaFree(flush);
+    return rc;
+  }
   std::vector<cudaEvent_t> ev(2 * n_steps);
   for (auto& x : ev) cudaEventCreate(&x);
   for (int64_t i = 0; i < n_steps; ++i) {
@@ -1448,7 +1538,7 @@ int dg_bench_steps(dg_ctx* c, int64_t n_steps, double dt, int64_t flush_bytes, d
     // second pass without the graph: events around each stage launch
     std::vector<cudaEvent_t> se(8 * n_steps);
     for (auto& x : se) cudaEventCreate(&x);
-    st[0] = st[1] = c->step;
+    const int64_t st[3] = {c->step, c->step, c->step + n_steps};
     CK(c, cudaMemcpyAsync(c->d_step, st, sizeof(st), cudaMemcpyHostToDevice, c->stream));
     for (int64_t i = 0; i < n_steps; ++i) {
       if (flush) k_flush<<<2 * c->num_sms, 512, 0, c->stream>>>(flush, nflush, (unsigned)i);

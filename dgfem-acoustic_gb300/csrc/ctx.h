@@ -47,7 +47,8 @@ struct dg_ctx {
   int* d_perm = nullptr;       // [np] mesh local -> internal
   double* d_ref = nullptr;     // [4][E*np] staging for reference-layout I/O
   double* partials = nullptr;  // [grid][5]
-  int64_t* d_step = nullptr;   // [0] global step, [1] first step of the current run
+  int64_t* d_step = nullptr;   // [0] global step, [1] first step of the current run, [2] one past its last
+  unsigned* d_ticket = nullptr;  // blocks of the step-end kernel that have read the step
   double* d_res = nullptr;     // [out_cap][5]
   double* d_obs = nullptr;     // [out_cap][n_obs][4]
   int64_t out_cap = 0;
@@ -105,11 +106,14 @@ struct dg_ctx {
   int64_t n_src_elems = 0;
   int64_t* d_src_elem = nullptr;
   int* d_src_eoff = nullptr;
+  std::vector<int64_t> src_elems;  // the same elements, ascending
+  bool src_obs_apart = true;       // no observer reads one of them
   // observers as given (internal node slots): the device lists depend on bb
   std::vector<int64_t> obs_off, obs_dof;
   std::vector<double> obs_w;
   // per-step graph
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph = nullptr, graph_n = nullptr;  // one step, kGraphSteps steps
+  bool pdl = false;  // the next stage launch is a programmatic dependent of the kernel before it
   double graph_dt = 0.0;
   int graph_kind = -1;  // 0 = RK4, 1 = Euler
   // bookkeeping

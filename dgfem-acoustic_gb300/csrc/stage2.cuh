@@ -57,6 +57,28 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// Programmatic dependent launch: waits until the kernels before this one in
+// the stream have completed (no effect when it was launched without the
+// attribute), then lets the next kernel's blocks start their own prologue.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launch of kfn; with pdl its blocks may start while the kernel before it in
+// the stream (which must be a kernel) drains: the kernel calls
+// grid_dependency_wait before it reads anything that one writes.
+template <typename... KA, typename... A>
+cudaError_t launch_kernel(void (*kfn)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool pdl, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = dim3((unsigned)threads), cfg.dynamicSmemBytes = smem, cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at, cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kfn, static_cast<KA>(args)...);
+}
+
 // Bounded wait for the phase with the given parity: at most `limit` polling
 // rounds (none when limit <= 0); false on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int limit = kWaitRounds) {

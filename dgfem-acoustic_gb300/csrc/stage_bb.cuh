@@ -326,6 +326,33 @@ __device__ __forceinline__ T bb_nodal_square(const T (&d)[C::NP]) {
   return sum;
 }
 
+// Residual sum of a thread's variable. FP32 squares overflow from 1.8e19 on, far
+// below the largest finite state: an element whose sum does is summed again
+// with its values scaled by 2^-64, into an FP64 remainder, so that the sum is
+// non-finite only when the state is.
+template <typename T>
+struct BBRes {
+  T s = (T)0;
+  double big = 0.0;
+  template <class C>
+  __device__ __forceinline__ void add(T (&d)[C::NP]) {
+    const T v = bb_nodal_square<C>(d), t = s + v;
+    if constexpr (sizeof(T) == 8) {
+      s = t;
+    } else {
+      if (t <= 3.4028234e38f) {
+        s = t;
+        return;
+      }
+#pragma unroll
+      for (int n = 0; n < C::NP; ++n) d[n] *= 5.421010862427522e-20f;  // 2^-64
+      big += (double)s + (double)bb_nodal_square<C>(d) * 3.402823669209385e38;  // 2^128
+      s = 0.f;
+    }
+  }
+  __device__ __forceinline__ double get() const { return (double)s + big; }
+};
+
 // RK operands of CH coefficients of this thread: loaded together (the first
 // group before the lift, so that its latency overlaps it), then combined with
 // dt*L and stored. In stages 4 and 5 out becomes the residual's difference.
@@ -409,7 +436,7 @@ __device__ __forceinline__ T bb_dt(const StageArgs<T>& a) {
 // by every thread once the tile's stage input is no longer read.
 template <class C, typename T, class Free>
 __device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, const T* y, const T* g, const int* gi,
-                                        const int* sFm, const unsigned char* sNb, T* sN, int lane, int role, T& racc,
+                                        const int* sFm, const unsigned char* sNb, T* sN, int lane, int role, BBRes<T>& racc,
                                         Free&& free_inputs) {
   constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, NV = C::NV, LW = C::LW, D = C::D;
   const T rhoc2 = bb_rhoc2<T>(a), inv_rho0 = bb_inv_rho0<T>(a);
@@ -512,7 +539,7 @@ __device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, con
     if (n0 > 0) ops.load(a, base, n0);
     ops.update(a, base, n0, dte, out);
   }
-  if (a.stage >= 4) racc += bb_nodal_square<C>(out);
+  if (a.stage >= 4) racc.template add<C>(out);
 }
 
 // One tile in the Q4 layout (FP32, 3-D). The flux phase is bb_tile's (a warp
@@ -527,7 +554,7 @@ __device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, con
 template <class C, class Free>
 __device__ __forceinline__ void bb_tile_q4(const StageArgs<float>& a, int64_t tile, const float* y, const float* g,
                                            const int* gi, const int* sFm, const unsigned char* sNb, float* sN, int tid,
-                                           int role, float& racc, Free&& free_inputs) {
+                                           int role, BBRes<float>& racc, Free&& free_inputs) {
   constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, LW = C::LW, D = C::D, P = C::P, SN = C::SN;
   const float rhoc2 = a.f_rhoc2, inv_rho0 = a.f_inv_rho0;
   const int lane = tid & 31;
@@ -631,7 +658,7 @@ __device__ __forceinline__ void bb_tile_q4(const StageArgs<float>& a, int64_t ti
     if (n0 > 0) ops.load(a, base, n0);
     ops.update(a, base, n0, dte, out);
   }
-  if (a.stage >= 4) racc += bb_nodal_square<C>(out);
+  if (a.stage >= 4) racc.template add<C>(out);
 }
 
 // Face tables in shared memory: element word offset of each face node, and
@@ -662,27 +689,33 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB, GA>::NT, MINB) stag
   const int role = ((tid >> 5) + blockIdx.x) % C::NV;
   const int nepi = a.stage == 1 || a.stage == 5 ? 1 : a.stage == 2 || a.stage == 3 ? 2 : a.stage == 4 ? 3 : 0;
 
-  auto issue = [&](int64_t tile, int b) {
+  auto issue_geometry = [&](int64_t tile, int b) {
     mbar_expect_tx(&bar[b], C::YB + C::GB + C::IB);
-    tma_load_1d(sY + (size_t)b * C::TW, a.y_in + tile * C::TW, C::YB, &bar[b]);
     tma_load_1d(sGF + (size_t)b * C::GW * C::LW, a.bbF + tile * C::GW * C::LW, C::GB, &bar[b]);
     tma_load_1d(sGI + (size_t)b * C::GI * C::LW, a.bbI + tile * C::GI * C::LW, C::IB, &bar[b]);
+  };
+  auto issue_state = [&](int64_t tile, int b) {
+    tma_load_1d(sY + (size_t)b * C::TW, a.y_in + tile * C::TW, C::YB, &bar[b]);
     // the tile's RK operands towards L2
     if (nepi >= 1 && a.u != a.y_in) prefetch_l2(a.u + tile * C::TW, C::YB);
     if (nepi >= 2) prefetch_l2(a.acc + tile * C::TW, C::YB);
     if (nepi >= 3) prefetch_l2(a.snap + tile * C::TW, C::YB);
   };
+  auto issue = [&](int64_t tile, int b) { issue_geometry(tile, b), issue_state(tile, b); };
 
   if (tid == 0) {
 #pragma unroll
     for (int b = 0; b < NBUF; ++b) mbar_init(&bar[b], 1);
     fence_mbar_init();
   }
+  // what no kernel before this one writes is fetched while they drain
+  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue_geometry(blockIdx.x, 0);
   bb_load_tables<C>(a, sFm, sNb, tid, C::NT);
+  grid_dependency_wait();
   __syncthreads();
-  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue(blockIdx.x, 0);
+  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue_state(blockIdx.x, 0);
 
-  T racc = (T)0;
+  BBRes<T> racc;
   bool ok = true;
   int it = 0;
   for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ++it) {
@@ -717,7 +750,7 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB, GA>::NT, MINB) stag
   if (a.stage >= 4) {
     // block sums per variable: a warp's lanes are one variable's (Q4: each
     // variable's are every fourth lane)
-    double v = (double)racc;
+    double v = racc.get();
 #pragma unroll
     for (int off = 16; off >= (C::Q4 ? 4 : 1); off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
     if constexpr (C::Q4) {
@@ -758,8 +791,8 @@ struct StageBB {
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    stage_bb_kernel<T, D, P, NBUF, MINB, GA><<<grid, C::NT, C::bytes, s>>>(a, err);
-    return cudaGetLastError();
+    return launch_kernel(stage_bb_kernel<T, D, P, NBUF, MINB, GA>, dim3((unsigned)grid), C::NT, C::bytes, s, a.pdl != 0,
+                         a, err);
   }
   static int blocks_per_sm() {
     if (set_attrs() != cudaSuccess) {

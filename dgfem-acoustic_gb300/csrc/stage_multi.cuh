@@ -71,7 +71,7 @@ __device__ __forceinline__ void multi_issue_tile(const StageArgs<float>& a, int6
 template <class C>
 __device__ __forceinline__ void multi_run_tile(const StageArgs<float>& a, int tile, unsigned char* slot, float* sN,
                                                const int* sFm, const unsigned char* sNb, int lane, int role,
-                                               float& racc) {
+                                               BBRes<float>& racc) {
   bb_tile<C, float>(a, tile, reinterpret_cast<const float*>(slot) + lane,
                     reinterpret_cast<const float*>(slot + C::YB) + lane,
                     reinterpret_cast<const int*>(slot + C::YB + C::GB) + lane, sFm, sNb, sN, lane, role, racc, []() {});
@@ -126,11 +126,11 @@ __global__ void __launch_bounds__(kMultiNT, kMultiMinBlocks) stage_multi_kernel(
   // rg; a block's items come in order after order, so each order's row is
   // written once, when the block moves on to the next order or finishes
   // (orders bit-set in wrote)
-  float racc = 0.f;
+  BBRes<float> racc;
   int rg = -1;
   unsigned wrote = 0;
   auto put_row = [&](int g, bool zero) {
-    double v = zero ? 0.0 : (double)racc;
+    double v = zero ? 0.0 : racc.get();
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
     if (lane == 0) sRed[role] = v;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kMultiNT, kMultiMinBlocks) stage_multi_kernel(
           tid == 0 ? sRed[0] : tid == 1 ? sRed[0] / c4 : tid < 4 ? sRed[tid - 1] : 0.0;
     }
     __syncthreads();
-    racc = 0.f;
+    racc = BBRes<float>();
     wrote |= 1u << g;
   };
   bool ok = true;

@@ -144,3 +144,62 @@ def test_state_and_snapshot_follow_a_change_of_kernel(pkg, dim, p):
     got = run([BB, -1, BB])
     for a, b, tol in zip(got, ref, (1e-12, 1e-10, 1e-11)):
         assert rel_l2(a, b) <= tol
+
+
+@pytest.mark.parametrize("dim,p,prec", [(2, 1, "fp64"), (2, 3, "fp32"), (3, 2, "fp64"), (3, 3, "fp32")])
+@pytest.mark.parametrize("chunks", [[21], [1, 7, 8, 5], [3] * 7])
+def test_sources_apart_from_observers_in_any_split_of_a_run(pkg, oracle, dim, p, prec, chunks):
+    """Where no observer reads a source's element, a step's end also places
+    the next step's sources; runs of one to 21 steps (around the 8 steps of
+    the longer step graph) follow the oracle, step index and source rows
+    included."""
+    mesh = _sized(pkg, dim, p, 6 if dim == 2 else (3, 3, 3))
+    ph = _phys(dim)
+    half = 5.0 if dim == 2 else 1.0
+    dt, nsteps = (2e-4 if dim == 2 else 1e-4), sum(chunks)
+    src = [-0.7 * half, -0.6 * half, -0.5 * half if dim == 3 else 0.0, 0.25 * half, 1.0, 60.0, 0.3, 1.0]
+    obs = [(0.6 * half, 0.6 * half, 0.6 * half if dim == 3 else 0.0, 0.3 * half)]
+    P = oracle.Problem(mesh, t_start=0.0, t_end=(nsteps - 0.5) * dt, dt=dt, t_rate=1.0,
+                       sources=[dict(kind=oracle.SRC_SINE, params=src)], observers=obs,
+                       ics=[(0.5 * half, 0.5 * half, 0.0, 0.1 * half, 1.0)], **ph)
+    ref = P.run()
+    sdofs, odofs, ows = _sources_observers(mesh, [src], obs)
+    npe = mesh["elem_nodes"].shape[1]
+    assert len(sdofs[0]) and len(odofs[0]) and not set(sdofs[0] // npe) & set(odofs[0] // npe)
+    times, _ = pkg.host.schedule(0.0, (nsteps - 0.5) * dt, dt, 1.0)
+    S = pkg.gpu.Solver(mesh, precision=pkg.gpu.DG_FP64 if prec == "fp64" else pkg.gpu.DG_FP32, **ph)
+    S.set_state(P.initial_state())
+    S.snapshot()
+    S.set_sources(sdofs)
+    S.set_source_values((src[4] * np.sin(2 * np.pi * src[5] * times + src[6]))[:, None])
+    S.set_observers(odofs, ows)
+    out = [S.run(n, dt) for n in chunks]
+    assert S.step == nsteps
+    tol = 1e-12 if prec == "fp64" else 1e-5
+    res, tr = np.concatenate([r for r, _ in out]), np.concatenate([o for _, o in out])
+    assert rel_l2(S.get_state()[:dim + 1], ref["state"][:dim + 1]) <= tol
+    assert rel_l2(res[:, :4], ref["residuals"][:, :4]) <= (1e-10 if prec == "fp64" else 1e-3)
+    assert rel_l2(tr, ref["obs"][:, :, [1, 2, 3, 4]]) <= tol * 10
+    S.close()
+
+
+@pytest.mark.parametrize("dim,p", [(2, 4), (3, 2)])
+def test_fp32_residual_of_a_large_finite_state_is_finite(pkg, dim, p):
+    """FP32 squares overflow from 1.8e19 on; a state beyond that is reported
+    as non-finite only when it is."""
+    mesh = _mesh(pkg, dim, p)
+    S = pkg.gpu.Solver(mesh, precision=pkg.gpu.DG_FP32, **_phys(dim))
+    u = smooth_state(mesh, seed=3)
+    for scale in (1.0, 1e25):
+        S.set_state(np.zeros_like(u))
+        S.snapshot()
+        S.set_state(u * scale)
+        res, _ = S.run(1, 1e-30)
+        m = (u * scale) ** 2
+        want = np.array([m[0].mean(), m[0].mean() / _phys(dim)["c0"] ** 4] + [m[q].mean() for q in (1, 2, 3)])
+        assert np.max(np.abs(res[0] - want)[want > 0] / want[want > 0]) <= 1e-5
+    u[0, 5] = np.inf
+    S.set_state(u)
+    with pytest.raises(pkg.gpu.SolverError, match="DG_ERR_NONFINITE"):
+        S.run(1, 1e-30)
+    S.close()
