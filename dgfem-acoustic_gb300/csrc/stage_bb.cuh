@@ -19,10 +19,15 @@
 //   f = n.F(y-) - h = 1/2 n.F(d) - 1/2 s c0 d,  d = y- - y+   (interior)
 //   f = (A_n - B) y-                                          (boundary).
 // Per variable and element 3-D p = 3 takes about 700 multiply-adds against
-// 2000 with the dense nodal operators, p = 4 about 1150 against 5800; FP64
-// runs at 2 multiply-adds per clock and SM on GB300, so FP64 stages are bound
-// by that count, and the FP32 stages were bound by the shared-memory loads of
-// the dense operators' entries, which are compile-time constants here.
+// 2000 with the dense nodal operators, p = 4 about 1150 against 5800. FP32
+// stages were bound by the shared-memory loads of the dense operators' entries,
+// which are compile-time constants here; they are now within a factor of two of
+// the memory floor. FP64 runs at 2 operations per clock and SM on GB300 and
+// bounds its stages by their count, which the fixed-point lift (bb_tile_fx)
+// halves again. Measured per RK4 step against the nodal kernels' best:
+// 196,608 tetrahedra of order 3, FP32, 0.61 -> 0.30 ms (floor 0.19); 131,712 of
+// order 4, FP32, 0.61 -> 0.37 (0.21); 24,576 of order 3, FP64, 2.24 -> 0.42
+// (0.05); 125,000 triangles of order 4, FP32, 0.14 -> 0.09 (0.07).
 //
 // Layout: arrays of tiles of 32 elements, [tile][variable][coefficient][32]:
 // a warp's lanes are the tile's elements, every load and store of a
@@ -157,7 +162,9 @@ struct BBCfg {
   static constexpr size_t oGF = oY + (size_t)NBUF * YB;
   static constexpr size_t oGI = oGF + (size_t)NBUF * GB;
   static constexpr size_t oN = oGI + (size_t)NBUF * IB;                 // [NF][NV][NFP][32]
-  static constexpr size_t oR = oN + (size_t)NF * NV * NFP * LW * sizeof(T);
+  static constexpr bool FX = sizeof(T) == 8;  // lift and elevation in fixed point (bb_tile_fx)
+  static constexpr size_t oX = oN + (size_t)NF * NV * NFP * LW * sizeof(T);  // int [NF][NV][32]: exponents (FX)
+  static constexpr size_t oR = oX + (FX ? (size_t)NF * NV * LW * 4 : 0);
   static constexpr size_t bytes = oR + NV * NV * sizeof(double);
   static_assert(NF == NV, "a block's warps are faces and variables in turn");
   static_assert(NFP <= 16 && NP <= 64, "tables hold 16 nodes per face");
@@ -542,6 +549,269 @@ __device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, con
   if (a.stage >= 4) racc.template add<C>(out);
 }
 
+// ---- FP64: fixed-point lift and elevation --------------------------------------
+//
+// GB300 runs 2 FP64 operations per clock and SM, but 128 integer ones. L0, the
+// layers of the lift and the degree elevation are combinations with small
+// integer weights, so FP64 kernels take them in 64-bit integers: the values
+// that enter (a face's fluxes, the gradient's coefficients) are rounded to 53
+// bits below the largest exponent among them, every sum is exact but for the
+// layers' divisions by 2, 3, 4 and 5 and the alignment of the faces' scales,
+// and the result is rounded to FP64 once. Weights grow a value by at most
+// (P+1)(P+3) in L0, 5 in the layers and 4 over the faces, 2^9.5 at P = 4, which
+// leaves the sign bit. An infinity or NaN makes the whole sum a NaN. 3-D p = 3:
+// 325 FP64 operations per thread instead of 740.
+
+__device__ __forceinline__ int fx_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// x as a multiple of 2^(E - 1075), E at least its biased exponent, rounded to
+// nearest: at most 2^53 in size.
+__device__ __forceinline__ long long fx_fix(double x, int E) {
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+  unsigned long long m =
+      ((unsigned long long)(((unsigned)hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x);
+  if (e == 0) m = 0;  // zero, and subnormal values far below any scale
+  const int s = min(E - e, 63);
+  m = (m + ((1ull << s) >> 1)) >> s;
+  return hi < 0 ? -(long long)m : (long long)m;
+}
+// v 2^-d, rounded to nearest
+__device__ __forceinline__ long long fx_shift(long long v, int d) {
+  const int s = min(d, 62);
+  return (v + ((1ll << s) >> 1)) >> s;
+}
+// (double)v, by two additions
+__device__ __forceinline__ double fx_double(long long v) {
+  const double h = __hiloint2double(0x45300000, (int)((unsigned)(v >> 32) ^ 0x80000000u));
+  const double l = __hiloint2double(0x43300000, (int)(unsigned)v);
+  return (h - 19342822341709703277445120.0) + l;  // 2^84 + 2^63 + 2^52
+}
+// 2^(E - 1075); NaN for the exponent of infinities and NaNs. E >= 54.
+__device__ __forceinline__ double fx_scale(int E) {
+  // 2^(E - 1075) = 2^(E - 1023 - 52): exponent field E - 52
+  return E == 0x7ff ? __hiloint2double(0x7ff80000, 0) : __hiloint2double((E - 52) << 20, 0);
+}
+constexpr int kFxMinExp = 64;  // scales below 2^-1011 are not resolved
+
+template <class C, int M>
+__device__ __forceinline__ long long fx_stencil_at(const long long (&f)[C::NFP]) {
+  constexpr int D = C::D, P = C::P;
+  using L = BLat<D - 1, P, M>;
+  constexpr int w0 = (L::b.a[0] + 1) * (L::b.a[0] + 1) + (L::b.a[1] + 1) * (L::b.a[1] + 1) +
+                     (D == 3 ? (L::b.a[2] + 1) * (L::b.a[2] + 1) : 0);
+  long long s = (long long)w0 * f[M];
+  bb_for<D * D>([&](auto ij_) {
+    constexpr int i = decltype(ij_)::value / D, j = decltype(ij_)::value % D;
+    if constexpr (i != j && L::b.a[j] > 0) {
+      constexpr int n = bb_index(D - 1, P, bb_add(bb_add(L::b, i, 1), j, -1));
+      constexpr int w = (L::b.a[i] + 1) * L::b.a[j];
+      s += (long long)w * f[n];
+    }
+  });
+  return s;
+}
+
+// v / N rounded (N = 2, 3, 4, 5)
+template <int N>
+__device__ __forceinline__ long long fx_div(long long v) {
+  if constexpr (N == 2) return (v + 1) >> 1;
+  else if constexpr (N == 4) return (v + 2) >> 2;
+  else return __mul64hi(v + N / 2, N == 3 ? 0x5555555555555556ll : 0x3333333333333334ll);
+}
+
+// Adds layers J .. P of face F's lift to out (bb_layers in integers).
+template <class C, int F, int J>
+__device__ __forceinline__ void fx_layers(const long long (&prev)[bb_np(C::D - 1, C::P - J + 1)],
+                                          long long (&out)[C::NP]) {
+  constexpr int D = C::D, P = C::P;
+  if constexpr (J <= P) {
+    long long cur[bb_np(D - 1, P - J)];
+    bb_for<bb_np(D - 1, P - J)>([&](auto g_) {
+      using L = BLat<D - 1, P - J, decltype(g_)::value>;
+      long long s = 0;
+      bb_for<D>([&](auto k_) {
+        constexpr int k = decltype(k_)::value;
+        constexpr int n = bb_index(D - 1, P - J + 1, bb_add(L::b, k, 1));
+        constexpr int w = L::b.a[k] + 1;
+        s -= (long long)w * prev[n];
+      });
+      s = fx_div<J + 1>(s);
+      cur[decltype(g_)::value] = s;
+      constexpr int a = bb_layer_index(D, P, F, J, L::b);
+      out[a] += s;
+    });
+    if constexpr (J < P) fx_layers<C, F, J + 1>(cur, out);
+  }
+}
+
+// The gradient's coefficients t (degree P-1) of variable q's volume term: the
+// volume term is -elevation(t) (bb_volume without the elevation).
+template <class C>
+__device__ __forceinline__ void fx_gradient(const double* y, const double* g, int q, double rhoc2, double inv_rho0,
+                                            double (&t)[bb_np(C::D, C::P - 1)]) {
+  constexpr int D = C::D, P = C::P, NP = C::NP, LW = C::LW;
+  BBGrad<double, D> gv;
+#pragma unroll
+  for (int r = 0; r < D; ++r) gv.g[r] = g[(C::oGV + r) * LW];
+  gv.done();
+  BBGrad<double, D> gm[D];
+  if (q == 0) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+#pragma unroll
+      for (int r = 0; r < D; ++r) gm[d].g[r] = rhoc2 * g[(C::oG + r * D + d) * LW];
+      gm[d].done();
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < D; ++r) gm[0].g[r] = inv_rho0 * g[(C::oG + r * D + q - 1) * LW];
+    gm[0].done();
+  }
+  const double* yq = y + q * NP * LW;
+  bb_for<bb_np(D, P - 1)>([&](auto b_) {
+    using L = BLat<D, P - 1, decltype(b_)::value>;
+    constexpr int n0 = bb_index(D, P, bb_add(L::b, 0, 1)), n1 = bb_index(D, P, bb_add(L::b, 1, 1)),
+                  n2 = bb_index(D, P, bb_add(L::b, 2, 1)), n3 = D == 3 ? bb_index(D, P, bb_add(L::b, 3, 1)) : 0;
+    double s = gv.template add<n0, n1, n2, n3, LW>(0.0, yq);
+    if (q == 0) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) s = gm[d].template add<n0, n1, n2, n3, LW>(s, y + (1 + d) * NP * LW);
+    } else {
+      s = gm[0].template add<n0, n1, n2, n3, LW>(s, y);
+    }
+    t[decltype(b_)::value] = s;
+  });
+}
+
+// One tile of an FP64 state (see above): bb_tile with fluxes and gradient in
+// FP64, stencil, lift and elevation in fixed point. sN holds the faces'
+// stencil results as integers, sX [NF][NV][32] their exponents.
+template <class C, class Free>
+__device__ __forceinline__ void bb_tile_fx(const StageArgs<double>& a, int64_t tile, const double* y, const double* g,
+                                           const int* gi, const int* sFm, const unsigned char* sNb, long long* sN,
+                                           int* sX, int lane, int role, BBRes<double>& racc, Free&& free_inputs) {
+  constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, NV = C::NV, LW = C::LW, D = C::D, P = C::P;
+  const double rhoc2 = a.ph.rhoc2, inv_rho0 = a.ph.inv_rho0;
+  // ---- this face's neighbour trace ----
+  const int nbr = gi[role * LW], code = gi[(NF + role) * LW];
+  const bool boundary = code & kCodeBoundary;
+  const bool in_tile = boundary || (nbr >> 5) == tile;
+  double up[NV][NFP];
+  {
+    const double* nb =
+        in_tile ? y - lane + (boundary ? lane : (nbr & 31)) : a.y_in + (int64_t)(nbr >> 5) * C::TW + (nbr & 31);
+    const int slot = (code & kCodeLfMask) * C::NPERM + ((code >> kCodePermShift) & kCodePermMask);
+    uint32_t w[4];
+    *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(sNb + (boundary ? 0 : slot) * 16);
+#pragma unroll
+    for (int m = 0; m < NFP; ++m) {
+      const double* p = nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * LW;
+#pragma unroll
+      for (int q = 0; q < NV; ++q) up[q][m] = p[q * NP * LW];
+    }
+  }
+  // ---- this variable's gradient ----
+  double t[bb_np(D, P - 1)];
+  fx_gradient<C>(y, g, role, rhoc2, inv_rho0, t);
+  // ---- this face's flux ----
+  {
+    const double* gf = g + role * (D + 1) * LW;
+    double np_[D], nu_[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) np_[d] = rhoc2 * gf[d * LW], nu_[d] = inv_rho0 * gf[d * LW];
+    const double A = gf[D * LW];
+    const int* fm = sFm + role * 16;
+    if (boundary) {
+      const double* Bg = a.bbM + (int64_t)nbr * NV * NV;
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        double um[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) um[q] = y[q * NP * LW + fm[m]];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          double s = 0.0;
+#pragma unroll
+          for (int qq = 0; qq < NV; ++qq) s += __ldg(Bg + q * NV + qq) * um[qq];
+          up[q][m] = s;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        double d[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) d[q] = y[q * NP * LW + fm[m]] - up[q][m];
+        double s = A * d[0];
+#pragma unroll
+        for (int k = 0; k < D; ++k) s += np_[k] * d[1 + k];
+        up[0][m] = s;
+#pragma unroll
+        for (int k = 0; k < D; ++k) up[1 + k][m] = A * d[1 + k] + nu_[k] * d[0];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      int E = kFxMinExp;
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) E = max(E, fx_exponent(up[q][m]));
+      long long f[NFP];
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) f[m] = fx_fix(up[q][m], E);
+      long long* sf = sN + (role * NV + q) * NFP * LW + lane;
+      bb_for<NFP>([&](auto m_) { sf[decltype(m_)::value * LW] = fx_stencil_at<C, decltype(m_)::value>(f); });
+      sX[(role * NV + q) * LW + lane] = E;
+    }
+  }
+  const double dte = a.dt * g[C::oS * LW];
+  __syncthreads();
+  free_inputs();
+  // ---- this variable's elevation and lift ----
+  const int64_t base = tile * C::TW + role * NP * LW + lane;
+  BBOps<C, double> ops;
+  ops.load(a, base, 0);
+  int E = kFxMinExp, ef[NF];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) ef[f] = sX[(f * NV + role) * LW + lane], E = max(E, ef[f]);
+#pragma unroll
+  for (int b = 0; b < bb_np(D, P - 1); ++b) E = max(E, fx_exponent(t[b]));
+  long long acc[NP];
+#pragma unroll
+  for (int n = 0; n < NP; ++n) acc[n] = 0;
+  bb_for<bb_np(D, P - 1)>([&](auto b_) {
+    using L = BLat<D, P - 1, decltype(b_)::value>;
+    const long long v = fx_fix(t[decltype(b_)::value], E);
+    bb_for<D + 1>([&](auto k_) {
+      constexpr int k = decltype(k_)::value;
+      constexpr int n = bb_index(D, P, bb_add(L::b, k, 1));
+      constexpr int w = L::b.a[k] + 1;
+      acc[n] -= (long long)w * v;
+    });
+  });
+  bb_for<NF>([&](auto f_) {
+    constexpr int f = decltype(f_)::value;
+    long long l0[NFP];
+#pragma unroll
+    for (int m = 0; m < NFP; ++m) l0[m] = fx_shift(sN[((f * NV + role) * NFP + m) * LW + lane], E - ef[f]);
+    bb_for<NFP>([&](auto m_) {
+      constexpr int n = bb_layer_index(D, P, f, 0, bb_lattice(D - 1, P, decltype(m_)::value));
+      acc[n] += l0[decltype(m_)::value];
+    });
+    fx_layers<C, f, 1>(l0, acc);
+  });
+  // ---- RK update: dt L is acc in units of dt 2^(E - 1075) ----
+  double out[NP];
+#pragma unroll
+  for (int n = 0; n < NP; ++n) out[n] = fx_double(acc[n]);
+  const double unit = dte * fx_scale(E);
+#pragma unroll
+  for (int n0 = 0; n0 < NP; n0 += C::CH) {
+    if (n0 > 0) ops.load(a, base, n0);
+    ops.update(a, base, n0, unit, out);
+  }
+  if (a.stage >= 4) racc.template add<C>(out);
+}
+
 // One tile in the Q4 layout (FP32, 3-D). The flux phase is bb_tile's (a warp
 // per face, a lane per element) with all variables of a node in one 16-byte
 // load: the neighbour trace touches two elements' values per sector instead
@@ -742,6 +1012,9 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB, GA>::NT, MINB) stag
     };
     if constexpr (C::Q4)
       bb_tile_q4<C>(a, tile, y, g, gi, sFm, sNb, sN, tid, role, racc, free_inputs);
+    else if constexpr (C::FX)
+      bb_tile_fx<C>(a, tile, y + lane, g + lane, gi + lane, sFm, sNb, reinterpret_cast<long long*>(sN),
+                    reinterpret_cast<int*>(sm + C::oX), lane, role, racc, free_inputs);
     else
       bb_tile<C, T>(a, tile, y + lane, g + lane, gi + lane, sFm, sNb, sN, lane, role, racc, free_inputs);
   }

@@ -8,14 +8,14 @@ namespace dgk {
 namespace {
 // per (dim, order): candidate (NBUF, MINB, GA)
 #define DGK_BB_VARIANTS(X) \
-  X(2, 1, 2, 10, 0) X(2, 1, 1, 12, 0)  \
-  X(2, 2, 2, 8, 0) X(2, 2, 1, 8, 0)    \
-  X(2, 3, 2, 6, 0) X(2, 3, 1, 6, 0)    \
-  X(2, 4, 2, 4, 0) X(2, 4, 1, 5, 0)    \
-  X(3, 1, 2, 6, 0) X(3, 1, 1, 8, 0)    \
-  X(3, 2, 2, 3, 0) X(3, 2, 1, 4, 0) X(3, 2, 1, 5, 1)    \
-  X(3, 3, 2, 2, 0) X(3, 3, 1, 3, 0) X(3, 3, 1, 3, 1)    \
-  X(3, 4, 1, 2, 0) X(3, 4, 1, 1, 0)
+  X(2, 1, 2, 10, 0) X(2, 1, 2, 8, 0)  \
+  X(2, 2, 2, 8, 0) X(2, 2, 2, 6, 0)   \
+  X(2, 3, 2, 6, 0) X(2, 3, 2, 5, 0)   \
+  X(2, 4, 2, 4, 0) X(2, 4, 1, 5, 0)   \
+  X(3, 1, 2, 6, 0) X(3, 1, 2, 5, 0)   \
+  X(3, 2, 2, 3, 0) X(3, 2, 1, 4, 0)   \
+  X(3, 3, 2, 2, 0) X(3, 3, 1, 3, 0)   \
+  X(3, 4, 1, 2, 0)
 }  // namespace
 
 cudaError_t launch_stage_bb(int dim, int order, int variant, const StageArgs<double>& a, int grid, int* err,

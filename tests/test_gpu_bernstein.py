@@ -203,3 +203,33 @@ def test_fp32_residual_of_a_large_finite_state_is_finite(pkg, dim, p):
     with pytest.raises(pkg.gpu.SolverError, match="DG_ERR_NONFINITE"):
         S.run(1, 1e-30)
     S.close()
+
+
+@pytest.mark.parametrize("dim,p", [(2, 1), (2, 4), (3, 2), (3, 4)])
+def test_fp64_fixed_point_follows_the_scale_of_the_state(pkg, oracle, dim, p):
+    """The FP64 kernels lift in integers at the scale of each element's data:
+    a state times a power of two gives the right-hand side times it, bit for
+    bit, over the exponent range; elements at rest beside loud ones and
+    variables of very different size keep the single right-hand side's bound."""
+    mesh = _mesh(pkg, dim, p)
+    ph = _phys(dim)
+    S = pkg.gpu.Solver(mesh, precision=pkg.gpu.DG_FP64, **ph)
+    u = smooth_state(mesh, seed=21)
+    k = S.rhs(u, 0.5)
+    for e in (-600, -52, 1, 300, 900):
+        np.testing.assert_array_equal(S.rhs(np.ldexp(u, e), 0.5), np.ldexp(k, e))
+    assert np.all(S.rhs(np.zeros_like(u), 0.5) == 0.0)
+    npe = mesh["elem_nodes"].shape[1]
+    quiet = u.copy()
+    quiet[:, :u.shape[1] // npe // 2 * npe] = 0.0
+    uneven = u * np.array([1e6, 1.0, 1e-6, 1e-3])[:, None]
+    for v in (quiet, uneven):
+        if dim == 2:
+            v[3] = 0.0
+        ref = oracle.Problem(mesh, dt=1e-4, **ph).stage(v)
+        assert rel_l2(S.rhs(v, 1e-4)[:dim + 1], ref[:dim + 1]) <= 5e-11
+    bad = u.copy()
+    bad[0, 0], bad[1, npe * 7] = np.nan, np.inf
+    r = S.rhs(bad, 1e-4).reshape(4, -1, npe)
+    assert not np.isfinite(r[0, 0]).any() and not np.isfinite(r[1, 7]).all()
+    S.close()
