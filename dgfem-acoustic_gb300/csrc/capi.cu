@@ -307,6 +307,7 @@ dgk::StageArgs<T> stage_args(dg_ctx* c, int stage, const T* y_in, T* y_out, T* k
   a.bbF = (const T*)c->bbF;
   a.bbI = c->bbI;
   a.bbM = (const T*)c->bbM;
+  a.bbC = a.bbM + c->n_bfaces * c->nv * c->nv;
   a.Dt = (const T*)c->Dt;
   a.LIFT = (const T*)c->LIFT;
   a.cslot = c->ncurved > 0 ? c->cslot : nullptr;

@@ -34,6 +34,7 @@ constexpr int kCodePermShift = 2;      // corner permutation index (3 bits)
 constexpr int kCodePermMask = 0x7;
 constexpr int kCodeNegPenalty = 1 << 5;  // penalty sign s_f = -1
 constexpr int kCodeBoundary = 1 << 6;    // boundary face; nbr slot holds the boundary index
+constexpr int kCodePlainBoundary = 1 << 7;  // its flux has the five-term form (StageArgs::bbC)
 
 // Compile-time shape of a (dim, order) pair.
 template <int D, int P>
@@ -140,6 +141,7 @@ struct StageArgs {
   const T* bbF;
   const int* bbI;
   const T* bbM;
+  const T* bbC;  // [boundary faces][8]
   const T* Dt;     // [D][NP(j)][NP(i)]
   const T* LIFT;   // [NF*NFP(k)][NP(i)]
   const short* fmask;   // [NF*NFP]

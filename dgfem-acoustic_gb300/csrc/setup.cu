@@ -387,7 +387,7 @@ __global__ void k_penalty_hist(const int* geoI, int reci, int nf, int64_t E, uns
 // face of the padded mesh (padding elements: zero records).
 template <typename T>
 __global__ void k_bb_geo(const double* geo64, int recf, const int* geoI, int reci, const double* bm64, int D,
-                         int64_t E, int64_t Epad, double rho0, double c0, int gw, T* outF, int* outI, T* outM) {
+                         int64_t E, int64_t Epad, double rho0, double c0, int gw, T* outF, int* outI, T* outM, T* outC) {
   const int nf = D + 1, NV = D + 1;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= Epad * nf) return;
@@ -419,13 +419,34 @@ __global__ void k_bb_geo(const double* geo64, int recf, const int* geoI, int rec
   }
   if (e < E && (code & dgk::kCodeBoundary)) {
     const double rc2 = rho0 * c0 * c0;
+    double M[4][4], n[3] = {gf[0], gf[1], D == 3 ? gf[2] : 0.0};
     for (int a = 0; a < NV; ++a)
       for (int b = 0; b < NV; ++b) {
         double an = a == b ? vn : 0.0;
-        if (a == 0 && b > 0) an = rc2 * gf[b - 1];
-        if (a > 0 && b == 0) an = gf[a - 1] / rho0;
-        outM[(int64_t)nbr * NV * NV + a * NV + b] = (T)(sJ * (an - bm64[(int64_t)nbr * NV * NV + a * NV + b]));
+        if (a == 0 && b > 0) an = rc2 * n[b - 1];
+        if (a > 0 && b == 0) an = n[a - 1] / rho0;
+        M[a][b] = sJ * (an - bm64[(int64_t)nbr * NV * NV + a * NV + b]);
+        outM[(int64_t)nbr * NV * NV + a * NV + b] = (T)M[a][b];
       }
+    // A wall, and an absorbing boundary but for the outflow through faces whose
+    // tangent frame is oblique, take p and v to
+    //   f0 = a p + b t,   f_k = e v_k + m_k (c p + f t),   t = m.v,  m = 0.5 sJ n:
+    // the coefficients from M, and whether they give M back to rounding
+    double b0 = 0.0, c1 = 0.0, nn = 0.0, tr = 0.0;
+    for (int a = 0; a < D; ++a) {
+      b0 += M[0][1 + a] * n[a], c1 += M[1 + a][0] * n[a], tr += M[1 + a][1 + a];
+      for (int b = 0; b < D; ++b) nn += n[a] * M[1 + a][1 + b] * n[b];
+    }
+    const double ev = (tr - nn) / (D - 1), h = 0.5 * sJ;
+    double off = 0.0;
+    for (int a = 0; a < D; ++a) {
+      off = fmax(off, fabs(M[0][1 + a] - b0 * n[a]) / (rho0 * c0));
+      off = fmax(off, fabs(M[1 + a][0] - c1 * n[a]) * (rho0 * c0));
+      for (int b = 0; b < D; ++b) off = fmax(off, fabs(M[1 + a][1 + b] - ((a == b ? ev : 0.0) + (nn - ev) * n[a] * n[b])));
+    }
+    T* oc = outC + (int64_t)nbr * 8;
+    oc[0] = (T)M[0][0], oc[1] = (T)(b0 / h), oc[2] = (T)(c1 / h), oc[3] = (T)ev, oc[4] = (T)((nn - ev) / (h * h));
+    if (off <= 8.9e-16 * sJ * (c0 + fabs(vn))) ri[(nf + f) * 32] = code | dgk::kCodePlainBoundary;
   }
 }
 
@@ -613,15 +634,15 @@ int run_setup(dg_ctx* c, const dg_mesh_desc* mesh, const double* elem_v0, const 
       const size_t ts = c->prec == DG_FP32 ? 4 : 8;
       SETUP_CK(dev_alloc(c, &c->bbF, Epad * gw * ts));
       SETUP_CK(dev_alloc(c, (void**)&c->bbI, Epad * 2 * nf * sizeof(int)));
-      SETUP_CK(dev_alloc(c, &c->bbM, nbm * ts));
+      SETUP_CK(dev_alloc(c, &c->bbM, (nbm + 8 * std::max<int64_t>(c->n_bfaces, 1)) * ts));
       if (c->prec == DG_FP32)
         k_bb_geo<float><<<blocks(Epad * nf, 128), 128, 0, st>>>(geo64, recf64, c->geoI, reci, bm64, D, E, Epad,
                                                                 c->ph.rho0, c->ph.c0, gw, (float*)c->bbF, c->bbI,
-                                                                (float*)c->bbM);
+                                                                (float*)c->bbM, (float*)c->bbM + c->n_bfaces * c->nv * c->nv);
       else
         k_bb_geo<double><<<blocks(Epad * nf, 128), 128, 0, st>>>(geo64, recf64, c->geoI, reci, bm64, D, E, Epad,
                                                                  c->ph.rho0, c->ph.c0, gw, (double*)c->bbF, c->bbI,
-                                                                 (double*)c->bbM);
+                                                                 (double*)c->bbM, (double*)c->bbM + c->n_bfaces * c->nv * c->nv);
       SETUP_CK(cudaGetLastError());
       SETUP_CK(cudaStreamSynchronize(st));
       rc = bb_setup_basis(c);

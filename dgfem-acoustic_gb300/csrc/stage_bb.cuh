@@ -137,11 +137,10 @@ __host__ __device__ constexpr double bb_value(int d, int p, int i, int j) {
 // NBUF_: stage-input buffers (2: the next tile arrives while this one
 // computes; 1: after its flux phase), MINB: blocks per SM that the register
 // budget allows for.
-template <typename T_, int D_, int P_, int NBUF_, int MINB_, int GA_>
+template <typename T_, int D_, int P_, int NBUF_, int MINB_>
 struct BBCfg {
   using T = T_;
   static constexpr int D = D_, P = P_, NBUF = NBUF_, MINB = MINB_;
-  static constexpr bool ASYNC = GA_ != 0;  // neighbour traces by cp.async into sN, else into registers
   using S = Shape<D_, P_>;
   static constexpr int NP = S::NP, NF = S::NF, NFP = S::NFP, NV = S::NV, NPERM = S::NPERM;
   static constexpr int LW = 32;                 // elements per tile
@@ -151,6 +150,8 @@ struct BBCfg {
   // [tile][coefficient][32][4], else one plane each, [tile][variable][coefficient][32]
   static constexpr bool Q4 = sizeof(T) == 4 && D == 3;
   static constexpr int SQ = Q4 ? 1 : NP * LW, SN = Q4 ? 4 * LW : LW, SE = Q4 ? 4 : 1;  // word strides
+  // word in the tile of the first coefficient that a thread owns in the update
+  __host__ __device__ static constexpr int first_word(int tid, int role) { return Q4 ? tid : role * NP * LW + (tid & 31); }
   static constexpr int oGV = NF * (D + 1), oG = oGV + D, oS = oG + D * D, GW = oS + 1;  // geometry words
   static constexpr int GI = 2 * NF;             // neighbour, code
   static constexpr int CH = sizeof(T) == 8 ? 6 : 10;  // coefficients whose RK operands are in flight together
@@ -360,14 +361,53 @@ struct BBRes {
   __device__ __forceinline__ double get() const { return (double)s + big; }
 };
 
-// RK operands of CH coefficients of this thread: loaded together (the first
-// group before the lift, so that its latency overlaps it), then combined with
-// dt*L and stored. In stages 4 and 5 out becomes the residual's difference.
-template <class C, typename T>
-struct BBOps {
+// What a tile's body meets outside the tile, for the kernels that run one
+// stage per launch: other tiles' stage input and the RK arrays, in global
+// memory. RK operands of CH coefficients of this thread are loaded together
+// (the first group before the lift, so that its latency overlaps it), then
+// combined with dt*L and stored; in stages 4 and 5 out becomes the residual's
+// difference.
+template <class C, class Free>
+struct BBGlobalEnv {
+  using T = typename C::T;
   static constexpr int CH = C::CH, SN = C::SN, NP = C::NP;
+  // the trace's loads come first: their latency overlaps the volume term
+  static constexpr bool kTraceLast = false;
+  const StageArgs<T>& a;
+  int64_t base;      // this thread's first coefficient in the arrays
+  Free free_inputs;  // called by every thread once the stage input is no longer read
   T x0[CH], x1[CH], x2[CH];
-  __device__ __forceinline__ void load(const StageArgs<T>& a, int64_t base, int n0) {
+  __device__ __forceinline__ BBGlobalEnv(const StageArgs<T>& a_, int64_t b, Free f) : a(a_), base(b), free_inputs(f) {}
+  // Values at the neighbour's face nodes: node m has coefficient (w byte m) of
+  // the element whose first word is y_nb in shared memory (in_tile) or word
+  // `word` of the stage input.
+  template <int NFP>
+  __device__ __forceinline__ void gather(bool in_tile, const T* y_nb, int64_t word, const uint32_t (&w)[4],
+                                         T (&up)[C::NV][NFP]) {
+    const T* nb = in_tile ? y_nb : a.y_in + word;
+#pragma unroll
+    for (int m = 0; m < NFP; ++m) {
+      const T* p = nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * SN;
+#pragma unroll
+      for (int q = 0; q < C::NV; ++q) up[q][m] = p[q * C::SQ];
+    }
+  }
+  template <int NFP>
+  __device__ __forceinline__ void gather(bool in_tile, const float* y_nb, int64_t word, const uint32_t (&w)[4],
+                                         float4 (&up)[NFP]) {
+    const float* nb = in_tile ? y_nb : a.y_in + word;
+#pragma unroll
+    for (int m = 0; m < NFP; ++m)
+      up[m] = *reinterpret_cast<const float4*>(nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * SN);
+  }
+  // the face data of the tile are in shared memory
+  __device__ __forceinline__ bool sync() {
+    __syncthreads();
+    free_inputs();
+    return true;
+  }
+  __device__ __forceinline__ bool residual() const { return a.stage >= 4; }
+  __device__ __forceinline__ void load(int n0) {
     const int stage = a.stage;
     if (stage == 0) return;
     const T* u = a.u + base;
@@ -387,7 +427,7 @@ struct BBOps {
         if (n0 + i < NP) x2[i] = sn[(n0 + i) * SN];
     }
   }
-  __device__ __forceinline__ void update(const StageArgs<T>& a, int64_t base, int n0, T dte, T (&out)[NP]) {
+  __device__ __forceinline__ void update(int n0, T dte, T (&out)[NP]) {
     const int stage = a.stage;
     T* ac = a.acc + base;
     T* yo = a.y_out + base;
@@ -439,54 +479,33 @@ __device__ __forceinline__ T bb_dt(const StageArgs<T>& a) {
   if constexpr (sizeof(T) == 4) return a.f_dt; else return a.dt;
 }
 
-// One tile: y, g, gi at this lane in shared memory. free_inputs() is called
-// by every thread once the tile's stage input is no longer read.
-template <class C, typename T, class Free>
-__device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, const T* y, const T* g, const int* gi,
-                                        const int* sFm, const unsigned char* sNb, T* sN, int lane, int role, BBRes<T>& racc,
-                                        Free&& free_inputs) {
+// One tile: y, g, gi at this lane in shared memory; env: BBGlobalEnv, or what
+// keeps the RK arrays elsewhere. False when env's barrier said to stop.
+template <class C, typename T, class Env>
+__device__ __forceinline__ bool bb_tile(const StageArgs<T>& a, Env& env, int64_t tile, const T* y, const T* g,
+                                        const int* gi, const int* sFm, const unsigned char* sNb, T* sN, int lane,
+                                        int role, BBRes<T>& racc) {
   constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, NV = C::NV, LW = C::LW, D = C::D;
   const T rhoc2 = bb_rhoc2<T>(a), inv_rho0 = bb_inv_rho0<T>(a);
   // ---- this face's neighbour trace ----
   const int nbr = gi[role * LW], code = gi[(NF + role) * LW];
   const bool boundary = code & kCodeBoundary;
   const bool in_tile = boundary || (nbr >> 5) == tile;
-  const T* nb = in_tile ? y - lane + (boundary ? lane : (nbr & 31)) : a.y_in + (int64_t)(nbr >> 5) * C::TW + (nbr & 31);
   T up[NV][NFP];
-  uint32_t w[4];
   T* sf = sN + role * NV * NFP * LW + lane;  // this thread's face data
-  {
+  auto trace = [&]() {
     const int slot = (code & kCodeLfMask) * C::NPERM + ((code >> kCodePermShift) & kCodePermMask);
+    uint32_t w[4];
     *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(sNb + (boundary ? 0 : slot) * 16);
-    if constexpr (C::ASYNC) {
-      if (!in_tile) {
-#pragma unroll
-        for (int m = 0; m < NFP; ++m) {
-          const T* p = nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * LW;
-#pragma unroll
-          for (int q = 0; q < NV; ++q) {
-            if constexpr (sizeof(T) == 4)
-              cp_async4(sf + (q * NFP + m) * LW, p + q * NP * LW);
-            else
-              cp_async8(sf + (q * NFP + m) * LW, p + q * NP * LW);
-          }
-        }
-      }
-      cp_async_commit();
-    } else {
-#pragma unroll
-      for (int m = 0; m < NFP; ++m) {
-        const T* p = nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * LW;
-#pragma unroll
-        for (int q = 0; q < NV; ++q) up[q][m] = p[q * NP * LW];
-      }
-    }
-  }
+    env.template gather<NFP>(in_tile, y - lane + (boundary ? lane : (nbr & 31)),
+                             (int64_t)(nbr >> 5) * C::TW + (nbr & 31), w, up);
+  };
+  if constexpr (!Env::kTraceLast) trace();
   // ---- this variable's volume term ----
   T out[NP];
   bb_volume<C>(y, g, role, rhoc2, inv_rho0, out);
+  if constexpr (Env::kTraceLast) trace();
   // ---- this face's flux ----
-  if constexpr (C::ASYNC) cp_async_wait_all();
   {
     const T* gf = g + role * (D + 1) * LW;
     T np_[D], nu_[D];
@@ -510,16 +529,9 @@ __device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, con
         }
       }
     } else {
-      const T* pb = in_tile ? nb : sf;
-      const int qs = in_tile ? NP * LW : NFP * LW;
 #pragma unroll
       for (int m = 0; m < NFP; ++m) {
         T d[NV];
-        if constexpr (C::ASYNC) {
-          const T* p = pb + (in_tile ? (int)((w[m / 4] >> (8 * (m % 4))) & 0xffu) : m) * LW;
-#pragma unroll
-          for (int q = 0; q < NV; ++q) up[q][m] = p[q * qs];
-        }
 #pragma unroll
         for (int q = 0; q < NV; ++q) d[q] = y[q * NP * LW + fm[m]] - up[q][m];
         T s = A * d[0];
@@ -534,19 +546,17 @@ __device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, con
     for (int q = 0; q < NV; ++q) bb_face_stencil<C>(up[q], sf + q * NFP * LW);
   }
   const T dte = bb_dt<T>(a) * g[C::oS * LW];
-  __syncthreads();
-  free_inputs();
+  if (!env.sync()) return false;
   // ---- this variable's lift and RK update ----
-  const int64_t base = tile * C::TW + role * NP * LW + lane;
-  BBOps<C, T> ops;
-  ops.load(a, base, 0);
+  env.load(0);
   bb_lift<C, NV * NFP * LW, LW>(sN + role * NFP * LW + lane, out);
 #pragma unroll
   for (int n0 = 0; n0 < NP; n0 += C::CH) {
-    if (n0 > 0) ops.load(a, base, n0);
-    ops.update(a, base, n0, dte, out);
+    if (n0 > 0) env.load(n0);
+    env.update(n0, dte, out);
   }
-  if (a.stage >= 4) racc.template add<C>(out);
+  if (env.residual()) racc.template add<C>(out);
+  return true;
 }
 
 // ---- FP64: fixed-point lift and elevation --------------------------------------
@@ -560,7 +570,7 @@ __device__ __forceinline__ void bb_tile(const StageArgs<T>& a, int64_t tile, con
 // and the result is rounded to FP64 once. Weights grow a value by at most
 // (P+1)(P+3) in L0, 5 in the layers and 4 over the faces, 2^9.5 at P = 4, which
 // leaves the sign bit. An infinity or NaN makes the whole sum a NaN. 3-D p = 3:
-// 325 FP64 operations per thread instead of 740.
+// 285 FP64 operations per thread instead of 740.
 
 __device__ __forceinline__ int fx_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 
@@ -580,11 +590,15 @@ __device__ __forceinline__ long long fx_shift(long long v, int d) {
   const int s = min(d, 62);
   return (v + ((1ll << s) >> 1)) >> s;
 }
-// (double)v, by two additions
+// v rounded to FP64, put together from its bits (two FP64 additions would take
+// four times as long)
 __device__ __forceinline__ double fx_double(long long v) {
-  const double h = __hiloint2double(0x45300000, (int)((unsigned)(v >> 32) ^ 0x80000000u));
-  const double l = __hiloint2double(0x43300000, (int)(unsigned)v);
-  return (h - 19342822341709703277445120.0) + l;  // 2^84 + 2^63 + 2^52
+  const unsigned long long m0 = (unsigned long long)(v < 0 ? -v : v);
+  const int z = __clzll(m0);
+  const unsigned long long m = m0 << (z & 63);
+  // 53 bits, rounded; the leading one and a carry add to the exponent
+  const unsigned long long b = ((unsigned long long)(1085 - z) << 52) + (m >> 11) + ((m >> 10) & 1);
+  return v == 0 ? 0.0 : __longlong_as_double((long long)(b | ((unsigned long long)v & 0x8000000000000000ull)));
 }
 // 2^(E - 1075); NaN for the exponent of infinities and NaNs. E >= 54.
 __device__ __forceinline__ double fx_scale(int E) {
@@ -686,10 +700,10 @@ __device__ __forceinline__ void fx_gradient(const double* y, const double* g, in
 // One tile of an FP64 state (see above): bb_tile with fluxes and gradient in
 // FP64, stencil, lift and elevation in fixed point. sN holds the faces'
 // stencil results as integers, sX [NF][NV][32] their exponents.
-template <class C, class Free>
-__device__ __forceinline__ void bb_tile_fx(const StageArgs<double>& a, int64_t tile, const double* y, const double* g,
-                                           const int* gi, const int* sFm, const unsigned char* sNb, long long* sN,
-                                           int* sX, int lane, int role, BBRes<double>& racc, Free&& free_inputs) {
+template <class C, class Env>
+__device__ __forceinline__ bool bb_tile_fx(const StageArgs<double>& a, Env& env, int64_t tile, const double* y,
+                                           const double* g, const int* gi, const int* sFm, const unsigned char* sNb,
+                                           long long* sN, int* sX, int lane, int role, BBRes<double>& racc) {
   constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, NV = C::NV, LW = C::LW, D = C::D, P = C::P;
   const double rhoc2 = a.ph.rhoc2, inv_rho0 = a.ph.inv_rho0;
   // ---- this face's neighbour trace ----
@@ -697,22 +711,28 @@ __device__ __forceinline__ void bb_tile_fx(const StageArgs<double>& a, int64_t t
   const bool boundary = code & kCodeBoundary;
   const bool in_tile = boundary || (nbr >> 5) == tile;
   double up[NV][NFP];
-  {
-    const double* nb =
-        in_tile ? y - lane + (boundary ? lane : (nbr & 31)) : a.y_in + (int64_t)(nbr >> 5) * C::TW + (nbr & 31);
+  auto trace = [&]() {
     const int slot = (code & kCodeLfMask) * C::NPERM + ((code >> kCodePermShift) & kCodePermMask);
     uint32_t w[4];
     *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(sNb + (boundary ? 0 : slot) * 16);
+    env.template gather<NFP>(in_tile, y - lane + (boundary ? lane : (nbr & 31)),
+                             (int64_t)(nbr >> 5) * C::TW + (nbr & 31), w, up);
+  };
+  if constexpr (!Env::kTraceLast) trace();
+  // boundary faces' coefficients, before they are needed
+  const bool any_boundary = __any_sync(0xffffffffu, boundary);
+  const bool plain_boundary = !__any_sync(0xffffffffu, boundary && !(code & kCodePlainBoundary));
+  double bc[5] = {};
+  if (any_boundary && plain_boundary) {
+    bc[0] = bc[3] = g[(role * (D + 1) + D) * LW], bc[1] = rhoc2, bc[2] = inv_rho0, bc[4] = 0.0;
+    if (boundary)
 #pragma unroll
-    for (int m = 0; m < NFP; ++m) {
-      const double* p = nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * LW;
-#pragma unroll
-      for (int q = 0; q < NV; ++q) up[q][m] = p[q * NP * LW];
-    }
+      for (int i = 0; i < 5; ++i) bc[i] = __ldg(a.bbC + (int64_t)nbr * 8 + i);
   }
   // ---- this variable's gradient ----
   double t[bb_np(D, P - 1)];
   fx_gradient<C>(y, g, role, rhoc2, inv_rho0, t);
+  if constexpr (Env::kTraceLast) trace();
   // ---- this face's flux ----
   {
     const double* gf = g + role * (D + 1) * LW;
@@ -721,7 +741,23 @@ __device__ __forceinline__ void bb_tile_fx(const StageArgs<double>& a, int64_t t
     for (int d = 0; d < D; ++d) np_[d] = rhoc2 * gf[d * LW], nu_[d] = inv_rho0 * gf[d * LW];
     const double A = gf[D * LW];
     const int* fm = sFm + role * 16;
-    if (boundary) {
+    if (any_boundary && plain_boundary) {
+      // interior faces and walls in one form (k_bb_geo): 17 FP64 operations per
+      // node in 3-D, where a branch each would take 14 and 16
+#pragma unroll
+      for (int m = 0; m < NFP; ++m) {
+        double d[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) d[q] = y[q * NP * LW + fm[m]] - (boundary ? 0.0 : up[q][m]);
+        double s = gf[0] * d[1];
+#pragma unroll
+        for (int k = 1; k < D; ++k) s += gf[k * LW] * d[1 + k];
+        up[0][m] = bc[0] * d[0] + bc[1] * s;
+        const double r = bc[2] * d[0] + bc[4] * s;
+#pragma unroll
+        for (int k = 0; k < D; ++k) up[1 + k][m] = bc[3] * d[1 + k] + gf[k * LW] * r;
+      }
+    } else if (boundary) {
       const double* Bg = a.bbM + (int64_t)nbr * NV * NV;
 #pragma unroll
       for (int m = 0; m < NFP; ++m) {
@@ -764,12 +800,9 @@ __device__ __forceinline__ void bb_tile_fx(const StageArgs<double>& a, int64_t t
     }
   }
   const double dte = a.dt * g[C::oS * LW];
-  __syncthreads();
-  free_inputs();
+  if (!env.sync()) return false;
   // ---- this variable's elevation and lift ----
-  const int64_t base = tile * C::TW + role * NP * LW + lane;
-  BBOps<C, double> ops;
-  ops.load(a, base, 0);
+  env.load(0);
   int E = kFxMinExp, ef[NF];
 #pragma unroll
   for (int f = 0; f < NF; ++f) ef[f] = sX[(f * NV + role) * LW + lane], E = max(E, ef[f]);
@@ -806,10 +839,11 @@ __device__ __forceinline__ void bb_tile_fx(const StageArgs<double>& a, int64_t t
   const double unit = dte * fx_scale(E);
 #pragma unroll
   for (int n0 = 0; n0 < NP; n0 += C::CH) {
-    if (n0 > 0) ops.load(a, base, n0);
-    ops.update(a, base, n0, unit, out);
+    if (n0 > 0) env.load(n0);
+    env.update(n0, unit, out);
   }
-  if (a.stage >= 4) racc.template add<C>(out);
+  if (env.residual()) racc.template add<C>(out);
+  return true;
 }
 
 // One tile in the Q4 layout (FP32, 3-D). The flux phase is bb_tile's (a warp
@@ -821,10 +855,10 @@ __device__ __forceinline__ void bb_tile_fx(const StageArgs<double>& a, int64_t t
 // coupling of the variables goes through shuffles within an element's four
 // lanes (every lane forms t_j = H_j . D u with H_j the metric column that its
 // neighbour lane ^ (j+1) needs, zero where it needs none).
-template <class C, class Free>
-__device__ __forceinline__ void bb_tile_q4(const StageArgs<float>& a, int64_t tile, const float* y, const float* g,
-                                           const int* gi, const int* sFm, const unsigned char* sNb, float* sN, int tid,
-                                           int role, BBRes<float>& racc, Free&& free_inputs) {
+template <class C, class Env>
+__device__ __forceinline__ bool bb_tile_q4(const StageArgs<float>& a, Env& env, int64_t tile, const float* y,
+                                           const float* g, const int* gi, const int* sFm, const unsigned char* sNb,
+                                           float* sN, int tid, int role, BBRes<float>& racc) {
   constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, LW = C::LW, D = C::D, P = C::P, SN = C::SN;
   const float rhoc2 = a.f_rhoc2, inv_rho0 = a.f_inv_rho0;
   const int lane = tid & 31;
@@ -833,16 +867,14 @@ __device__ __forceinline__ void bb_tile_q4(const StageArgs<float>& a, int64_t ti
   const bool boundary = code & kCodeBoundary;
   const bool in_tile = boundary || (nbr >> 5) == tile;
   float4 up[NFP];
-  {
-    const float* nb = in_tile ? y + 4 * (boundary ? lane : (nbr & 31))
-                              : a.y_in + (int64_t)(nbr >> 5) * C::TW + 4 * (nbr & 31);
+  auto trace = [&]() {
     const int slot = (code & kCodeLfMask) * C::NPERM + ((code >> kCodePermShift) & kCodePermMask);
     uint32_t w[4];
     *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(sNb + (boundary ? 0 : slot) * 16);
-#pragma unroll
-    for (int m = 0; m < NFP; ++m)
-      up[m] = *reinterpret_cast<const float4*>(nb + ((w[m / 4] >> (8 * (m % 4))) & 0xffu) * SN);
-  }
+    env.template gather<NFP>(in_tile, y + 4 * (boundary ? lane : (nbr & 31)),
+                             (int64_t)(nbr >> 5) * C::TW + 4 * (nbr & 31), w, up);
+  };
+  if constexpr (!Env::kTraceLast) trace();
   // ---- volume term of this thread's variable q of element el ----
   const int q = tid & 3, el = tid >> 2;
   float out[NP];
@@ -877,6 +909,7 @@ __device__ __forceinline__ void bb_tile_q4(const StageArgs<float>& a, int64_t ti
       });
     });
   }
+  if constexpr (Env::kTraceLast) trace();
   // ---- this face's flux ----
   {
     const float* gf = g + role * (D + 1) * LW + lane;
@@ -916,19 +949,32 @@ __device__ __forceinline__ void bb_tile_q4(const StageArgs<float>& a, int64_t ti
     });
   }
   const float dte = a.f_dt * g[C::oS * LW + el];
-  __syncthreads();
-  free_inputs();
+  if (!env.sync()) return false;
   // ---- this variable's lift and RK update ----
-  const int64_t base = tile * C::TW + tid;
-  BBOps<C, float> ops;
-  ops.load(a, base, 0);
+  env.load(0);
   bb_lift<C, NFP * SN, SN>(sN + tid, out);
 #pragma unroll
   for (int n0 = 0; n0 < NP; n0 += C::CH) {
-    if (n0 > 0) ops.load(a, base, n0);
-    ops.update(a, base, n0, dte, out);
+    if (n0 > 0) env.load(n0);
+    env.update(n0, dte, out);
   }
-  if (a.stage >= 4) racc.template add<C>(out);
+  if (env.residual()) racc.template add<C>(out);
+  return true;
+}
+
+// The tile body of configuration C (y, g, gi: the tile's buffers).
+template <class C, class Env, typename T>
+__device__ __forceinline__ bool bb_tile_any(const StageArgs<T>& a, Env& env, int64_t tile, const T* y, const T* g,
+                                            const int* gi, const int* sFm, const unsigned char* sNb, T* sN, int* sX,
+                                            int tid, int role, BBRes<T>& racc) {
+  const int lane = tid & 31;
+  if constexpr (C::Q4)
+    return bb_tile_q4<C>(a, env, tile, y, g, gi, sFm, sNb, sN, tid, role, racc);
+  else if constexpr (C::FX)
+    return bb_tile_fx<C>(a, env, tile, y + lane, g + lane, gi + lane, sFm, sNb, reinterpret_cast<long long*>(sN), sX,
+                         lane, role, racc);
+  else
+    return bb_tile<C, T>(a, env, tile, y + lane, g + lane, gi + lane, sFm, sNb, sN, lane, role, racc);
 }
 
 // Face tables in shared memory: element word offset of each face node, and
@@ -941,9 +987,9 @@ __device__ __forceinline__ void bb_load_tables(const StageArgs<T>& a, int* sFm, 
     sNb[i] = i % 16 < C::NFP ? (unsigned char)a.nbrnode[i / 16 * C::NFP + i % 16] : (unsigned char)0;
 }
 
-template <typename T, int D, int P, int NBUF, int MINB, int GA>
-__global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB, GA>::NT, MINB) stage_bb_kernel(const StageArgs<T> a, int* err) {
-  using C = BBCfg<T, D, P, NBUF, MINB, GA>;
+template <typename T, int D, int P, int NBUF, int MINB>
+__global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB>::NT, MINB) stage_bb_kernel(const StageArgs<T> a, int* err) {
+  using C = BBCfg<T, D, P, NBUF, MINB>;
   extern __shared__ __align__(128) unsigned char sm[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(sm + C::oBar);
   int* sFm = reinterpret_cast<int*>(sm + C::oFm);
@@ -1010,13 +1056,8 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB, GA>::NT, MINB) stag
     auto free_inputs = [&]() {
       if constexpr (NBUF == 1) issue_next();
     };
-    if constexpr (C::Q4)
-      bb_tile_q4<C>(a, tile, y, g, gi, sFm, sNb, sN, tid, role, racc, free_inputs);
-    else if constexpr (C::FX)
-      bb_tile_fx<C>(a, tile, y + lane, g + lane, gi + lane, sFm, sNb, reinterpret_cast<long long*>(sN),
-                    reinterpret_cast<int*>(sm + C::oX), lane, role, racc, free_inputs);
-    else
-      bb_tile<C, T>(a, tile, y + lane, g + lane, gi + lane, sFm, sNb, sN, lane, role, racc, free_inputs);
+    BBGlobalEnv<C, decltype(free_inputs)> env(a, (int64_t)tile * C::TW + C::first_word(tid, role), free_inputs);
+    bb_tile_any<C>(a, env, tile, y, g, gi, sFm, sNb, sN, reinterpret_cast<int*>(sm + C::oX), tid, role, racc);
   }
   if (!ok && tid == 0) atomicOr(err, 1);
 
@@ -1047,11 +1088,11 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB, GA>::NT, MINB) stag
   }
 }
 
-template <typename T, int D, int P, int NBUF, int MINB, int GA>
+template <typename T, int D, int P, int NBUF, int MINB>
 struct StageBB {
-  using C = BBCfg<T, D, P, NBUF, MINB, GA>;
+  using C = BBCfg<T, D, P, NBUF, MINB>;
   static cudaError_t set_attrs() {
-    auto kfn = stage_bb_kernel<T, D, P, NBUF, MINB, GA>;
+    auto kfn = stage_bb_kernel<T, D, P, NBUF, MINB>;
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::bytes);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1064,7 +1105,7 @@ struct StageBB {
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    return launch_kernel(stage_bb_kernel<T, D, P, NBUF, MINB, GA>, dim3((unsigned)grid), C::NT, C::bytes, s, a.pdl != 0,
+    return launch_kernel(stage_bb_kernel<T, D, P, NBUF, MINB>, dim3((unsigned)grid), C::NT, C::bytes, s, a.pdl != 0,
                          a, err);
   }
   static int blocks_per_sm() {
@@ -1073,7 +1114,7 @@ struct StageBB {
       return 0;
     }
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stage_bb_kernel<T, D, P, NBUF, MINB, GA>, C::NT, C::bytes) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stage_bb_kernel<T, D, P, NBUF, MINB>, C::NT, C::bytes) !=
         cudaSuccess) {
       cudaGetLastError();
       return 0;

@@ -19,9 +19,9 @@
 
 namespace dgk {
 
-using MultiC2 = BBCfg<float, 2, 2, 2, 1, 0>;
-using MultiC3 = BBCfg<float, 2, 3, 2, 1, 0>;
-using MultiC4 = BBCfg<float, 2, 4, 2, 1, 0>;
+using MultiC2 = BBCfg<float, 2, 2, 2, 1>;
+using MultiC3 = BBCfg<float, 2, 3, 2, 1>;
+using MultiC4 = BBCfg<float, 2, 4, 2, 1>;
 constexpr int kMultiNT = MultiC4::NT;
 static_assert(MultiC2::NT == kMultiNT && MultiC3::NT == kMultiNT, "every order's tile takes the whole block");
 // blocks per SM the register budget is set for
@@ -72,9 +72,10 @@ template <class C>
 __device__ __forceinline__ void multi_run_tile(const StageArgs<float>& a, int tile, unsigned char* slot, float* sN,
                                                const int* sFm, const unsigned char* sNb, int lane, int role,
                                                BBRes<float>& racc) {
-  bb_tile<C, float>(a, tile, reinterpret_cast<const float*>(slot) + lane,
-                    reinterpret_cast<const float*>(slot + C::YB) + lane,
-                    reinterpret_cast<const int*>(slot + C::YB + C::GB) + lane, sFm, sNb, sN, lane, role, racc, []() {});
+  auto keep = []() {};
+  BBGlobalEnv<C, decltype(keep)> env(a, (int64_t)tile * C::TW + C::first_word(lane, role), keep);
+  bb_tile_any<C>(a, env, tile, reinterpret_cast<const float*>(slot), reinterpret_cast<const float*>(slot + C::YB),
+                 reinterpret_cast<const int*>(slot + C::YB + C::GB), sFm, sNb, sN, (int*)nullptr, lane, role, racc);
 }
 
 __global__ void __launch_bounds__(kMultiNT, kMultiMinBlocks) stage_multi_kernel(const MultiArgs m, int* err) {
