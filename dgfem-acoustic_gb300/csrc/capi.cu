@@ -289,6 +289,7 @@ constexpr int kGraphSteps = 8;
 void drop_graphs(dg_ctx* c) {
   if (c->graph) cudaGraphExecDestroy(c->graph), c->graph = nullptr;
   if (c->graph_n) cudaGraphExecDestroy(c->graph_n), c->graph_n = nullptr;
+  c->persist.stale = true;
 }
 
 template <typename T>
@@ -332,7 +333,7 @@ template <typename T>
 cudaError_t launch_stage_t(dg_ctx* c, int stage, const T* y_in, T* y_out, T* k_out, double dt) {
   const dgk::StageArgs<T> a = stage_args<T>(c, stage, y_in, y_out, k_out, dt);
   if (dgk::is_bb_variant(c->variant))
-    return dgk::launch_stage_bb(c->dim, c->order, c->variant - dgk::kBBVariant, a, c->grid2, c->d_err, c->stream);
+    return dgk::launch_stage_bb(c->dim, c->order, dgk::bb_variant_index(c->variant), a, c->grid2, c->d_err, c->stream);
   if (dgk::is_tc_variant(c->variant)) {
     if constexpr (sizeof(T) == 4)
       return dgk::is_tc3_variant(c->variant)
@@ -521,13 +522,20 @@ int run_steps(dg_ctx* c, int kind, int64_t n_steps, double dt, double* residuals
   if (n_steps == 0) return DG_OK;
   int rc = ensure_out_cap(c, n_steps);
   if (rc) return rc;
-  const int64_t many = n_steps / kGraphSteps, rest = n_steps % kGraphSteps;
-  if (many > 0) rc = build_graph(c, kind, dt, kGraphSteps);
-  if (!rc && rest > 0) rc = build_graph(c, kind, dt, 1);
-  if (!rc) rc = begin_run(c, n_steps);
-  if (rc) return rc;
-  for (int64_t i = 0; i < many; ++i) CK(c, cudaGraphLaunch(c->graph_n, c->stream));
-  for (int64_t i = 0; i < rest; ++i) CK(c, cudaGraphLaunch(c->graph, c->stream));
+  // a single step in the many-steps kernel takes up to 12 us more than its graph,
+  // each further one 5 to 20 us less (3-D order 2, 1,080 elements: 92 against 81
+  // us for one, 525 against 576 for ten)
+  if (kind == 0 && n_steps >= 4 && dgk::is_persist_variant(c->variant) && dgc::persist_ready(c)) {
+    CK(c, dgc::persist_run(c, n_steps, dt));
+  } else {
+    const int64_t many = n_steps / kGraphSteps, rest = n_steps % kGraphSteps;
+    if (many > 0) rc = build_graph(c, kind, dt, kGraphSteps);
+    if (!rc && rest > 0) rc = build_graph(c, kind, dt, 1);
+    if (!rc) rc = begin_run(c, n_steps);
+    if (rc) return rc;
+    for (int64_t i = 0; i < many; ++i) CK(c, cudaGraphLaunch(c->graph_n, c->stream));
+    for (int64_t i = 0; i < rest; ++i) CK(c, cudaGraphLaunch(c->graph, c->stream));
+  }
   std::vector<double> res(n_steps * 5);
   CK(c, cudaMemcpyAsync(res.data(), c->d_res, n_steps * 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   if (obs && c->n_obs > 0)
@@ -566,14 +574,15 @@ void to_dev_ops(const dgref::RefElement& re, std::vector<T>& Dt, std::vector<T>&
 // curved-element path; the baseline and pipelined kernels take the curved
 // right-hand side.
 bool variant_handles_mesh(const dg_ctx* c, int v) {
+  if (dgk::is_persist_variant(v)) return bb_mesh(c) && dgc::persist_fits(c);
   if (dgk::is_bb_variant(v)) return bb_mesh(c);
   return c->ncurved == 0 || !(dgk::is_tc_variant(v) || v >= dgk::kStage3Variant);
 }
 
 dgk::Stage2Info stage2_info(const dg_ctx* c, int v) {
   if (dgk::is_bb_variant(v))
-    return c->prec == DG_FP32 ? dgk::stage_bb_info_f32(c->dim, c->order, v - dgk::kBBVariant)
-                              : dgk::stage_bb_info_f64(c->dim, c->order, v - dgk::kBBVariant);
+    return c->prec == DG_FP32 ? dgk::stage_bb_info_f32(c->dim, c->order, dgk::bb_variant_index(v))
+                              : dgk::stage_bb_info_f64(c->dim, c->order, dgk::bb_variant_index(v));
   if (dgk::is_wide_variant(v))
     return c->prec == DG_FP32 ? dgk::stage4_info(c->dim, c->order, v - dgk::kWideVariant)
                               : dgk::Stage2Info{0, 0, 0, 0, 0, 0};
@@ -668,6 +677,7 @@ int upload_observers(dg_ctx* c) {
     }
   }
   const int64_t total = off[n_obs];
+  if (c->bb) c->obs_bb_off = off, c->obs_bb_slot = dof, c->obs_bb_w = w;
   CK(c, cudaMalloc(&c->d_obs_dof, std::max<int64_t>(total, 1) * sizeof(int64_t)));
   CK(c, cudaMalloc(&c->d_obs_off, (n_obs + 1) * sizeof(int64_t)));
   CK(c, cudaMalloc(&c->d_obs_w, std::max<int64_t>(total, 1) * sizeof(double)));
@@ -824,6 +834,15 @@ void tune_cache_store(const std::string& key, int v) {
   }
 }
 
+// Where all tiles of an FP64 mesh fit on the GPU at once, runs take the many-steps
+// kernel, which was the faster one on every such mesh (1.06 to 1.45 times, see
+// stage_persist.cuh), and only the other launches the Bernstein-basis kernel
+// selected.
+void take_persistent(dg_ctx* c) {
+  if (dgk::is_bb_variant(c->variant) && !dgk::is_persist_variant(c->variant))
+    set_variant(c, dgk::kPersistVariant + dgk::bb_variant_index(c->variant));
+}
+
 // Autotuner: times RK stages 1-3 (stage input, u and accumulator reads;
 // accumulator and next-stage writes) of every kernel variant on this mesh
 // and keeps the fastest. want >= -1 forces a variant instead; want == -3
@@ -838,7 +857,10 @@ int select_variant(dg_ctx* c, int want) {
   const std::string key = tune_key(c);
   if (want == -3) {
     int v = -1;
-    if (tune_cache_lookup(key, &v) && set_variant(c, v)) return apply_layout(c);
+    if (tune_cache_lookup(key, &v) && set_variant(c, v)) {
+      take_persistent(c);
+      return apply_layout(c);
+    }
   }
   std::vector<int> cands;
   auto offer = [&](int first, int count, bool contiguous) {
@@ -923,6 +945,7 @@ int select_variant(dg_ctx* c, int want) {
   cudaStreamSynchronize(c->stream);
   set_variant(c, best_v);
   tune_cache_store(key, best_v);
+  take_persistent(c);
   return apply_layout(c);
 }
 
@@ -935,6 +958,9 @@ cudaError_t enqueue_inject(dg_ctx* c) { return ::enqueue_inject(c); }
 cudaError_t enqueue_finalize(dg_ctx* c, int nparts) { return ::enqueue_finalize(c, nparts); }
 dgk::StageArgs<float> stage_args_f32(dg_ctx* c, int stage, const float* y_in, float* y_out, double dt) {
   return ::stage_args<float>(c, stage, y_in, y_out, nullptr, dt);
+}
+dgk::StageArgs<double> stage_args_f64(dg_ctx* c, int stage, const double* y_in, double* y_out, double dt) {
+  return ::stage_args<double>(c, stage, y_in, y_out, nullptr, dt);
 }
 int ensure_out_cap(dg_ctx* c, int64_t n) { return ::ensure_out_cap(c, n); }
 int create_ctx(const dg_mesh_desc* mesh, const dg_phys* phys, int precision, int device, const double* elem_v0,
@@ -1201,6 +1227,7 @@ int dg_destroy(dg_ctx* c) {
   if (!c) return DG_OK;
   drop_graphs(c);
   for (void* p : c->allocs) cudaFree(p);
+  dgc::persist_free(c);
   void* extra[] = {c->d_res, c->d_obs, c->d_src_dof, c->d_src_off, c->d_src_ids, c->d_srcval, c->d_src_elem, c->d_src_eoff,
                    c->d_obs_dof, c->d_obs_off, c->d_obs_w, c->d_obs_part, c->d_obs_cnt, c->d_obs_bmap,
                    c->d_obs_bfirst};
@@ -1288,7 +1315,7 @@ int dg_set_sources(dg_ctx* c, int n_src, const int64_t* offsets, const int64_t* 
     if (p) cudaFree(p);
   c->d_src_dof = nullptr, c->d_src_off = nullptr, c->d_src_ids = nullptr;
   c->d_src_elem = nullptr, c->d_src_eoff = nullptr, c->n_src_elems = 0;
-  c->src_elems.clear();
+  c->src_elems.clear(), c->src_dof.clear();
   c->n_src = n_src;
   c->n_src_dofs = (int64_t)hd.size();
   drop_graphs(c);
@@ -1314,7 +1341,7 @@ int dg_set_sources(dg_ctx* c, int n_src, const int64_t* offsets, const int64_t* 
   CK(c, cudaMemcpyAsync(c->d_src_eoff, heo.data(), heo.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
   c->n_src_elems = (int64_t)he.size();
-  c->src_elems.swap(he);
+  c->src_elems.swap(he), c->src_dof.swap(hd);
   note_overlap(c);
   return DG_OK;
 }
@@ -1448,6 +1475,11 @@ int dg_kernel_info(dg_ctx* c, int variant, int* out) {
   dgk::Stage2Info si = stage2_info(c, variant);
   // available exactly when dg_tune accepts it
   if (!variant_handles_mesh(c, variant) || si.nc == 0 || si.blocks_per_sm <= 0 || c->Epad % si.et != 0) return DG_OK;
+  if (dgk::is_persist_variant(variant)) {
+    const dgk::PersistInfo pi = dgk::persist_info(c->dim, c->order);
+    out[0] = si.et, out[1] = pi.nt, out[2] = pi.smem_bytes, out[3] = pi.blocks_per_sm, out[4] = (int)(c->Epad / si.et);
+    return DG_OK;
+  }
   out[0] = si.et, out[1] = si.nt, out[2] = si.smem_bytes, out[3] = si.blocks_per_sm;
   out[4] = (int)std::min<int64_t>(c->Epad / si.et, (int64_t)si.blocks_per_sm * c->num_sms);
   return DG_OK;

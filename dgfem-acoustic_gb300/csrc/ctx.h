@@ -106,11 +106,26 @@ struct dg_ctx {
   int64_t n_src_elems = 0;
   int64_t* d_src_elem = nullptr;
   int* d_src_eoff = nullptr;
-  std::vector<int64_t> src_elems;  // the same elements, ascending
+  std::vector<int64_t> src_elems, src_dof;  // the same elements and node slots, ascending
   bool src_obs_apart = true;       // no observer reads one of them
   // observers as given (internal node slots): the device lists depend on bb
   std::vector<int64_t> obs_off, obs_dof;
   std::vector<double> obs_w;
+  // the same per coefficient of the tiles (bb)
+  std::vector<int64_t> obs_bb_off, obs_bb_slot;
+  std::vector<double> obs_bb_w;
+  // many steps per launch (persist.cu): lists by tile and buffers, rebuilt when
+  // sources, observers or the kernel have changed
+  struct Persist {
+    bool stale = true;
+    int steps = 0, groups = 0;  // steps per launch, (tile, observer) pairs
+    int* ints = nullptr;        // the lists
+    void* inputs = nullptr;     // published stage inputs, two
+    uint32_t seq = 1;           // number of the next input
+    double *weights = nullptr, *obs_w = nullptr, *partials = nullptr, *gsum = nullptr;
+    int *sel_first = nullptr, *sel = nullptr, *snode_first = nullptr, *snode = nullptr, *grp_first = nullptr, *ent_first = nullptr, *ent_word = nullptr, *obs_first = nullptr,
+        *obs_grp = nullptr;
+  } persist;
   // per-step graph
   cudaGraphExec_t graph = nullptr, graph_n = nullptr;  // one step, kGraphSteps steps
   bool pdl = false;  // the next stage launch is a programmatic dependent of the kernel before it

@@ -259,13 +259,25 @@ Stage2Info stage4_info(int dim, int order, int variant);
 // Bernstein-basis stage kernel (stage_bb.cuh): variant ids kBBVariant + k;
 // the state is in tiles of 32 elements' coefficients.
 constexpr int kBBVariant = 64;
-inline bool is_bb_variant(int v) { return v >= kBBVariant && v < kBBVariant + 16; }
+inline bool is_bb_variant(int v) { return v >= kBBVariant && v < kBBVariant + 32; }
+inline int bb_variant_index(int v) { return (v - kBBVariant) & 15; }
 cudaError_t launch_stage_bb(int dim, int order, int variant, const StageArgs<float>& a, int grid, int* err,
                             cudaStream_t s);
 cudaError_t launch_stage_bb(int dim, int order, int variant, const StageArgs<double>& a, int grid, int* err,
                             cudaStream_t s);
 Stage2Info stage_bb_info_f32(int dim, int order, int variant);
 Stage2Info stage_bb_info_f64(int dim, int order, int variant);
+// Many steps of a small FP64 mesh in one launch (stage_persist.cuh): variant
+// kPersistVariant + k, whose other launches (single right-hand sides, Euler
+// steps, step graphs) are those of variant kBBVariant + k.
+constexpr int kPersistVariant = kBBVariant + 16;
+inline bool is_persist_variant(int v) { return v >= kPersistVariant && v < kPersistVariant + 16; }
+struct PersistInfo {
+  int nt, smem_bytes, blocks_per_sm;
+};
+struct PersistArgs;
+cudaError_t launch_persist(int dim, int order, const PersistArgs& p, int grid, int* err, cudaStream_t s);
+PersistInfo persist_info(int dim, int order);
 // geometry words of one element (floating-point) in the kernel's record
 inline int bb_geo_words(int dim) { return (dim + 1) * (dim + 1) + dim + dim * dim + 1; }
 // Mixed-order stage kernel of the batched ensemble (stage_multi.cuh): 2-D,

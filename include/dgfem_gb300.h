@@ -91,7 +91,7 @@ typedef struct {
   int64_t device_bytes;
   double setup_ms;
   int kernel_variant; /* stage kernel in use: 64 + k Bernstein-basis variant k (straight-sided triangles and
-                         tetrahedra), else -1 baseline, 0..15 pipelined variant k, 16..22 tensor-core kernel,
+                         tetrahedra), 80 + k the same with the many-steps kernel in dg_run, else -1 baseline, 0..15 pipelined variant k, 16..22 tensor-core kernel,
                          32.. constant-operator variant, 48.. wide-chunk variant */
   int kernel_grid;    /* blocks of each stage-kernel launch (persistent blocks for variants >= 0) */
   int64_t n_curved;   /* curved elements (high-order nodes off the straight-sided lattice), integrated
@@ -173,13 +173,17 @@ int dg_vtu_writer_stats(const dg_vtu_writer* w, int64_t* files_written, int* com
  * triangles and tetrahedra, both precisions; there the only ones that are
  * timed). The Bernstein-basis kernels hold the state as Bernstein
  * coefficients: a change to or from them converts state and snapshot, to
- * rounding. Returns
+ * rounding; 80 + k: variant 64 + k, with dg_run calls of four or more steps in
+ * one cooperative launch per 64 steps (FP64 contexts whose tiles of 32 elements
+ * all fit on the GPU at once; there what a selection by timing ends with).
+ * Returns
  * DG_ERR_ARG for a variant that does not exist for this element type or
  * precision. */
 int dg_tune(dg_ctx* ctx, int variant);
 
 /* Polling rounds that each bounded device wait of the stage kernels (the
- * mbarrier waits for their TMA copies and tensor-core work) makes before it
+ * mbarrier waits for their TMA copies and tensor-core work, the many-steps
+ * kernel's waits for neighbouring tiles) makes before it
  * gives up (default 2^20; 0 gives up at once). A kernel whose wait gives up
  * issues no further copy, waits with the default limit for the copies it
  * already issued, sets the context's error flag and returns; the dg_run call
