@@ -154,7 +154,7 @@ struct BBCfg {
   __host__ __device__ static constexpr int first_word(int tid, int role) { return Q4 ? tid : role * NP * LW + (tid & 31); }
   static constexpr int oGV = NF * (D + 1), oG = oGV + D, oS = oG + D * D, GW = oS + 1;  // geometry words
   static constexpr int GI = 2 * NF;             // neighbour, code
-  static constexpr int CH = sizeof(T) == 8 ? 6 : 10;  // coefficients whose RK operands are in flight together
+  static constexpr int CH = sizeof(T) == 8 ? 6 : 7;  // coefficients whose RK operands are in flight together
   static constexpr uint32_t YB = TW * sizeof(T), GB = GW * LW * sizeof(T), IB = GI * LW * 4;
   static constexpr size_t oBar = 0;                                     // NBUF mbarriers
   static constexpr size_t oFm = 64;                                     // int [NF][16]: element word offset of a face node
@@ -367,17 +367,31 @@ struct BBRes {
 // (the first group before the lift, so that its latency overlaps it), then
 // combined with dt*L and stored; in stages 4 and 5 out becomes the residual's
 // difference.
+//
+// FP64 keeps the classical accumulator k1 + 2 k2 + 2 k3. FP32, bound by memory,
+// has none: the inputs of stages 2 to 4 stay, and the step ends with
+//   u + ((y2 - u) + 2 (y3 - u) + (y4 - u)) / 3 + dt k4 / 6,
+// 14 state words moved per step where the accumulator takes 18. The differences
+// are exact to the roundings of y2 .. y4.
 template <class C, class Free>
 struct BBGlobalEnv {
   using T = typename C::T;
   static constexpr int CH = C::CH, SN = C::SN, NP = C::NP;
   // the trace's loads come first: their latency overlaps the volume term
   static constexpr bool kTraceLast = false;
+  // FP32: this thread's part of the stage input stays in shared memory until the
+  // update (not with one buffer, which the next tile enters at the barrier)
+  static constexpr bool OWN = sizeof(T) == 4 && C::NBUF == 2;
   const StageArgs<T>& a;
   int64_t base;      // this thread's first coefficient in the arrays
+  const T* own;      // the same in the tile's stage input
   Free free_inputs;  // called by every thread once the stage input is no longer read
-  T x0[CH], x1[CH], x2[CH];
-  __device__ __forceinline__ BBGlobalEnv(const StageArgs<T>& a_, int64_t b, Free f) : a(a_), base(b), free_inputs(f) {}
+  // FP32: u of all coefficients before the lift, the other operands of stage 4
+  // in groups
+  static constexpr int NU = sizeof(T) == 4 ? NP : CH;
+  T x0[NU], x1[CH], x2[CH], x3[CH];
+  __device__ __forceinline__ BBGlobalEnv(const StageArgs<T>& a_, int64_t b, const T* y, Free f)
+      : a(a_), base(b), own(OWN ? y : a_.y_in + b), free_inputs(f) {}
   // Values at the neighbour's face nodes: node m has coefficient (w byte m) of
   // the element whose first word is y_nb in shared memory (in_tile) or word
   // `word` of the stage input.
@@ -407,62 +421,101 @@ struct BBGlobalEnv {
     return true;
   }
   __device__ __forceinline__ bool residual() const { return a.stage >= 4; }
+  __device__ __forceinline__ void operands(int n0, T (&x)[CH], const T* p) const {
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+      if (n0 + i < NP) x[i] = p[(n0 + i) * SN];
+  }
   __device__ __forceinline__ void load(int n0) {
     const int stage = a.stage;
     if (stage == 0) return;
-    const T* u = a.u + base;
-    const T* ac = a.acc + base;
-    const T* sn = a.snap + base;
+    if constexpr (sizeof(T) == 4) {
+      if (stage >= 2 && n0 == 0) {
 #pragma unroll
-    for (int i = 0; i < CH; ++i)
-      if (n0 + i < NP) x0[i] = u[(n0 + i) * SN];
-    if (stage >= 2 && stage <= 4) {
-#pragma unroll
-      for (int i = 0; i < CH; ++i)
-        if (n0 + i < NP) x1[i] = ac[(n0 + i) * SN];
-    }
-    if (stage >= 4) {
-#pragma unroll
-      for (int i = 0; i < CH; ++i)
-        if (n0 + i < NP) x2[i] = sn[(n0 + i) * SN];
+        for (int n = 0; n < NP; ++n) x0[n] = a.u[base + n * SN];
+      }
+      if (OWN ? stage >= 4 : stage == 1 || stage == 4) operands(n0, x3, OWN ? a.snap + base : own);
+      if (stage == 4) operands(n0, x1, a.y2 + base), operands(n0, x2, a.y3 + base);
+    } else {
+      operands(n0, x0, a.u + base);
+      if (stage >= 2 && stage <= 4) operands(n0, x1, a.acc + base);
+      if (stage >= 4) operands(n0, x2, a.snap + base);
     }
   }
   __device__ __forceinline__ void update(int n0, T dte, T (&out)[NP]) {
     const int stage = a.stage;
-    T* ac = a.acc + base;
     T* yo = a.y_out + base;
     if (stage == 0) {
       T* ko = a.k_out + base;
 #pragma unroll
       for (int i = 0; i < CH; ++i)
         if (n0 + i < NP) ko[(n0 + i) * SN] = dte * out[n0 + i];
-    } else if (stage == 1) {
+      return;
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (stage <= 3) {
+        const T c = stage == 3 ? dte : (T)0.5 * dte;
 #pragma unroll
-      for (int i = 0; i < CH; ++i)
-        if (n0 + i < NP) {
-          ac[(n0 + i) * SN] = dte * out[n0 + i];
-          yo[(n0 + i) * SN] = x0[i] + ((T)0.5 * dte) * out[n0 + i];
-        }
-    } else if (stage <= 3) {
-      const T c = stage == 3 ? dte : (T)0.5 * dte, c2 = (T)2 * dte;
+        for (int i = 0; i < CH; ++i)
+          if (n0 + i < NP)
+            yo[(n0 + i) * SN] = (stage > 1 ? x0[n0 + i] : OWN ? own[(n0 + i) * SN] : x3[i]) + c * out[n0 + i];
+      } else {
+        T* un_ = stage == 4 ? a.u + base : yo;
+        const T* sn = a.snap + base;
+        const T c = dte * (T)(1.0 / 6.0);
 #pragma unroll
-      for (int i = 0; i < CH; ++i)
-        if (n0 + i < NP) {
-          ac[(n0 + i) * SN] = x1[i] + c2 * out[n0 + i];
-          yo[(n0 + i) * SN] = x0[i] + c * out[n0 + i];
-        }
+        for (int i = 0; i < CH; ++i)
+          if (n0 + i < NP) {
+            const T u = x0[n0 + i], y4 = OWN ? own[(n0 + i) * SN] : x3[i];
+            const T un = stage == 4 ? u + (((x1[i] - u) + (y4 - u) + (T)2 * (x2[i] - u)) * (T)(1.0 / 3.0) + c * out[n0 + i])
+                                    : u + dte * out[n0 + i];
+            un_[(n0 + i) * SN] = un;
+            out[n0 + i] = (OWN ? x3[i] : sn[(n0 + i) * SN]) - un;
+          }
+      }
     } else {
-      T* un_ = stage == 4 ? a.u + base : yo;
+      T* ac = a.acc + base;
+      if (stage == 1) {
 #pragma unroll
-      for (int i = 0; i < CH; ++i)
-        if (n0 + i < NP) {
-          const T un = stage == 4 ? x0[i] + (x1[i] + dte * out[n0 + i]) * (T)(1.0 / 6.0) : x0[i] + dte * out[n0 + i];
-          un_[(n0 + i) * SN] = un;
-          out[n0 + i] = x2[i] - un;
-        }
+        for (int i = 0; i < CH; ++i)
+          if (n0 + i < NP) {
+            ac[(n0 + i) * SN] = dte * out[n0 + i];
+            yo[(n0 + i) * SN] = x0[i] + ((T)0.5 * dte) * out[n0 + i];
+          }
+      } else if (stage <= 3) {
+        const T c = stage == 3 ? dte : (T)0.5 * dte, c2 = (T)2 * dte;
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+          if (n0 + i < NP) {
+            ac[(n0 + i) * SN] = x1[i] + c2 * out[n0 + i];
+            yo[(n0 + i) * SN] = x0[i] + c * out[n0 + i];
+          }
+      } else {
+        T* un_ = stage == 4 ? a.u + base : yo;
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+          if (n0 + i < NP) {
+            const T un = stage == 4 ? x0[i] + (x1[i] + dte * out[n0 + i]) * (T)(1.0 / 6.0) : x0[i] + dte * out[n0 + i];
+            un_[(n0 + i) * SN] = un;
+            out[n0 + i] = x2[i] - un;
+          }
+      }
     }
   }
 };
+
+// A tile's RK operands towards L2.
+template <class C, typename T>
+__device__ __forceinline__ void prefetch_operands(const StageArgs<T>& a, int64_t tile) {
+  if (a.stage == 0) return;
+  if (a.u != a.y_in) prefetch_l2(a.u + tile * C::TW, C::YB);
+  if constexpr (sizeof(T) == 8) {
+    if (a.stage >= 2 && a.stage <= 4) prefetch_l2(a.acc + tile * C::TW, C::YB);
+  } else {
+    if (a.stage == 4) prefetch_l2(a.y2 + tile * C::TW, C::YB), prefetch_l2(a.y3 + tile * C::TW, C::YB);
+  }
+  if (a.stage >= 4) prefetch_l2(a.snap + tile * C::TW, C::YB);
+}
 
 // constants in the working precision (FP32: rounded on the host, a conversion
 // per thread and tile runs at the FP64 rate)
@@ -1003,7 +1056,6 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB>::NT, MINB) stage_bb
   // the pressure's volume term is the longest: its warp is another scheduler's
   // in each block that shares an SM
   const int role = ((tid >> 5) + blockIdx.x) % C::NV;
-  const int nepi = a.stage == 1 || a.stage == 5 ? 1 : a.stage == 2 || a.stage == 3 ? 2 : a.stage == 4 ? 3 : 0;
 
   auto issue_geometry = [&](int64_t tile, int b) {
     mbar_expect_tx(&bar[b], C::YB + C::GB + C::IB);
@@ -1012,10 +1064,7 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB>::NT, MINB) stage_bb
   };
   auto issue_state = [&](int64_t tile, int b) {
     tma_load_1d(sY + (size_t)b * C::TW, a.y_in + tile * C::TW, C::YB, &bar[b]);
-    // the tile's RK operands towards L2
-    if (nepi >= 1 && a.u != a.y_in) prefetch_l2(a.u + tile * C::TW, C::YB);
-    if (nepi >= 2) prefetch_l2(a.acc + tile * C::TW, C::YB);
-    if (nepi >= 3) prefetch_l2(a.snap + tile * C::TW, C::YB);
+    prefetch_operands<C>(a, tile);
   };
   auto issue = [&](int64_t tile, int b) { issue_geometry(tile, b), issue_state(tile, b); };
 
@@ -1056,7 +1105,8 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB>::NT, MINB) stage_bb
     auto free_inputs = [&]() {
       if constexpr (NBUF == 1) issue_next();
     };
-    BBGlobalEnv<C, decltype(free_inputs)> env(a, (int64_t)tile * C::TW + C::first_word(tid, role), free_inputs);
+    BBGlobalEnv<C, decltype(free_inputs)> env(a, (int64_t)tile * C::TW + C::first_word(tid, role), y + C::first_word(tid, role),
+                                              free_inputs);
     bb_tile_any<C>(a, env, tile, y, g, gi, sFm, sNb, sN, reinterpret_cast<int*>(sm + C::oX), tid, role, racc);
   }
   if (!ok && tid == 0) atomicOr(err, 1);

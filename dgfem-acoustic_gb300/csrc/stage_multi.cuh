@@ -57,15 +57,12 @@ __device__ __forceinline__ int multi_slot(const MultiArgs& m, int item, int* til
 
 template <class C>
 __device__ __forceinline__ void multi_issue_tile(const StageArgs<float>& a, int64_t tile, unsigned char* slot,
-                                                 uint64_t* bar, int nepi) {
+                                                 uint64_t* bar) {
   mbar_expect_tx(bar, C::YB + C::GB + C::IB);
   tma_load_1d(slot, a.y_in + tile * C::TW, C::YB, bar);
   tma_load_1d(slot + C::YB, a.bbF + tile * C::GW * C::LW, C::GB, bar);
   tma_load_1d(slot + C::YB + C::GB, a.bbI + tile * C::GI * C::LW, C::IB, bar);
-  // the tile's RK operands towards L2
-  if (nepi >= 1 && a.u != a.y_in) prefetch_l2(a.u + tile * C::TW, C::YB);
-  if (nepi >= 2) prefetch_l2(a.acc + tile * C::TW, C::YB);
-  if (nepi >= 3) prefetch_l2(a.snap + tile * C::TW, C::YB);
+  prefetch_operands<C>(a, tile);
 }
 
 template <class C>
@@ -73,7 +70,8 @@ __device__ __forceinline__ void multi_run_tile(const StageArgs<float>& a, int ti
                                                const int* sFm, const unsigned char* sNb, int lane, int role,
                                                BBRes<float>& racc) {
   auto keep = []() {};
-  BBGlobalEnv<C, decltype(keep)> env(a, (int64_t)tile * C::TW + C::first_word(lane, role), keep);
+  BBGlobalEnv<C, decltype(keep)> env(a, (int64_t)tile * C::TW + C::first_word(lane, role),
+                                       reinterpret_cast<const float*>(slot) + C::first_word(lane, role), keep);
   bb_tile_any<C>(a, env, tile, reinterpret_cast<const float*>(slot), reinterpret_cast<const float*>(slot + C::YB),
                  reinterpret_cast<const int*>(slot + C::YB + C::GB), sFm, sNb, sN, (int*)nullptr, lane, role, racc);
 }
@@ -91,15 +89,14 @@ __global__ void __launch_bounds__(kMultiNT, kMultiMinBlocks) stage_multi_kernel(
   const int tid = threadIdx.x, lane = tid & 31;
   const int role = ((tid >> 5) + blockIdx.x) % MultiC4::NV;
   const int stage = m.g[0].stage;
-  const int nepi = stage == 1 ? 1 : stage == 4 ? 3 : 2;
 
   auto issue = [&](int item, int b) {
     int tile;
     const int g = multi_slot(m, item, &tile);
     unsigned char* slot = slots + (size_t)b * L::SLOT;
-    if (g == 0) multi_issue_tile<MultiC2>(m.g[0], tile, slot, &bar[b], nepi);
-    if (g == 1) multi_issue_tile<MultiC3>(m.g[1], tile, slot, &bar[b], nepi);
-    if (g == 2) multi_issue_tile<MultiC4>(m.g[2], tile, slot, &bar[b], nepi);
+    if (g == 0) multi_issue_tile<MultiC2>(m.g[0], tile, slot, &bar[b]);
+    if (g == 1) multi_issue_tile<MultiC3>(m.g[1], tile, slot, &bar[b]);
+    if (g == 2) multi_issue_tile<MultiC4>(m.g[2], tile, slot, &bar[b]);
   };
 
   if (tid == 0) {
