@@ -7,13 +7,12 @@
 //
 // Instances of one element type (dim, order) are concatenated into one
 // disjoint-union mesh and solved by one context whose geometry records carry
-// each element's own mean flow and time step. Every step is one CUDA graph.
-// For 2-D FP32 instances of orders 2-4 (the ensemble study) every RK stage of
-// all instances is one persistent launch of the mixed-order stage kernel
-// (stage_multi.cuh), whose blocks take tiles of every order from a work
-// queue; otherwise the per-type contexts run their source injection, four
-// fused RK4 stages and observer reductions on their own streams as parallel
-// branches of the graph.
+// each element's own mean flow and time step. The contexts run their source
+// injection, four RK4 stages and observer reductions on their own streams as
+// parallel branches of one CUDA graph, eight steps long where the run is.
+// Optionally, for 2-D FP32 instances of orders 2-4, every RK stage of all
+// instances is one persistent launch of the mixed-order stage kernel
+// (stage_multi.cuh), whose blocks take tiles of every order from a work queue.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,7 +30,8 @@
 namespace dgc {
 int create_ctx(const dg_mesh_desc* mesh, const dg_phys* phys, int precision, int device, const double* elem_v0,
                const double* elem_scale, dg_ctx** out, std::string* err);
-cudaError_t enqueue_step(dg_ctx* c, int kind, double dt, cudaEvent_t* ev);
+cudaError_t enqueue_step(dg_ctx* c, double dt, bool follows);
+bool chained(const dg_ctx* c);
 cudaError_t enqueue_inject(dg_ctx* c);
 cudaError_t enqueue_finalize(dg_ctx* c, int nparts);
 dgk::StageArgs<float> stage_args_f32(dg_ctx* c, int stage, const float* y_in, float* y_out, double dt);
@@ -69,7 +69,8 @@ struct dg_batch {
   bool sources_dirty = true, observers_dirty = true;
   cudaStream_t main = nullptr;
   cudaEvent_t fork = nullptr;
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph = nullptr, graph_n = nullptr;  // one step, kBatchSteps steps
+  bool chain = false;  // the graphs' steps end with the next step's sources where a group allows it
   // one launch per RK stage for all element orders (2-D FP32, orders 2-4):
   // slot k -> group holding order k + 2 (or -1), the four stages' work-queue
   // counters, the launch's grid
@@ -93,6 +94,11 @@ int fail(dg_batch* b, int code, const std::string& m) {
     cudaError_t e_ = (x);                                                                        \
     if (e_ != cudaSuccess) return fail((b), DG_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e_)); \
   } while (0)
+
+void drop_graphs(dg_batch* b) {
+  if (b->graph) cudaGraphExecDestroy(b->graph), b->graph = nullptr;
+  if (b->graph_n) cudaGraphExecDestroy(b->graph_n), b->graph_n = nullptr;
+}
 
 // Pushes staged states, sources and observers to the group contexts.
 int sync_inputs(dg_batch* b) {
@@ -128,7 +134,7 @@ int sync_inputs(dg_batch* b) {
       if (rc) return fail(b, rc, dg_last_error(g.ctx));
     }
     b->sources_dirty = false;
-    if (b->graph) cudaGraphExecDestroy(b->graph), b->graph = nullptr;
+    drop_graphs(b);
   }
   if (b->observers_dirty) {
     for (auto& g : b->groups) {
@@ -148,7 +154,7 @@ int sync_inputs(dg_batch* b) {
       if (rc) return fail(b, rc, dg_last_error(g.ctx));
     }
     b->observers_dirty = false;
-    if (b->graph) cudaGraphExecDestroy(b->graph), b->graph = nullptr;
+    drop_graphs(b);
   }
   return DG_OK;
 }
@@ -201,31 +207,42 @@ int build_fused_graph(dg_batch* b) {
   return DG_OK;
 }
 
-// One graph per step: every group's step as a parallel branch.
-int build_graph(dg_batch* b, int64_t n_steps) {
-  for (auto& g : b->groups) {
-    int rc = dgc::ensure_out_cap(g.ctx, n_steps);
-    if (rc) return fail(b, rc, dg_last_error(g.ctx));
-  }
-  if (b->graph) return DG_OK;
-  if (b->fused) return build_fused_graph(b);
+// Steps of the longer graph.
+constexpr int kBatchSteps = 8;
+
+// A graph of `steps` steps, every group's as a parallel branch: the groups do not
+// wait for one another between steps.
+int build_order_graph(dg_batch* b, int steps) {
   cudaGraph_t graph = nullptr;
   BCK(b, cudaStreamBeginCapture(b->main, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaEventRecord(b->fork, b->main);
   for (auto& g : b->groups) {
     if (err == cudaSuccess) err = cudaStreamWaitEvent(g.ctx->stream, b->fork, 0);
     // every instance's own dt sits in its elements' step scale
-    if (err == cudaSuccess) err = dgc::enqueue_step(g.ctx, 0, 1.0, nullptr);
+    for (int i = 0; i < steps && err == cudaSuccess; ++i) err = dgc::enqueue_step(g.ctx, 1.0, i > 0);
     if (err == cudaSuccess) err = cudaEventRecord(g.join, g.ctx->stream);
     if (err == cudaSuccess) err = cudaStreamWaitEvent(b->main, g.join, 0);
   }
   cudaError_t err2 = cudaStreamEndCapture(b->main, &graph);
   if (err != cudaSuccess) return fail(b, DG_ERR_CUDA, std::string("CUDA (capture): ") + cudaGetErrorString(err));
   BCK(b, err2);
-  err = cudaGraphInstantiate(&b->graph, graph, 0);
+  err = cudaGraphInstantiate(steps == 1 ? &b->graph : &b->graph_n, graph, 0);
   cudaGraphDestroy(graph);
   BCK(b, err);
   return DG_OK;
+}
+
+int build_graph(dg_batch* b, int64_t n_steps) {
+  for (auto& g : b->groups) {
+    int rc = dgc::ensure_out_cap(g.ctx, n_steps);
+    if (rc) return fail(b, rc, dg_last_error(g.ctx));
+  }
+  b->chain = !b->fused;
+  if (b->fused) return b->graph ? DG_OK : build_fused_graph(b);
+  int rc = DG_OK;
+  if (n_steps >= kBatchSteps && !b->graph_n) rc = build_order_graph(b, kBatchSteps);
+  if (!rc && n_steps % kBatchSteps && !b->graph) rc = build_order_graph(b, 1);
+  return rc;
 }
 
 // One launch per stage works on Bernstein coefficients: a group whose kernel
@@ -246,16 +263,22 @@ int group_layouts(dg_batch* b) {
   return DG_OK;
 }
 
-int launch_steps(dg_batch* b, int64_t n_steps, cudaEvent_t* ev) {
+int launch_steps(dg_batch* b, int64_t n_steps) {
   for (auto& g : b->groups) {
     int64_t st[3] = {b->step, b->step, b->step + n_steps};
     BCK(b, cudaMemcpyAsync(g.ctx->d_step, st, sizeof(st), cudaMemcpyHostToDevice, b->main));
   }
-  for (int64_t i = 0; i < n_steps; ++i) {
-    if (ev) cudaEventRecord(ev[2 * i], b->main);
-    BCK(b, cudaGraphLaunch(b->graph, b->main));
-    if (ev) cudaEventRecord(ev[2 * i + 1], b->main);
-  }
+  for (auto& g : b->groups)
+    if (b->chain && dgc::chained(g.ctx)) {
+      cudaStream_t own = g.ctx->stream;
+      g.ctx->stream = b->main;
+      cudaError_t e = dgc::enqueue_inject(g.ctx);
+      g.ctx->stream = own;
+      BCK(b, e);
+    }
+  const int64_t many = b->fused ? 0 : n_steps / kBatchSteps;
+  for (int64_t i = 0; i < many; ++i) BCK(b, cudaGraphLaunch(b->graph_n, b->main));
+  for (int64_t i = many * kBatchSteps; i < n_steps; ++i) BCK(b, cudaGraphLaunch(b->graph, b->main));
   return DG_OK;
 }
 
@@ -374,12 +397,13 @@ int dg_batch_create(int n, const dg_mesh_desc* meshes, const dg_phys* phys, cons
       b->fused_ok = false;
     }
   }
-  // one launch per stage is the default where the batch allows it (measured
-  // faster than one kernel per order on the 256-instance ensemble: 2.33
-  // against 2.45 ms per step); DGFEM_BATCH_FUSED=0 or dg_batch_set_fused(b, 0)
-  // selects one kernel per order
+  // One launch per stage only by choice (DGFEM_BATCH_FUSED=1 or
+  // dg_batch_set_fused(b, 1)): it runs every order at the registers and shared
+  // memory of the largest, and all orders wait for one another at every stage.
+  // us per step, one launch -> branches: 2 instances (0.12M unknowns) 39 -> 17,
+  // 16 (2.3M) 102 -> 38, 48 (28M) 450 -> 309.
   const char* ev = std::getenv("DGFEM_BATCH_FUSED");
-  b->fused = b->fused_ok && !(ev && std::strcmp(ev, "0") == 0);
+  b->fused = b->fused_ok && ev && std::strcmp(ev, "1") == 0;
   if (group_layouts(b) != DG_OK) return bail(DG_ERR_CUDA, b->err);
   *out = b;
   return DG_OK;
@@ -387,7 +411,7 @@ int dg_batch_create(int n, const dg_mesh_desc* meshes, const dg_phys* phys, cons
 
 int dg_batch_destroy(dg_batch* b) {
   if (!b) return DG_OK;
-  if (b->graph) cudaGraphExecDestroy(b->graph);
+  drop_graphs(b);
   for (auto& g : b->groups) {
     if (g.join) cudaEventDestroy(g.join);
     if (g.ctx) dg_destroy(g.ctx);
@@ -405,7 +429,7 @@ int dg_batch_set_fused(dg_batch* b, int on) {
     return fail(b, DG_ERR_ARG, "one launch per stage needs FP32 2-D straight-sided instances of orders 2-4 only");
   if (b->fused != (on != 0)) {
     b->fused = on != 0;
-    if (b->graph) cudaGraphExecDestroy(b->graph), b->graph = nullptr;
+    drop_graphs(b);
     return group_layouts(b);
   }
   return DG_OK;
@@ -481,7 +505,7 @@ int dg_batch_run(dg_batch* b, int64_t n_steps, double* obs) {
   if (n_steps == 0) return DG_OK;
   int rc = sync_inputs(b);
   if (!rc) rc = build_graph(b, n_steps);
-  if (!rc) rc = launch_steps(b, n_steps, nullptr);
+  if (!rc) rc = launch_steps(b, n_steps);
   if (rc) return rc;
   BCK(b, cudaStreamSynchronize(b->main));
   b->step += n_steps;
@@ -525,21 +549,19 @@ int dg_batch_bench(dg_batch* b, int64_t n_steps, double* step_ms) {
   int rc = sync_inputs(b);
   if (!rc) rc = build_graph(b, n_steps);
   if (rc) return rc;
-  std::vector<cudaEvent_t> ev(2 * n_steps);
+  cudaEvent_t ev[2];
   for (auto& e : ev) cudaEventCreate(&e);
-  rc = launch_steps(b, n_steps, ev.data());
+  cudaEventRecord(ev[0], b->main);
+  rc = launch_steps(b, n_steps);
+  cudaEventRecord(ev[1], b->main);
   if (!rc && cudaStreamSynchronize(b->main) != cudaSuccess) rc = fail(b, DG_ERR_CUDA, "synchronize failed");
-  double tot = 0.0;
-  for (int64_t i = 0; !rc && i < n_steps; ++i) {
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ev[2 * i], ev[2 * i + 1]);
-    tot += ms;
-  }
+  float tot = 0.f;
+  if (!rc) cudaEventElapsedTime(&tot, ev[0], ev[1]);
   for (auto& e : ev) cudaEventDestroy(e);
   if (rc) return rc;
   b->step += n_steps;
   for (auto& g : b->groups) g.state_valid = false, g.ctx->step = b->step;
-  if (step_ms) *step_ms = tot / n_steps;
+  if (step_ms) *step_ms = (double)tot / n_steps;
   return DG_OK;
 }
 

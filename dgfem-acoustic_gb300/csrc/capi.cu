@@ -956,7 +956,10 @@ int select_variant(dg_ctx* c, int want) {
 
 namespace dgc {
 void set_global_error(const std::string& m) { g_create_error = m; }
-cudaError_t enqueue_step(dg_ctx* c, int kind, double dt, cudaEvent_t* ev) { return ::enqueue_step(c, kind, dt, ev); }
+cudaError_t enqueue_step(dg_ctx* c, double dt, bool follows) {
+  return ::enqueue_step(c, 0, dt, nullptr, ::chained(c), follows);
+}
+bool chained(const dg_ctx* c) { return ::chained(c); }
 cudaError_t enqueue_inject(dg_ctx* c) { return ::enqueue_inject(c); }
 cudaError_t enqueue_finalize(dg_ctx* c, int nparts) { return ::enqueue_finalize(c, nparts); }
 dgk::StageArgs<float> stage_args_f32(dg_ctx* c, int stage, const float* y_in, float* y_out, double dt) {
