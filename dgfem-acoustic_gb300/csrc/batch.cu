@@ -20,7 +20,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <exception>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "bb.cuh"
@@ -44,7 +46,11 @@ struct dg_batch {
     dg_ctx* ctx = nullptr;
     int dim = 0, order = 0, np = 0;
     std::vector<int> inst;            // member instances in order
-    std::vector<double> state;        // reference-layout staging [4][E*np]
+    // reference-layout staging [4][N], page-locked where that memory can be had:
+    // the copy of the whole group runs at the link's rate
+    double* state = nullptr;
+    int64_t N = 0;
+    bool pinned = false;
     bool state_dirty = false, state_valid = false;
     int own_variant = -2;             // kernel selected before one launch per stage took its layout (-2: none)
     cudaEvent_t join = nullptr;
@@ -100,11 +106,31 @@ void drop_graphs(dg_batch* b) {
   if (b->graph_n) cudaGraphExecDestroy(b->graph_n), b->graph_n = nullptr;
 }
 
+// The four variables' planes of n values, by a thread each where they are large:
+// a fresh array of the caller's costs as much in page faults as in copying.
+void copy_planes(double* dst, int64_t dst_stride, const double* src, int64_t src_stride, int64_t n) {
+  auto plane = [=](int q) { std::memcpy(dst + q * dst_stride, src + q * src_stride, n * sizeof(double)); };
+  std::thread t[3];
+  for (int q = 0; q < 3; ++q) {
+    if (n >= 1 << 15) {
+      try {
+        t[q] = std::thread(plane, q);
+        continue;
+      } catch (const std::exception&) {  // no thread to be had
+      }
+    }
+    plane(q);
+  }
+  plane(3);
+  for (auto& x : t)
+    if (x.joinable()) x.join();
+}
+
 // Pushes staged states, sources and observers to the group contexts.
 int sync_inputs(dg_batch* b) {
   for (auto& g : b->groups)
     if (g.state_dirty) {
-      int rc = dg_set_state(g.ctx, g.state.data());
+      int rc = dg_set_state(g.ctx, g.state);
       if (rc) return fail(b, rc, dg_last_error(g.ctx));
       g.state_dirty = false;
     }
@@ -367,7 +393,14 @@ int dg_batch_create(int n, const dg_mesh_desc* meshes, const dg_phys* phys, cons
     std::string e;
     int rc = dgc::create_ctx(&md, &ph, precision, device, v0.data(), scale.data(), &g.ctx, &e);
     if (rc) return bail(rc, e);
-    g.state.assign(4 * elem_off * g.np, 0.0);
+    g.N = elem_off * g.np;
+    g.pinned = cudaMallocHost((void**)&g.state, 4 * g.N * sizeof(double)) == cudaSuccess;
+    if (!g.pinned) {
+      cudaGetLastError();
+      g.state = (double*)std::malloc(4 * g.N * sizeof(double));
+      if (!g.state) return bail(DG_ERR_CUDA, "host memory for the state");
+    }
+    std::memset(g.state, 0, 4 * g.N * sizeof(double));
     b->total_dofs += elem_off * g.np * (g.dim + 1);
     if (cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming) != cudaSuccess) return bail(DG_ERR_CUDA, "event");
   }
@@ -415,6 +448,8 @@ int dg_batch_destroy(dg_batch* b) {
   for (auto& g : b->groups) {
     if (g.join) cudaEventDestroy(g.join);
     if (g.ctx) dg_destroy(g.ctx);
+    if (g.pinned) cudaFreeHost(g.state);
+    else std::free(g.state);
   }
   if (b->fork) cudaEventDestroy(b->fork);
   if (b->main) cudaStreamDestroy(b->main);
@@ -447,8 +482,8 @@ int dg_batch_info(const dg_batch* b, int* n_groups, int64_t* total_dofs) {
 int dg_batch_set_state(dg_batch* b, int inst, const double* u) {
   if (!b || !u || inst < 0 || inst >= (int)b->inst_group.size()) return DG_ERR_ARG;
   auto& g = b->groups[b->inst_group[inst]];
-  const int64_t N = (int64_t)g.state.size() / 4, n = b->inst_E[inst] * g.np, off = b->inst_elem_off[inst] * g.np;
-  for (int q = 0; q < 4; ++q) std::memcpy(&g.state[q * N + off], u + q * n, n * sizeof(double));
+  const int64_t n = b->inst_E[inst] * g.np, off = b->inst_elem_off[inst] * g.np;
+  copy_planes(g.state + off, g.N, u, n, n);
   g.state_dirty = true;
   return DG_OK;
 }
@@ -458,13 +493,13 @@ int dg_batch_get_state(dg_batch* b, int inst, double* u) {
   int rc = sync_inputs(b);
   if (rc) return rc;
   auto& g = b->groups[b->inst_group[inst]];
-  const int64_t N = (int64_t)g.state.size() / 4, n = b->inst_E[inst] * g.np, off = b->inst_elem_off[inst] * g.np;
+  const int64_t n = b->inst_E[inst] * g.np, off = b->inst_elem_off[inst] * g.np;
   if (!g.state_valid) {
-    rc = dg_get_state(g.ctx, g.state.data());
+    rc = dg_get_state(g.ctx, g.state);
     if (rc) return fail(b, rc, dg_last_error(g.ctx));
     g.state_valid = true;
   }
-  for (int q = 0; q < 4; ++q) std::memcpy(u + q * n, &g.state[q * N + off], n * sizeof(double));
+  copy_planes(u, n, g.state + off, g.N, n);
   return DG_OK;
 }
 

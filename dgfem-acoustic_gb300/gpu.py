@@ -214,7 +214,7 @@ class Solver:
         """State [4][E*Np] in the reference layout; into `out` (float64,
         C-contiguous, e.g. from pinned_empty) when given."""
         if out is None:
-            out = np.zeros((4, self.ndof))
+            out = np.empty((4, self.ndof))
         elif out.dtype != np.float64 or not out.flags.c_contiguous or out.size != 4 * self.ndof:
             raise ValueError("out must be a C-contiguous float64 array of 4 * E * Np values")
         self._ck(lib().dg_get_state(self.h, _dp(out)), "dg_get_state")
@@ -222,7 +222,7 @@ class Solver:
 
     def rhs(self, u, dt):
         u = np.ascontiguousarray(u, dtype=np.float64).reshape(4, self.ndof)
-        k = np.zeros_like(u)
+        k = np.empty_like(u)
         self._ck(lib().dg_rhs(self.h, _dp(u), dt, _dp(k)), "dg_rhs")
         return k
 
@@ -434,7 +434,7 @@ class Batch:
 
     def get_state(self, i):
         E, npe = self.sizes[i]
-        u = np.zeros((4, E * npe))
+        u = np.empty((4, E * npe))
         self._ck(_batch_lib().dg_batch_get_state(self.h, i, _dp(u)), "dg_batch_get_state")
         return u
 
@@ -543,13 +543,13 @@ class Network:
         self._ck(_mlp_lib().dg_mlp_set_params(self.h, _fp(p)), "dg_mlp_set_params")
 
     def get_params(self):
-        p = np.zeros(self.n_params, dtype=np.float32)
+        p = np.empty(self.n_params, dtype=np.float32)
         self._ck(_mlp_lib().dg_mlp_get_params(self.h, _fp(p)), "dg_mlp_get_params")
         return p
 
     def forward(self, x):
         x = np.ascontiguousarray(x, dtype=np.float32).reshape(-1, self.widths[0])
-        y = np.zeros((x.shape[0], self.widths[-1]), dtype=np.float32)
+        y = np.empty((x.shape[0], self.widths[-1]), dtype=np.float32)
         self._ck(_mlp_lib().dg_mlp_forward(self.h, _fp(x), x.shape[0], _fp(y)), "dg_mlp_forward")
         return y
 
@@ -559,7 +559,7 @@ class Network:
     def gradient(self, x, t):
         x = np.ascontiguousarray(x, dtype=np.float32).reshape(-1, self.widths[0])
         t = np.ascontiguousarray(t, dtype=np.float32).reshape(x.shape[0], self.widths[-1])
-        g = np.zeros(self.n_params, dtype=np.float32)
+        g = np.empty(self.n_params, dtype=np.float32)
         loss = C.c_double()
         self._ck(_mlp_lib().dg_mlp_gradient(self.h, _fp(x), _fp(t), x.shape[0], _fp(g), C.byref(loss)),
                  "dg_mlp_gradient")
