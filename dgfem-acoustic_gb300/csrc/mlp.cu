@@ -467,13 +467,15 @@ constexpr size_t mlpf_max_smem = 227 * 1024;
 bool use_fused(const dg_mlp* m) { return m->fused && !m->tc; }
 
 // Groups of 8 rows per tile (1, 2 or 4) of a fused pass over n rows: the one
-// with the least time over its waves of tiles, by what a tile of each takes
-// (mlp_fused.cuh; at 8 rows the weight stream bounds it).
+// with the least time over its waves of tiles. A wave of the surrogate's tiles
+// takes 13, 22 and 38 us (8, 16 and 32 rows: the latency of the weight stream's
+// chunks, then the matrix instructions); 2000 rows: 31, 27 and 41 us in all,
+// 3648: 43, 48 and 41, 20,000: 228, 203 and 193.
 int pick_groups(const dg_mlp* m, int64_t n, int ka, int kb, bool bwd) {
   int best = 1;
   double best_cost = 1e300;
   const int groups[3] = {1, 2, 4};
-  const double cost[3] = {10, 13, 21};
+  const double cost[3] = {13, 22, 38};
   for (int k = 0; k < 3; ++k) {
     if (mlpf::pass_smem(8 * groups[k], mlpf::stages(groups[k], bwd), ka, kb) > mlpf_max_smem) break;
     const int64_t tiles = (n + 8 * groups[k] - 1) / (8 * groups[k]);
@@ -498,7 +500,7 @@ template <bool TRAIN>
 int fused_forward(dg_mlp* m, const float* x, const int* idx, int64_t n, float* y) {
   const int k = pick_groups(m, n, m->fwd_ka, m->fwd_kb, false), rows = 8 * k;
   auto go = [&](auto kfn) {
-    kfn<<<pass_grid(m, n, rows), mlpf::kThreads, mlpf::pass_smem(rows, mlpf::stages(k, false), m->fwd_ka, m->fwd_kb), m->stream>>>(
+    kfn<<<pass_grid(m, n, rows), mlpf::kBlock, mlpf::pass_smem(rows, mlpf::stages(k, false), m->fwd_ka, m->fwd_kb), m->stream>>>(
         m->net, m->wt, m->fwd_chunks, x, idx, n, y, m->fwd_ka, m->d_err);
   };
   if (k == 1)
@@ -516,7 +518,7 @@ int fused_forward(dg_mlp* m, const float* x, const int* idx, int64_t n, float* y
 int fused_backward(dg_mlp* m, const float* t, const int* idx, int64_t n, double* loss) {
   const int k = pick_groups(m, n, m->bwd_ka, m->bwd_kb, true), rows = 8 * k, L = (int)m->w.size() - 1;
   auto go = [&](auto kfn) {
-    kfn<<<pass_grid(m, n, rows), mlpf::kThreads, mlpf::pass_smem(rows, mlpf::stages(k, true), m->bwd_ka, m->bwd_kb), m->stream>>>(
+    kfn<<<pass_grid(m, n, rows), mlpf::kBlock, mlpf::pass_smem(rows, mlpf::stages(k, true), m->bwd_ka, m->bwd_kb), m->stream>>>(
         m->net, m->wb, m->bwd_chunks, m->X[L], t, idx, n, m->bwd_ka, m->d_err);
   };
   if (k == 1)

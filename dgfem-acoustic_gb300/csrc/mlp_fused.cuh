@@ -42,7 +42,8 @@ constexpr uint32_t kChunkBytes = kKC * kNC * 2;
 // leaves beside the surrogate's activations; BWD: its 512-wide gradients)
 __host__ __device__ constexpr int stages(int NT, bool bwd) { return NT == 1 ? 5 : NT == 2 ? 4 : bwd ? 2 : 3; }
 constexpr int kCopies = 4;  // bulk copies of a chunk
-constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr int kThreads = 512, kWarps = kThreads / 32;  // that compute
+constexpr int kBlock = kThreads + 32;                  // and the warp that issues the weight stream
 constexpr int kDwN = 64, kDwK = 32, kDwB = 32, kDwGroups = 4, kDwThreads = 128 * kDwGroups, kLossBlocks = 64;
 static_assert(kWarps * 16 == kNC, "a warp per 16 outputs of a block");
 
@@ -80,64 +81,63 @@ inline size_t pass_smem(int R, int S, int ka, int kb) {
   return 128 + (size_t)S * kChunkBytes + (size_t)3 * R * (row_stride(ka) + row_stride(kb)) * 2;
 }
 
+// The computing threads' barriers (the stream's warp takes no part).
+__device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
+__device__ __forceinline__ bool sync_compute_or(bool v) {
+  int r;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.b32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.b32 %0, 1, 0, q;\n}"
+      : "=r"(r)
+      : "r"((int)v), "n"(kThreads)
+      : "memory");
+  return r != 0;
+}
+
 // The block's stream of weight chunks: `total` chunks per tile, cycled over
 // the block's tiles. Chunk i sits in slot i % kStages; full[] counts its
-// arrival, empty[] the warps that are done with it. Thread 0 issues.
+// arrival, empty[] the warps that are done with it. A warp of its own issues:
+// with a computing thread as the issuer, the others waited for its warp at the
+// end of every layer (5 of 21 us).
 template <int kStages>
 struct Stream {
   unsigned char* ring;
   uint64_t *full, *empty;
-  // computing: slot and phase of the current chunk
-  int slot;
-  uint32_t phase;
-  // issuing (thread 0): next chunk of the stream, its slot, how often that slot
-  // was used, chunks left
-  const __nv_bfloat16* src;
-  int total, at, islot, uses;
-  int64_t left;
+  int slot = 0;  // of the current chunk, and its phase
+  uint32_t phase = 0u;
 
-  __device__ void issue() {
-    dgk::mbar_expect_tx(&full[islot], kChunkBytes);
-    const __nv_bfloat16* g = src + (int64_t)at * (kKC * kNC);
-#pragma unroll
-    for (int k = 0; k < kCopies; ++k)
-      dgk::tma_load_1d(ring + (size_t)islot * kChunkBytes + k * (kChunkBytes / kCopies), g + k * (kKC * kNC / kCopies),
-                       kChunkBytes / kCopies, &full[islot]);
-    if (++at == total) at = 0;
-    if (++islot == kStages) islot = 0, ++uses;
-    --left;
-  }
-  __device__ void start(const __nv_bfloat16* s, int t, int64_t n) {
-    slot = 0, phase = 0u;
-    src = s, total = t, at = 0, islot = 0, uses = 0, left = n;
-    if (threadIdx.x == 0)
-      for (int k = 0; k < kStages && left > 0; ++k) issue();
-  }
-  // Waits for the current chunk; thread 0 first refills the slot of the chunk
-  // before it (all warps are done with that one, or about to be). False on
-  // timeout.
-  __device__ bool wait(bool first) {
+  // The issuing thread's part: n chunks. False when a slot did not come free;
+  // returns after every issued chunk has landed.
+  __device__ bool produce(const __nv_bfloat16* src, int total, int64_t n) {
+    int at = 0, sl = 0, uses = 0;  // next chunk, its slot, how often that slot was used
     bool ok = true;
-    if (threadIdx.x == 0 && !first && left > 0) {
-      ok = dgk::mbar_wait(&empty[islot], (uint32_t)(uses - 1) & 1u);
-      if (ok) issue();
+    for (; n > 0; --n) {
+      if (uses > 0 && !dgk::mbar_wait(&empty[sl], (uint32_t)(uses - 1) & 1u)) {
+        ok = false;
+        break;
+      }
+      dgk::mbar_expect_tx(&full[sl], kChunkBytes);
+      const __nv_bfloat16* g = src + (int64_t)at * (kKC * kNC);
+#pragma unroll
+      for (int k = 0; k < kCopies; ++k)
+        dgk::tma_load_1d(ring + (size_t)sl * kChunkBytes + k * (kChunkBytes / kCopies), g + k * (kKC * kNC / kCopies),
+                         kChunkBytes / kCopies, &full[sl]);
+      if (++at == total) at = 0;
+      if (++sl == kStages) sl = 0, ++uses;
     }
-    return dgk::mbar_wait(&full[slot], phase) && ok;
+    for (int s = 0; s < kStages; ++s) {
+      const int u = uses + (s < sl ? 1 : 0);
+      if (u > 0) dgk::mbar_wait(&full[s], (uint32_t)(u - 1) & 1u);
+    }
+    return ok;
   }
+  // the current chunk; false on timeout
+  __device__ bool wait() { return dgk::mbar_wait(&full[slot], phase); }
   __device__ const uint4* chunk() const { return reinterpret_cast<const uint4*>(ring + (size_t)slot * kChunkBytes); }
   __device__ void release() {
     __syncwarp();
     if ((threadIdx.x & 31) == 0)
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(dgk::smem_u32(&empty[slot])) : "memory");
     if (++slot == kStages) slot = 0, phase ^= 1u;
-  }
-  // thread 0, before the block leaves: every issued chunk has landed (the last
-  // use of each slot)
-  __device__ void drain() {
-    for (int s = 0; s < kStages; ++s) {
-      const int n = uses + (s < islot ? 1 : 0);
-      if (n > 0) dgk::mbar_wait(&full[s], (uint32_t)(n - 1) & 1u);
-    }
   }
 };
 
@@ -189,7 +189,7 @@ __device__ __forceinline__ float gelu_grad(float z) {
 }
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint4& a, uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, "
       "%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -197,7 +197,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint4& a, uint32_t
 }
 // the same from zero
 __device__ __forceinline__ void mma_bf16_0(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, "
       "%10, %10};"
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
@@ -213,41 +213,51 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16*
 // past K up to whole chunks) times weights, summed over K. The warp's 16
 // outputs: acc[t][..] holds output 16 warp + lane / 4 (+ 8 for the last two) of
 // rows 8 t + 2 (lane % 4) (+ 1 for the odd ones). False (in every thread) when
-// a chunk did not arrive. first: the block's first chunk comes next.
+// a chunk did not arrive.
 template <int NT, int S>
-__device__ __forceinline__ bool layer_block(Pass<S>& p, const Act& x, int K, bool& first, float (&acc)[NT][4]) {
+__device__ __forceinline__ bool layer_block(Pass<S>& p, const Act& x, int K, float (&acc)[NT][4]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float c[NT][4];  // middle and tail products
+  // middle and tail products, a chain each where the registers allow it
+  constexpr int NCH = NT == 4 ? 1 : 2;
+  float c[NCH][NT][4];
 #pragma unroll
   for (int t = 0; t < NT; ++t)
 #pragma unroll
-    for (int u = 0; u < 4; ++u) acc[t][u] = c[t][u] = 0.f;
+    for (int u = 0; u < 4; ++u) acc[t][u] = c[0][t][u] = c[NCH - 1][t][u] = 0.f;
   bool ok = true;
   // ldmatrix: lane's row of matrix lane / 8, whose 8 values start at step 8 (lane / 8)
   const __nv_bfloat16* xl = x.p + (lane & 7) * x.ld + (lane >> 3) * 8;
   for (int k0 = 0; k0 < K; k0 += kKC) {
-    ok = ok && p.st.wait(first);
-    first = false;
+    ok = ok && p.st.wait();
     const uint4* w = p.st.chunk() + warp * 32 + lane;
+    // H x 32 steps at a time: one ldmatrix per 8 rows, plane and 32 steps
+    constexpr int H = NT == 1 ? 2 : 1;
+    static_assert(kKC == 64, "two halves of a chunk");
 #pragma unroll
-    for (int h = 0; h < kKC / 32; ++h) {  // 32 steps: two A fragments, one ldmatrix per 8 rows and plane
-      const uint4 a0 = w[(2 * h) * (kNC / 16) * 32], a1 = w[(2 * h + 1) * (kNC / 16) * 32];
+    for (int h0 = 0; h0 < 2; h0 += H) {
+      uint4 a[2 * H];
+#pragma unroll
+      for (int h = 0; h < 2 * H; ++h) a[h] = w[(2 * h0 + h) * (kNC / 16) * 32];
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        const __nv_bfloat16* xt = xl + t * 8 * x.ld + k0 + 32 * h;
-        uint32_t b[4];
-        float d0[4], d1[4];
-        ldmatrix4(b, xt);
-        mma_bf16_0(d0, a0, b[0], b[1]);
-        mma_bf16_0(d1, a1, b[2], b[3]);
+        uint32_t b[H][3][4];
 #pragma unroll
-        for (int s = 1; s < 3; ++s) {
-          ldmatrix4(b, xt + s * x.plane);
-          mma_bf16(c[t], a0, b[0], b[1]);
-          mma_bf16(c[t], a1, b[2], b[3]);
+        for (int h = 0; h < H; ++h)
+#pragma unroll
+          for (int s = 0; s < 3; ++s) ldmatrix4(b[h][s], xl + t * 8 * x.ld + k0 + 32 * (h0 + h) + s * x.plane);
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          float d0[4], d1[4];
+          mma_bf16_0(d0, a[2 * h], b[h][0][0], b[h][0][1]);
+          mma_bf16_0(d1, a[2 * h + 1], b[h][0][2], b[h][0][3]);
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            mma_bf16(c[s % NCH][t], a[2 * h], b[h][1 + s][0], b[h][1 + s][1]);
+            mma_bf16(c[s % NCH][t], a[2 * h + 1], b[h][1 + s][2], b[h][1 + s][3]);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) acc[t][u] = (acc[t][u] + d0[u]) + d1[u];
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[t][u] = (acc[t][u] + d0[u]) + d1[u];
       }
     }
     p.st.release();
@@ -255,15 +265,15 @@ __device__ __forceinline__ bool layer_block(Pass<S>& p, const Act& x, int K, boo
 #pragma unroll
   for (int t = 0; t < NT; ++t)
 #pragma unroll
-    for (int u = 0; u < 4; ++u) acc[t][u] += c[t][u];
-  return !__syncthreads_or(!ok);
+    for (int u = 0; u < 4; ++u) acc[t][u] += NCH == 2 ? c[0][t][u] + c[NCH - 1][t][u] : c[0][t][u];
+  return !sync_compute_or(!ok);
 }
 
 // Forward pass of n rows: x [.][w0] (row idx[r] of it when idx is given) to y
 // [n][wL]; TRAIN also stores the gathered inputs, every layer's input and
 // pre-activation.
 template <int NT, bool TRAIN>
-__global__ void __launch_bounds__(kThreads, 1) k_forward(const Net net, const __nv_bfloat16* wstream, int chunks,
+__global__ void __launch_bounds__(kBlock, 1) k_forward(const Net net, const __nv_bfloat16* wstream, int chunks,
                                                          const float* __restrict__ x, const int* __restrict__ idx,
                                                          int64_t n, float* __restrict__ y, int ka, int* err) {
   constexpr int R = 8 * NT, S = stages(NT, false);
@@ -272,8 +282,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_forward(const Net net, const __
   const int tid = threadIdx.x, lane = tid & 31;
   const int oc = (tid >> 5) * 16 + (lane >> 2), rc = 2 * (lane & 3);  // this lane's first output and row
   const int64_t tiles = (n + R - 1) / R, mine = (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
-  p.st.start(wstream, chunks, mine * chunks);
-  bool ok = true, first = true;  // first: no chunk used yet
+  if (tid >= kThreads) {
+    if (tid == kThreads && !p.st.produce(wstream, chunks, mine * chunks)) atomicOr(err, 1);
+    return;
+  }
+  bool ok = true;
   for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
     const int64_t r0 = tile * R;
     const int K0 = net.w[0], K0p = up(K0, kKC);
@@ -289,26 +302,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_forward(const Net net, const __
         }
       }
     }
-    __syncthreads();
+    sync_compute();
     for (int l = 0; l < net.L && ok; ++l) {
       const int K = net.w[l], N = net.w[l + 1], Np = up(N, kKC);
       const bool last = l == net.L - 1;
       const Act xa = p.act(l & 1, K, R), xn = p.act(~l & 1, N, R);
       for (int n0 = 0; n0 < N && ok; n0 += kNC) {
-        float acc[NT][4];
-        ok = layer_block<NT, S>(p, xa, K, first, acc);
+        float acc[NT][4], bias[2];  // the biases, in flight while the block is summed
+#pragma unroll
+        for (int h = 0; h < 2; ++h) bias[h] = n0 + oc + 8 * h < N ? net.b[l][n0 + oc + 8 * h] : 0.f;
+        ok = layer_block<NT, S>(p, xa, K, acc);
         if (!ok) break;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int o = n0 + oc + 8 * h;
-          const float bias = o < N ? net.b[l][o] : 0.f;
 #pragma unroll
           for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
               const int r = 8 * t + rc + u;
               const int64_t row = r0 + r;
-              const float z = acc[t][2 * h + u] + bias;
+              const float z = acc[t][2 * h + u] + bias[h];
               if (last) {
                 if (o < N && row < n) y[row * N + o] = z;
               } else if (o < Np) {
@@ -319,13 +333,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_forward(const Net net, const __
             }
         }
       }
-      __syncthreads();  // the next layer's inputs are written, this layer's read
+      sync_compute();  // the next layer's inputs are written, this layer's read
     }
   }
-  if (tid == 0) {
-    p.st.drain();
-    if (!ok) atomicOr(err, 1);
-  }
+  if (tid == 0 && !ok) atomicOr(err, 1);
 }
 
 // Gradients with respect to every layer's pre-activation, in place of the
@@ -333,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_forward(const Net net, const __
 // idx is given): dY = 2 (y - t) / (n wL), then layer by layer
 // dZ_l = (dZ_{l+1} W_l) GELU'(Z_l).
 template <int NT>
-__global__ void __launch_bounds__(kThreads, 1) k_backward(const Net net, const __nv_bfloat16* wstream, int chunks,
+__global__ void __launch_bounds__(kBlock, 1) k_backward(const Net net, const __nv_bfloat16* wstream, int chunks,
                                                           const float* __restrict__ y, const float* __restrict__ t_,
                                                           const int* __restrict__ idx, int64_t n, int ka, int* err) {
   constexpr int R = 8 * NT, S = stages(NT, true);
@@ -344,8 +355,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_backward(const Net net, const _
   const int64_t tiles = (n + R - 1) / R, mine = (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
   const int NL = net.w[net.L];
   const float sc = 2.f / (float)(n * NL);
-  p.st.start(wstream, chunks, mine * chunks);
-  bool ok = true, first = true;  // first: no chunk used yet
+  if (tid >= kThreads) {
+    if (tid == kThreads && !p.st.produce(wstream, chunks, mine * chunks)) atomicOr(err, 1);
+    return;
+  }
+  bool ok = true;
   for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
     const int64_t r0 = tile * R;
     const int NLp = up(NL, kKC);
@@ -368,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_backward(const Net net, const _
         }
       }
     }
-    __syncthreads();
+    sync_compute();
     for (int l = net.L - 1; l >= 1 && ok; --l) {
       const int K = net.w[l + 1], N = net.w[l], Np = up(N, kKC), turn = net.L - 1 - l;
       const Act xa = p.act(turn & 1, K, R), xn = p.act(~turn & 1, N, R);
@@ -386,7 +400,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_backward(const Net net, const _
               z[h][t][u] = o < N && row < n ? net.Z[l][row * N + o] : 0.f;
             }
         float acc[NT][4];
-        ok = layer_block<NT, S>(p, xa, K, first, acc);
+        ok = layer_block<NT, S>(p, xa, K, acc);
         if (!ok) break;
 #pragma unroll
         for (int h = 0; h < 2; ++h)
@@ -404,14 +418,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_backward(const Net net, const _
               if (o < Np) xn.put(r, o, d);
             }
       }
-      __syncthreads();
+      sync_compute();
     }
-    __syncthreads();  // (one layer: the buffer is rewritten by the next tile)
+    sync_compute();  // (one layer: the buffer is rewritten by the next tile)
   }
-  if (tid == 0) {
-    p.st.drain();
-    if (!ok) atomicOr(err, 1);
-  }
+  if (tid == 0 && !ok) atomicOr(err, 1);
 }
 
 // Weight and bias gradients of every layer, dW_l = dZ_{l+1}^T X_l and the
