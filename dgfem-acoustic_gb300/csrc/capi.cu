@@ -322,6 +322,7 @@ dgk::StageArgs<T> stage_args(dg_ctx* c, int stage, const T* y_in, T* y_out, T* k
   a.stage = stage;
   a.wait_limit = c->wait_limit;
   a.pdl = c->pdl ? 1 : 0;
+  a.reverse = c->turns && (stage == 2 || stage == 4);
   a.dt = dt;
   a.c0sq = c->c0sq;
   a.ph = c->ph;
@@ -1192,6 +1193,10 @@ int dgc::create_ctx(const dg_mesh_desc* mesh, const dg_phys* phys, int precision
   if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_perm, c->np * sizeof(int));
   if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_perm, c->perm_c2i.data(), c->np * sizeof(int), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_ref, 4 * c->E * c->np * sizeof(double));
+  // what a stage leaves in L2 is worth turning round for (stage_bb.cuh)
+  int l2 = 0;
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device);
+  c->turns = precision == DG_FP32 && (int64_t)c->nv * c->Epad * c->np * 4 <= l2;
   c->max_grid = std::max(c->grid, 2 * c->num_sms);
   for (int v = 0; v < 8; ++v) {
     dgk::Stage2Info si = stage2_info(c, v);

@@ -128,6 +128,7 @@ struct dg_ctx {
   } persist;
   // per-step graph
   cudaGraphExec_t graph = nullptr, graph_n = nullptr;  // one step, kGraphSteps steps
+  bool turns = false;  // alternate stages take the tiles in opposite directions
   bool pdl = false;  // the next stage launch is a programmatic dependent of the kernel before it
   double graph_dt = 0.0;
   int graph_kind = -1;  // 0 = RK4, 1 = Euler

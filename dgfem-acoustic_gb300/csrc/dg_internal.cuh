@@ -157,6 +157,7 @@ struct StageArgs {
   int ntiles;
   int stage;       // 0: k only, 1..4: RK4 stages, 5: Euler (y_out = u + k)
   int wait_limit;  // polling rounds of a bounded device wait before it gives up
+  int reverse;     // tiles from the last to the first (stage_bb.cuh)
   int pdl;         // launched as a programmatic dependent of the kernel before it (stage_bb.cuh)
   double dt;
   double c0sq;

@@ -1073,17 +1073,24 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB>::NT, MINB) stage_bb
     for (int b = 0; b < NBUF; ++b) mbar_init(&bar[b], 1);
     fence_mbar_init();
   }
+  // Alternate stages may go through the tiles in opposite directions, so that what
+  // the stage before touched last is still in L2. For FP32 states of up to an L2:
+  // 196,608 tetrahedra of order 3 (63 MB) 284 -> 275 us per step, 614,400 triangles
+  // of order 2 (44 MB) 168 -> 166; 254,016 tetrahedra of order 4 (142 MB) 703 ->
+  // 709, and FP64 kernels, which do not wait for memory, 0.5 % slower.
+  auto tile_at = [&](int i) { return a.reverse ? a.ntiles - 1 - i : i; };
   // what no kernel before this one writes is fetched while they drain
-  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue_geometry(blockIdx.x, 0);
+  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue_geometry(tile_at(blockIdx.x), 0);
   bb_load_tables<C>(a, sFm, sNb, tid, C::NT);
   grid_dependency_wait();
   __syncthreads();
-  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue_state(blockIdx.x, 0);
+  if (tid == 0 && (int)blockIdx.x < a.ntiles) issue_state(tile_at(blockIdx.x), 0);
 
   BBRes<T> racc;
   bool ok = true;
   int it = 0;
-  for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ++it) {
+  for (int i = blockIdx.x; i < a.ntiles; i += gridDim.x, ++it) {
+    const int tile = tile_at(i);
     const int b = NBUF == 2 ? it & 1 : 0;
     const bool got = mbar_wait(&bar[b], (NBUF == 2 ? it >> 1 : it) & 1, a.wait_limit);
     if (__syncthreads_or(!got)) {  // also: every thread is done with the previous tile
@@ -1091,11 +1098,11 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB>::NT, MINB) stage_bb
       if (tid == 0) mbar_wait(&bar[b], (NBUF == 2 ? it >> 1 : it) & 1);  // drained (full limit)
       break;
     }
-    const int next = tile + gridDim.x;
+    const int next = i + gridDim.x;
     auto issue_next = [&]() {
       if (tid == 0 && next < a.ntiles) {
         fence_proxy_async();
-        issue(next, NBUF == 2 ? b ^ 1 : 0);
+        issue(tile_at(next), NBUF == 2 ? b ^ 1 : 0);
       }
     };
     if constexpr (NBUF == 2) issue_next();
