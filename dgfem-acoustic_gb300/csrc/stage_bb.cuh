@@ -164,6 +164,11 @@ struct BBCfg {
   static constexpr size_t oGI = oGF + (size_t)NBUF * GB;
   static constexpr size_t oN = oGI + (size_t)NBUF * IB;                 // [NF][NV][NFP][32]
   static constexpr bool FX = sizeof(T) == 8;  // lift and elevation in fixed point (bb_tile_fx)
+  // the gradient in fixed point as well (fx_gradient): in 3-D, where the pressure's
+  // thread has sixteen products per coefficient, up to order 3; in 2-D it cost
+  // registers and gained nothing (order 3: 47.5 -> 51.5 us per step), and neither
+  // did the fluxes in 3-D (381 -> 626 us, spilled registers)
+  static constexpr bool FXG = FX && D == 3 && P <= 3;
   static constexpr size_t oX = oN + (size_t)NF * NV * NFP * LW * sizeof(T);  // int [NF][NV][32]: exponents (FX)
   static constexpr size_t oR = oX + (FX ? (size_t)NF * NV * LW * 4 : 0);
   static constexpr size_t bytes = oR + NV * NV * sizeof(double);
@@ -623,7 +628,8 @@ __device__ __forceinline__ bool bb_tile(const StageArgs<T>& a, Env& env, int64_t
 // and the result is rounded to FP64 once. Weights grow a value by at most
 // (P+1)(P+3) in L0, 5 in the layers and 4 over the faces, 2^9.5 at P = 4, which
 // leaves the sign bit. An infinity or NaN makes the whole sum a NaN. 3-D p = 3:
-// 285 FP64 operations per thread instead of 740.
+// 180 FP64 operations per thread (with the gradient, see fx_gradient) instead of
+// 740.
 
 __device__ __forceinline__ int fx_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 
@@ -714,8 +720,8 @@ __device__ __forceinline__ void fx_layers(const long long (&prev)[bb_np(C::D - 1
 // The gradient's coefficients t (degree P-1) of variable q's volume term: the
 // volume term is -elevation(t) (bb_volume without the elevation).
 template <class C>
-__device__ __forceinline__ void fx_gradient(const double* y, const double* g, int q, double rhoc2, double inv_rho0,
-                                            double (&t)[bb_np(C::D, C::P - 1)]) {
+__device__ __forceinline__ void fp64_gradient(const double* y, const double* g, int q, double rhoc2, double inv_rho0,
+                                              double (&t)[bb_np(C::D, C::P - 1)]) {
   constexpr int D = C::D, P = C::P, NP = C::NP, LW = C::LW;
   BBGrad<double, D> gv;
 #pragma unroll
@@ -748,6 +754,129 @@ __device__ __forceinline__ void fx_gradient(const double* y, const double* g, in
     }
     t[decltype(b_)::value] = s;
   });
+}
+
+// A fixed-point value as two digits, hi 2^29 + lo, both of its sign: sums and
+// differences are taken digit by digit, and a product is three 32-bit
+// multiply-adds (that of the low digits, 2^-57 of the largest, is left out).
+struct FxDigits {
+  int hi, lo;
+};
+// x as a multiple of 2^(E - 1075 - X), below 2^(53 + X) in size
+template <int X>
+__device__ __forceinline__ FxDigits fx_digits(double x, int E) {
+  const int h = __double2hiint(x), e = (h >> 20) & 0x7ff;
+  unsigned long long m =
+      ((unsigned long long)(((unsigned)h & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x);
+  if (e == 0) m = 0;
+  m = (m << X) >> min(E - e, 63);
+  const FxDigits d{(int)(m >> 29), (int)((unsigned)m & 0x1fffffffu)};
+  return h < 0 ? FxDigits{-d.hi, -d.lo} : d;
+}
+// v 2^-d rounded, d of either sign (the caller's value has room to grow)
+__device__ __forceinline__ long long fx_scaled(long long v, int d) { return d >= 0 ? fx_shift(v, d) : v << min(-d, 62); }
+
+template <bool FXG>
+struct FxPick {
+  using type = double;
+};
+template <>
+struct FxPick<true> {
+  using type = long long;
+};
+// The biased exponent that covers values v in units of 2^U, E at least.
+template <int N>
+__device__ __forceinline__ int fx_top(const long long (&v)[N], int U, int E) {
+  unsigned long long m = 0;
+#pragma unroll
+  for (int n = 0; n < N; ++n) m |= (unsigned long long)(v[n] < 0 ? -v[n] : v[n]);
+  return m == 0 ? E : min(max(E, U + 64 - __clzll((long long)m) + 1022), 0x7ff);
+}
+__device__ __forceinline__ int fx_size(double x) { return __double2hiint(x) & 0x7fffffff; }
+__device__ __forceinline__ int fx_group(int m) { return max(m >> 20, kFxMinExp); }  // exponent of the largest fx_size
+// The unit of products of state digits (exponent Ey) and metric digits (Eg).
+__device__ __forceinline__ int fx_unit(int Ey, int Eg) { return Ey - 1079 + Eg - 1080 + 58; }
+// A sum of products of digits.
+struct FxSum {
+  long long hh = 0, tt = 0;
+  __device__ __forceinline__ void add(const FxDigits& d, const FxDigits& g) {
+    hh += (long long)d.hi * g.hi;
+    tt += (long long)d.hi * g.lo + (long long)d.lo * g.hi;
+  }
+  __device__ __forceinline__ long long get() const { return hh + ((tt + (1 << 28)) >> 29); }
+};
+
+// The gradient's coefficients t (degree P-1) of variable q's volume term, in
+// units of 2^U: the volume term is -elevation(t) (bb_volume without the
+// elevation). bad: an infinity or NaN among the inputs.
+//
+// In fixed point too: the state's coefficients take 57 bits below the largest
+// exponent among those of the element, the metric 58, so that sums of nine
+// products of coefficient differences stay below 2^63. A multiply-add takes an
+// SM sub-partition 64 cycles in FP64 and some 10 here, a conversion some 30. us
+// per step: 24,576 tetrahedra of order 3 374 -> 339, 48,000 of order 2 352 -> 310,
+// 48,000 of order 1 155 -> 146, 7,722 of order 2 67 -> 64.
+template <class C>
+__device__ __forceinline__ void fx_gradient(const double* y, const double* g, int q, double rhoc2, double inv_rho0,
+                                            long long (&t)[bb_np(C::D, C::P - 1)], int& U, bool& bad) {
+  constexpr int D = C::D, P = C::P, NP = C::NP, LW = C::LW, NB = bb_np(D, P - 1);
+  auto top = [&](const double* c, int m) {
+#pragma unroll
+    for (int n = 0; n < NP; ++n) m = max(m, fx_size(c[n * LW]));
+    return m;
+  };
+  FxSum sum[NB];
+  // adds sum_r G_r (c[b + e_r] - c[b + e_0]) of one variable's coefficients
+  auto add = [&](const double* v, int E, const FxDigits (&G)[D]) {
+    FxDigits c[NP];
+#pragma unroll
+    for (int n = 0; n < NP; ++n) c[n] = fx_digits<4>(v[n * LW], E);
+    bb_for<NB>([&](auto b_) {
+      constexpr int b = decltype(b_)::value;
+      using L = BLat<D, P - 1, b>;
+      constexpr int n0 = bb_index(D, P, bb_add(L::b, 0, 1));
+      bb_for<D>([&](auto r_) {
+        constexpr int r = decltype(r_)::value;
+        constexpr int n = bb_index(D, P, bb_add(L::b, r + 1, 1));
+        sum[b].add(FxDigits{c[n].hi - c[n0].hi, c[n].lo - c[n0].lo}, G[r]);
+      });
+    });
+  };
+  // this variable along the mean flow
+  FxDigits G[D];
+  int m = 0;
+#pragma unroll
+  for (int r = 0; r < D; ++r) m = max(m, fx_size(g[(C::oGV + r) * LW]));
+  const int Ev = fx_group(m), Ey = fx_group(top(y + q * NP * LW, 0));
+#pragma unroll
+  for (int r = 0; r < D; ++r) G[r] = fx_digits<5>(g[(C::oGV + r) * LW], Ev);
+  add(y + q * NP * LW, Ey, G);
+#pragma unroll
+  for (int b = 0; b < NB; ++b) t[b] = sum[b].get(), sum[b] = FxSum();
+  // the velocity's divergence, or the pressure's derivative
+  const int nv = q == 0 ? D : 1;
+  const double scale = q == 0 ? rhoc2 : inv_rho0;
+  auto metric = [&](int v, int r) { return scale * g[(C::oG + r * D + (q == 0 ? v : q - 1)) * LW]; };
+  int mo = 0;
+  m = 0;
+#pragma unroll 1
+  for (int v = 0; v < nv; ++v) {
+    mo = top(y + (q == 0 ? 1 + v : 0) * NP * LW, mo);
+#pragma unroll
+    for (int r = 0; r < D; ++r) m = max(m, fx_size(metric(v, r)));
+  }
+  const int Eo = fx_group(mo), Eg = fx_group(m);
+#pragma unroll 1
+  for (int v = 0; v < nv; ++v) {
+#pragma unroll
+    for (int r = 0; r < D; ++r) G[r] = fx_digits<5>(metric(v, r), Eg);
+    add(y + (q == 0 ? 1 + v : 0) * NP * LW, Eo, G);
+  }
+  const int U1 = fx_unit(Ey, Ev), U2 = fx_unit(Eo, Eg);
+  U = max(U1, U2);
+  bad = max(max(Ey, Ev), max(Eo, Eg)) == 0x7ff;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) t[b] = fx_shift(t[b], U - U1) + fx_shift(sum[b].get(), U - U2);
 }
 
 // One tile of an FP64 state (see above): bb_tile with fluxes and gradient in
@@ -783,8 +912,14 @@ __device__ __forceinline__ bool bb_tile_fx(const StageArgs<double>& a, Env& env,
       for (int i = 0; i < 5; ++i) bc[i] = __ldg(a.bbC + (int64_t)nbr * 8 + i);
   }
   // ---- this variable's gradient ----
-  double t[bb_np(D, P - 1)];
-  fx_gradient<C>(y, g, role, rhoc2, inv_rho0, t);
+  using Grad = typename FxPick<C::FXG>::type;
+  Grad t[bb_np(D, P - 1)];
+  int tU = 0;
+  bool bad = false;
+  if constexpr (C::FXG)
+    fx_gradient<C>(y, g, role, rhoc2, inv_rho0, t, tU, bad);
+  else
+    fp64_gradient<C>(y, g, role, rhoc2, inv_rho0, t);
   if constexpr (Env::kTraceLast) trace();
   // ---- this face's flux ----
   {
@@ -859,14 +994,22 @@ __device__ __forceinline__ bool bb_tile_fx(const StageArgs<double>& a, Env& env,
   int E = kFxMinExp, ef[NF];
 #pragma unroll
   for (int f = 0; f < NF; ++f) ef[f] = sX[(f * NV + role) * LW + lane], E = max(E, ef[f]);
+  if constexpr (C::FXG) {
+    E = bad ? 0x7ff : fx_top(t, tU, E);
+  } else {
 #pragma unroll
-  for (int b = 0; b < bb_np(D, P - 1); ++b) E = max(E, fx_exponent(t[b]));
+    for (int b = 0; b < bb_np(D, P - 1); ++b) E = max(E, fx_exponent(t[b]));
+  }
   long long acc[NP];
 #pragma unroll
   for (int n = 0; n < NP; ++n) acc[n] = 0;
   bb_for<bb_np(D, P - 1)>([&](auto b_) {
     using L = BLat<D, P - 1, decltype(b_)::value>;
-    const long long v = fx_fix(t[decltype(b_)::value], E);
+    long long v;
+    if constexpr (C::FXG)
+      v = fx_scaled(t[decltype(b_)::value], E - 1075 - tU);
+    else
+      v = fx_fix(t[decltype(b_)::value], E);
     bb_for<D + 1>([&](auto k_) {
       constexpr int k = decltype(k_)::value;
       constexpr int n = bb_index(D, P, bb_add(L::b, k, 1));
