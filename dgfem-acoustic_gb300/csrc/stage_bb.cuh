@@ -149,6 +149,10 @@ struct BBCfg {
   // Q4 (FP32, 3-D): the four variables of a coefficient side by side,
   // [tile][coefficient][32][4], else one plane each, [tile][variable][coefficient][32]
   static constexpr bool Q4 = sizeof(T) == 4 && D == 3;
+  // packed FP32 arithmetic for two variables in the fluxes and two metric columns
+  // in the volume term: 131,712 tetrahedra of order 4 361 -> 344 us per step, whose
+  // instructions bound them; at order 3 its register pairs cost more (271 -> 276)
+  static constexpr bool PACK2 = Q4 && P == 4;
   static constexpr int SQ = Q4 ? 1 : NP * LW, SN = Q4 ? 4 * LW : LW, SE = Q4 ? 4 : 1;  // word strides
   // word in the tile of the first coefficient that a thread owns in the update
   __host__ __device__ static constexpr int first_word(int tid, int role) { return Q4 ? tid : role * NP * LW + (tid & 31); }
@@ -271,6 +275,24 @@ __device__ __forceinline__ T bb_stencil_at(const T (&f)[C::NFP]) {
       constexpr int n = bb_index(D - 1, P, bb_add(bb_add(L::b, i, 1), j, -1));
       constexpr int w = (L::b.a[i] + 1) * L::b.a[j];
       s += (T)w * f[n];
+    }
+  });
+  return s;
+}
+// the same for two variables at once, in packed FP32 instructions
+template <class C, int M>
+__device__ __forceinline__ float2 bb_stencil_at(const float2 (&f)[C::NFP]) {
+  constexpr int D = C::D, P = C::P;
+  using L = BLat<D - 1, P, M>;
+  constexpr int w0 = (L::b.a[0] + 1) * (L::b.a[0] + 1) + (L::b.a[1] + 1) * (L::b.a[1] + 1) +
+                     (D == 3 ? (L::b.a[2] + 1) * (L::b.a[2] + 1) : 0);
+  float2 s = __fmul2_rn(make_float2((float)w0, (float)w0), f[M]);
+  bb_for<D * D>([&](auto ij_) {
+    constexpr int i = decltype(ij_)::value / D, j = decltype(ij_)::value % D;
+    if constexpr (i != j && L::b.a[j] > 0) {
+      constexpr int n = bb_index(D - 1, P, bb_add(bb_add(L::b, i, 1), j, -1));
+      constexpr int w = (L::b.a[i] + 1) * L::b.a[j];
+      s = __ffma2_rn(make_float2((float)w, (float)w), f[n], s);
     }
   });
   return s;
@@ -1076,6 +1098,7 @@ __device__ __forceinline__ bool bb_tile_q4(const StageArgs<float>& a, Env& env, 
   float out[NP];
   {
     float gv[3], H[3][3];
+    float2 h01[3], h2v[3];  // PACK2: (H_0, H_1) and (H_2, the metric along the mean flow)
 #pragma unroll
     for (int r = 0; r < 3; ++r) gv[r] = g[(C::oGV + r) * LW + el];
 #pragma unroll
@@ -1085,6 +1108,9 @@ __device__ __forceinline__ bool bb_tile_q4(const StageArgs<float>& a, Env& env, 
         const float x = g[(C::oG + r * D + j) * LW + el];
         H[j][r] = q == 0 ? inv_rho0 * x : q == j + 1 ? rhoc2 * x : 0.f;
       }
+    if constexpr (C::PACK2)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) h01[r] = make_float2(H[0][r], H[1][r]), h2v[r] = make_float2(H[2][r], gv[r]);
 #pragma unroll
     for (int n = 0; n < NP; ++n) out[n] = 0.f;
     const float* yq = y + tid;
@@ -1093,10 +1119,21 @@ __device__ __forceinline__ bool bb_tile_q4(const StageArgs<float>& a, Env& env, 
       constexpr int n0 = bb_index(D, P, bb_add(L::b, 0, 1)), n1 = bb_index(D, P, bb_add(L::b, 1, 1)),
                     n2 = bb_index(D, P, bb_add(L::b, 2, 1)), n3 = bb_index(D, P, bb_add(L::b, 3, 1));
       const float c0 = yq[n0 * SN], d1 = yq[n1 * SN] - c0, d2 = yq[n2 * SN] - c0, d3 = yq[n3 * SN] - c0;
-      float t = gv[0] * d1 + gv[1] * d2 + gv[2] * d3;
+      float t;
+      if constexpr (C::PACK2) {
+        const float2 e1 = make_float2(d1, d1), e2 = make_float2(d2, d2), e3 = make_float2(d3, d3);
+        const float2 a01 = __ffma2_rn(h01[2], e3, __ffma2_rn(h01[1], e2, __fmul2_rn(h01[0], e1)));
+        const float2 a2v = __ffma2_rn(h2v[2], e3, __ffma2_rn(h2v[1], e2, __fmul2_rn(h2v[0], e1)));
+        t = a2v.y;
+        t += __shfl_xor_sync(0xffffffffu, a01.x, 1);
+        t += __shfl_xor_sync(0xffffffffu, a01.y, 2);
+        t += __shfl_xor_sync(0xffffffffu, a2v.x, 3);
+      } else {
+        t = gv[0] * d1 + gv[1] * d2 + gv[2] * d3;
 #pragma unroll
-      for (int j = 0; j < 3; ++j)
-        t += __shfl_xor_sync(0xffffffffu, H[j][0] * d1 + H[j][1] * d2 + H[j][2] * d3, j + 1);
+        for (int j = 0; j < 3; ++j)
+          t += __shfl_xor_sync(0xffffffffu, H[j][0] * d1 + H[j][1] * d2 + H[j][2] * d3, j + 1);
+      }
       bb_for<D + 1>([&](auto k_) {
         constexpr int k = decltype(k_)::value;
         constexpr int n = bb_index(D, P, bb_add(L::b, k, 1));
@@ -1110,39 +1147,77 @@ __device__ __forceinline__ bool bb_tile_q4(const StageArgs<float>& a, Env& env, 
   {
     const float* gf = g + role * (D + 1) * LW + lane;
     const int* fm = sFm + role * 16;
-    float f[4][NFP];
-    const float* yl = y + 4 * lane;
-    if (boundary) {
-      const float* Bg = a.bbM + (int64_t)nbr * 16;
+    if constexpr (C::PACK2) {
+      float2 f01[NFP], f23[NFP];
+      const float* yl = y + 4 * lane;
+      if (boundary) {
+        const float* Bg = a.bbM + (int64_t)nbr * 16;
 #pragma unroll
-      for (int m = 0; m < NFP; ++m) {
-        const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
+        for (int m = 0; m < NFP; ++m) {
+          const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
+          float f[4];
 #pragma unroll
-        for (int v = 0; v < 4; ++v)
-          f[v][m] = __ldg(Bg + v * 4) * um.x + __ldg(Bg + v * 4 + 1) * um.y + __ldg(Bg + v * 4 + 2) * um.z +
-                    __ldg(Bg + v * 4 + 3) * um.w;
+          for (int v = 0; v < 4; ++v)
+            f[v] = __ldg(Bg + v * 4) * um.x + __ldg(Bg + v * 4 + 1) * um.y + __ldg(Bg + v * 4 + 2) * um.z +
+                   __ldg(Bg + v * 4 + 3) * um.w;
+          f01[m] = make_float2(f[0], f[1]), f23[m] = make_float2(f[2], f[3]);
+        }
+      } else {
+        const float A = gf[D * LW], n0 = gf[0], n1 = gf[LW], n2 = gf[2 * LW];
+        const float p0 = rhoc2 * n0, p1 = rhoc2 * n1, p2 = rhoc2 * n2;
+        const float2 A2 = make_float2(A, A), c01 = make_float2(p0, inv_rho0 * n0),
+                     u12 = make_float2(inv_rho0 * n1, inv_rho0 * n2), neg = make_float2(-1.f, -1.f);
+#pragma unroll
+        for (int m = 0; m < NFP; ++m) {
+          const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
+          const float2 d01 = __ffma2_rn(neg, make_float2(up[m].x, up[m].y), make_float2(um.x, um.y));
+          const float2 d23 = __ffma2_rn(neg, make_float2(up[m].z, up[m].w), make_float2(um.z, um.w));
+          f01[m] = __ffma2_rn(c01, make_float2(d01.y, d01.x), __fmul2_rn(A2, d01));
+          f01[m].x += p1 * d23.x + p2 * d23.y;
+          f23[m] = __ffma2_rn(u12, make_float2(d01.x, d01.x), __fmul2_rn(A2, d23));
+        }
       }
+      float* sf = sN + role * NFP * SN + 4 * lane;
+      bb_for<NFP>([&](auto m_) {
+        constexpr int m = decltype(m_)::value;
+        const float2 s01 = bb_stencil_at<C, m>(f01), s23 = bb_stencil_at<C, m>(f23);
+        *reinterpret_cast<float4*>(sf + m * SN) = make_float4(s01.x, s01.y, s23.x, s23.y);
+      });
     } else {
-      const float A = gf[D * LW], n0 = gf[0], n1 = gf[LW], n2 = gf[2 * LW];
-      const float p0 = rhoc2 * n0, p1 = rhoc2 * n1, p2 = rhoc2 * n2;
-      const float u0 = inv_rho0 * n0, u1 = inv_rho0 * n1, u2 = inv_rho0 * n2;
+      float f[4][NFP];
+      const float* yl = y + 4 * lane;
+      if (boundary) {
+        const float* Bg = a.bbM + (int64_t)nbr * 16;
 #pragma unroll
-      for (int m = 0; m < NFP; ++m) {
-        const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
-        const float dp = um.x - up[m].x, dx = um.y - up[m].y, dy = um.z - up[m].z, dz = um.w - up[m].w;
-        f[0][m] = A * dp + p0 * dx + p1 * dy + p2 * dz;
-        f[1][m] = A * dx + u0 * dp;
-        f[2][m] = A * dy + u1 * dp;
-        f[3][m] = A * dz + u2 * dp;
+        for (int m = 0; m < NFP; ++m) {
+          const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
+#pragma unroll
+          for (int v = 0; v < 4; ++v)
+            f[v][m] = __ldg(Bg + v * 4) * um.x + __ldg(Bg + v * 4 + 1) * um.y + __ldg(Bg + v * 4 + 2) * um.z +
+                      __ldg(Bg + v * 4 + 3) * um.w;
+        }
+      } else {
+        const float A = gf[D * LW], n0 = gf[0], n1 = gf[LW], n2 = gf[2 * LW];
+        const float p0 = rhoc2 * n0, p1 = rhoc2 * n1, p2 = rhoc2 * n2;
+        const float u0 = inv_rho0 * n0, u1 = inv_rho0 * n1, u2 = inv_rho0 * n2;
+#pragma unroll
+        for (int m = 0; m < NFP; ++m) {
+          const float4 um = *reinterpret_cast<const float4*>(yl + fm[m]);
+          const float dp = um.x - up[m].x, dx = um.y - up[m].y, dy = um.z - up[m].z, dz = um.w - up[m].w;
+          f[0][m] = A * dp + p0 * dx + p1 * dy + p2 * dz;
+          f[1][m] = A * dx + u0 * dp;
+          f[2][m] = A * dy + u1 * dp;
+          f[3][m] = A * dz + u2 * dp;
+        }
       }
+      float* sf = sN + role * NFP * SN + 4 * lane;
+      bb_for<NFP>([&](auto m_) {
+        constexpr int m = decltype(m_)::value;
+        *reinterpret_cast<float4*>(sf + m * SN) =
+            make_float4(bb_stencil_at<C, m>(f[0]), bb_stencil_at<C, m>(f[1]), bb_stencil_at<C, m>(f[2]),
+                        bb_stencil_at<C, m>(f[3]));
+      });
     }
-    float* sf = sN + role * NFP * SN + 4 * lane;
-    bb_for<NFP>([&](auto m_) {
-      constexpr int m = decltype(m_)::value;
-      *reinterpret_cast<float4*>(sf + m * SN) =
-          make_float4(bb_stencil_at<C, m>(f[0]), bb_stencil_at<C, m>(f[1]), bb_stencil_at<C, m>(f[2]),
-                      bb_stencil_at<C, m>(f[3]));
-    });
   }
   const float dte = a.f_dt * g[C::oS * LW + el];
   if (!env.sync()) return false;
