@@ -26,7 +26,7 @@
 // bounds its stages by their count, which the fixed-point sums (bb_tile_fx,
 // fx_gradient) quarter. Measured per RK4 step against the nodal kernels' best:
 // 196,608 tetrahedra of order 3, FP32, 0.61 -> 0.27 ms (floor 0.15); 131,712 of
-// order 4, FP32, 0.61 -> 0.37 (0.17); 24,576 of order 3, FP64, 2.24 -> 0.34
+// order 4, FP32, 0.61 -> 0.34 (0.17); 24,576 of order 3, FP64, 2.24 -> 0.34
 // (0.05); 125,000 triangles of order 4, FP32, 0.14 -> 0.085 (0.054).
 //
 // Layout: arrays of tiles of 32 elements, [tile][variable][coefficient][32]:
