@@ -9,13 +9,13 @@
 // (FP32 master copies for the optimiser), activations and gradients in FP32,
 // every sum accumulated in FP32.
 //
-// Networks whose widths are all at most 1024 run the fused passes of
-// mlp_fused.cuh: one launch for the forward pass, one for the chain of input
-// gradients, one for all weight gradients and the loss, one for the optimiser
-// step with every weight copy. Measured against one GEMM per layer (GB300, the
+// Networks whose layers fit beside the weight stream in shared memory (pass_fits)
+// run the fused passes of mlp_fused.cuh: one launch for the forward pass, one for
+// the chain of input gradients, one for all weight gradients and the loss, one for
+// the optimiser step with every weight copy. Measured against one GEMM per layer (GB300, the
 // 6-256-256-256-256-512 network): forward of 2000 rows on the device 95 -> 29
 // us, a training step of 256 rows 680 -> 79 us.
-// Wider networks, and dg_mlp_set_tensor_cores, use per-layer kernels: one GEMM
+// Other networks, and dg_mlp_set_tensor_cores, use per-layer kernels: one GEMM
 // serves the three products of a layer, Z = X W^T (forward), dX = dZ W (input
 // gradient) and dW = dZ^T X (weight gradient), on the CUDA cores (k_gemm: 64 x
 // 64 output tile, 16-deep K slices staged in shared memory, 4 x 4 outputs per
@@ -365,9 +365,10 @@ struct dg_mlp {
   int* bidx = nullptr;
   int64_t n_data = 0, bcap = 0;
   int64_t step = 0;  // Adam steps taken
-  // fused passes (mlp_fused.cuh; every width within kMaxWidth): the weights in
-  // the order the forward and the backward pass read them, the loss's ticket
-  bool fused = false;
+  // fused passes (mlp_fused.cuh): whether the forward pass fits, and whether the
+  // backward pass does too; the weights in the order the passes read them, the
+  // loss's ticket
+  bool fused = false, fused_bwd = false;
   mlpf::Net net{};
   __nv_bfloat16 *wt = nullptr, *wb = nullptr;
   int fwd_chunks = 0, bwd_chunks = 0;
@@ -464,7 +465,16 @@ int check_gemm_waits(dg_mlp* m) {
 
 constexpr size_t mlpf_max_smem = 227 * 1024;
 
-bool use_fused(const dg_mlp* m) { return m->fused && !m->tc; }
+// (train: the forward pass keeps the layers' inputs for the backward pass, which
+// is fused as well)
+bool use_fused(const dg_mlp* m, bool train) { return m->fused && (m->fused_bwd || !train) && !m->tc; }
+
+// Whether a pass's activations in the smallest tiles fit beside its weight
+// stream: the widest layer of each of the two buffers, which take the layers in
+// turn, rounded up to 64 and summed up to 1408.
+bool pass_fits(int ka, int kb, bool bwd) {
+  return mlpf::pass_smem(8, mlpf::stages(1, bwd), ka, kb) <= mlpf_max_smem;
+}
 
 // Groups of 8 rows per tile (1, 2 or 4) of a fused pass over n rows: the one
 // with the least time over its waves of tiles. A wave of the surrogate's tiles
@@ -565,6 +575,8 @@ cudaError_t fused_setup(dg_mlp* m) {
     net.goff[l] = go;
     go += (int64_t)((K + mlpf::kNC - 1) / mlpf::kNC) * mlpf::up(N, mlpf::kKC) * mlpf::kNC;
   }
+  if (!pass_fits(m->fwd_ka, m->fwd_kb, false)) return cudaSuccess;
+  m->fused_bwd = pass_fits(m->bwd_ka, m->bwd_kb, true);
   const int64_t cw = mlpf::kKC * mlpf::kNC;
   m->fwd_chunks = (int)(to / cw), m->bwd_chunks = (int)(go / cw);
   cudaError_t e = cudaMalloc(&m->wt, to * sizeof(__nv_bfloat16));
@@ -602,10 +614,11 @@ int refresh_bf16(dg_mlp* m) {
   return DG_OK;
 }
 
-// Forward pass of n rows already in X[0]; output in X[L].
-int forward(dg_mlp* m, int64_t n) {
+// Forward pass of n rows already in X[0]; output in X[L]. train: before
+// backward(), which reads every layer's input and pre-activation.
+int forward(dg_mlp* m, int64_t n, bool train) {
   const int L = (int)m->w.size() - 1;
-  if (use_fused(m)) return fused_forward<false>(m, m->X[0], nullptr, n, m->X[L]);
+  if (!train && use_fused(m, false)) return fused_forward<false>(m, m->X[0], nullptr, n, m->X[L]);
   for (int l = 0; l < L; ++l) {
     const int K = m->w[l], N = m->w[l + 1];
     const bool last = l == L - 1;
@@ -746,7 +759,7 @@ int dg_mlp_forward_device(dg_mlp* m, const float* x, int64_t n, float* y, void* 
   // other blocks write theirs: arrays that overlap go through a copy of x
   const uintptr_t xb = (uintptr_t)x, xe = (uintptr_t)(x + n * m->w.front());
   const uintptr_t yb = (uintptr_t)y, ye = (uintptr_t)(y + n * m->w.back());
-  if (use_fused(m) && (xe <= yb || ye <= xb)) {
+  if (use_fused(m, false) && (xe <= yb || ye <= xb)) {
     cudaStream_t keep = m->stream;
     if (stream) m->stream = (cudaStream_t)stream;
     const int rc = fused_forward<false>(m, x, nullptr, n, y);
@@ -760,7 +773,7 @@ int dg_mlp_forward_device(dg_mlp* m, const float* x, int64_t n, float* y, void* 
   m->stream = s;
   const int L = (int)m->w.size() - 1;
   cudaError_t e = cudaMemcpyAsync(m->X[0], x, n * m->w[0] * sizeof(float), cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess) rc = forward(m, n);
+  if (e == cudaSuccess) rc = forward(m, n, false);
   if (e == cudaSuccess && rc == DG_OK)
     e = cudaMemcpyAsync(y, m->X[L], n * m->w[L] * sizeof(float), cudaMemcpyDeviceToDevice, s);
   m->stream = keep;
@@ -775,7 +788,7 @@ int dg_mlp_forward(dg_mlp* m, const float* x, int64_t n, float* y) {
   if (rc != DG_OK) return rc;
   const int L = (int)m->w.size() - 1;
   MCK(m, cudaMemcpyAsync(m->X[0], x, n * m->w[0] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-  rc = forward(m, n);
+  rc = forward(m, n, false);
   if (rc != DG_OK) return rc;
   MCK(m, cudaMemcpyAsync(y, m->X[L], n * m->w[L] * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
   return check_gemm_waits(m);
@@ -789,12 +802,12 @@ int dg_mlp_gradient(dg_mlp* m, const float* x, const float* t, int64_t n, float*
   if (rc != DG_OK) return rc;
   const int L = (int)m->w.size() - 1;
   MCK(m, cudaMemcpyAsync(m->X[0], x, n * m->w[0] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-  if (use_fused(m)) rc = fused_forward<true>(m, m->X[0], nullptr, n, m->X[L]);
+  if (use_fused(m, true)) rc = fused_forward<true>(m, m->X[0], nullptr, n, m->X[L]);
   MCK(m, cudaMemcpyAsync(m->by, t, n * m->w[L] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-  if (use_fused(m)) {
+  if (use_fused(m, true)) {
     if (rc == DG_OK) rc = fused_backward(m, m->by, nullptr, n, m->loss);
   } else {
-    rc = forward(m, n);
+    rc = forward(m, n, true);
     if (rc == DG_OK) rc = mse(m, m->by, n);
     if (rc == DG_OK) rc = backward(m, n);
   }
@@ -828,7 +841,7 @@ int dg_mlp_train(dg_mlp* m, int64_t n_steps, int batch, double lr, double lr_fin
   int rc = ensure_cap(m, batch);
   if (rc != DG_OK) return rc;
   const int L = (int)m->w.size() - 1;
-  if (!use_fused(m)) rc = ensure_targets(m, batch);
+  if (!use_fused(m, true)) rc = ensure_targets(m, batch);
   if (rc != DG_OK) return rc;
   // one permutation of the training rows per epoch, drawn on the host
   const int64_t nd = m->n_data, steps_per_epoch = nd / batch;
@@ -849,13 +862,13 @@ int dg_mlp_train(dg_mlp* m, int64_t n_steps, int batch, double lr, double lr_fin
       if (e != cudaSuccess) break;
     }
     const int* idx = m->bidx + within * batch;
-    if (use_fused(m)) {
+    if (use_fused(m, true)) {
       rc = fused_forward<true>(m, m->tx, idx, batch, m->X[L]);
       if (rc == DG_OK) rc = fused_backward(m, m->ty, idx, batch, d_losses + s);
     } else {
       k_gather_rows<<<nblk((int64_t)batch * m->w[0], 256), 256, 0, m->stream>>>(m->tx, idx, batch, m->w[0], m->X[0]);
       k_gather_rows<<<nblk((int64_t)batch * m->w[L], 256), 256, 0, m->stream>>>(m->ty, idx, batch, m->w[L], m->by);
-      rc = forward(m, batch);
+      rc = forward(m, batch, true);
       if (rc == DG_OK) rc = mse(m, m->by, batch);
       if (rc == DG_OK) e = cudaMemcpyAsync(d_losses + s, m->loss, sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
       if (rc == DG_OK && e == cudaSuccess) rc = backward(m, batch);

@@ -35,7 +35,7 @@
 namespace mlpf {
 
 constexpr int kMaxLayers = 16;
-constexpr int kMaxWidth = 1024;  // activations of 4 rows and the weight stream fit in shared memory
+constexpr int kMaxWidth = 1024;  // of any layer (pass_fits in mlp.cu bounds the two buffers together)
 constexpr int kKC = 64, kNC = 256;  // contraction steps and outputs of one weight chunk
 constexpr uint32_t kChunkBytes = kKC * kNC * 2;
 // chunks in flight of a pass with NT groups of 8 rows (what shared memory

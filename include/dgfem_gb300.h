@@ -326,8 +326,11 @@ int dg_mlp_train(dg_mlp* m, int64_t n_steps, int batch, double lr, double lr_fin
 /* on != 0: the layers as single GEMMs on the tensor cores (tcgen05
  * kind::tf32, activations and gradients as TF32 head + tail, BF16 weights exact
  * in TF32, FP32 accumulation). 0, the default and the faster: the fused passes
- * (every width at most 1024; activations as exact sums of three BF16 values,
- * FP32 accumulation), wider networks as single GEMMs on the CUDA cores. A wait
+ * (activations as exact sums of three BF16 values, FP32 accumulation) where
+ * every width is at most 1024 and the widest even and the widest odd layer,
+ * rounded up to 64, sum to at most 1408 (counted from the inputs for the
+ * forward pass, from the outputs for gradients and training), other networks
+ * as single GEMMs on the CUDA cores. A wait
  * for weights or MMAs that runs out makes the synchronous calls return
  * DG_ERR_TIMEOUT. */
 int dg_mlp_set_tensor_cores(dg_mlp* m, int on);
