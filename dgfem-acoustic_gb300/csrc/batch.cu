@@ -259,13 +259,19 @@ int build_order_graph(dg_batch* b, int steps) {
 }
 
 int build_graph(dg_batch* b, int64_t n_steps) {
+  // a run longer than any before gets new result buffers: the graphs hold the
+  // old ones' addresses
+  int rc = DG_OK;
+  bool moved = false;
   for (auto& g : b->groups) {
-    int rc = dgc::ensure_out_cap(g.ctx, n_steps);
-    if (rc) return fail(b, rc, dg_last_error(g.ctx));
+    const int64_t cap = g.ctx->out_cap;
+    if (!rc && (rc = dgc::ensure_out_cap(g.ctx, n_steps))) fail(b, rc, dg_last_error(g.ctx));
+    moved |= rc || g.ctx->out_cap != cap;
   }
+  if (moved) drop_graphs(b);
+  if (rc) return rc;
   b->chain = !b->fused;
   if (b->fused) return b->graph ? DG_OK : build_fused_graph(b);
-  int rc = DG_OK;
   if (n_steps >= kBatchSteps && !b->graph_n) rc = build_order_graph(b, kBatchSteps);
   if (!rc && n_steps % kBatchSteps && !b->graph) rc = build_order_graph(b, 1);
   return rc;
