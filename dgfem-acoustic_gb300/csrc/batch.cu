@@ -37,6 +37,7 @@ bool chained(const dg_ctx* c);
 cudaError_t enqueue_inject(dg_ctx* c);
 cudaError_t enqueue_finalize(dg_ctx* c, int nparts);
 dgk::StageArgs<float> stage_args_f32(dg_ctx* c, int stage, const float* y_in, float* y_out, double dt);
+int set_state_elems(dg_ctx* c, const double* u, int64_t e0, int64_t e1);
 int ensure_out_cap(dg_ctx* c, int64_t n);
 void set_global_error(const std::string& m);
 }  // namespace dgc
@@ -58,6 +59,7 @@ struct dg_batch {
   std::vector<Group> groups;
   std::vector<int> inst_group;
   std::vector<int64_t> inst_elem_off, inst_E;
+  std::vector<char> inst_dirty;  // its part of the staging is to go to the device
   // per-instance sources and observers (instance-local dofs)
   struct Src {
     std::vector<int64_t> off{0}, dofs;
@@ -128,10 +130,21 @@ void copy_planes(double* dst, int64_t dst_stride, const double* src, int64_t src
 
 // Pushes staged states, sources and observers to the group contexts.
 int sync_inputs(dg_batch* b) {
+  // (only what was set: after a run the staging of the other instances is old)
   for (auto& g : b->groups)
     if (g.state_dirty) {
-      int rc = dg_set_state(g.ctx, g.state);
-      if (rc) return fail(b, rc, dg_last_error(g.ctx));
+      for (size_t j = 0; j < g.inst.size();) {
+        size_t k = j;
+        while (k < g.inst.size() && b->inst_dirty[g.inst[k]]) ++k;
+        if (k > j) {
+          const int64_t e0 = b->inst_elem_off[g.inst[j]];
+          const int64_t e1 = b->inst_elem_off[g.inst[k - 1]] + b->inst_E[g.inst[k - 1]];
+          const int rc = dgc::set_state_elems(g.ctx, g.state, e0, e1);
+          if (rc) return fail(b, rc, dg_last_error(g.ctx));
+        }
+        j = k + 1;
+      }
+      for (int i : g.inst) b->inst_dirty[i] = 0;
       g.state_dirty = false;
     }
   if (b->sources_dirty) {
@@ -341,6 +354,7 @@ int dg_batch_create(int n, const dg_mesh_desc* meshes, const dg_phys* phys, cons
   b->inst_group.assign(n, -1);
   b->inst_elem_off.assign(n, 0);
   b->inst_E.assign(n, 0);
+  b->inst_dirty.assign(n, 0);
   b->src.assign(n, {});
   b->obs.assign(n, {});
   std::map<std::pair<int, int>, int> gid;
@@ -490,6 +504,7 @@ int dg_batch_set_state(dg_batch* b, int inst, const double* u) {
   auto& g = b->groups[b->inst_group[inst]];
   const int64_t n = b->inst_E[inst] * g.np, off = b->inst_elem_off[inst] * g.np;
   copy_planes(g.state + off, g.N, u, n, n);
+  b->inst_dirty[inst] = 1;
   g.state_dirty = true;
   return DG_OK;
 }

@@ -21,22 +21,23 @@ Lay lay(const dg_ctx* c) {
   return c->prec == DG_FP32 && c->dim == 3 ? Lay{1, 4 * LW, 4, tw} : Lay{c->np * LW, LW, 1, tw};
 }
 
-// Reference layout -> tiles. One block per (tile, variable): the tile's
-// nodal values through shared memory (the reference layout is
+// Reference layout -> tiles, elements e0 to e1 - 1 (e1 = E: and the padding).
+// One block per (tile, variable) from e0's tile on: the tile's nodal values through shared memory (the reference layout is
 // element-major), one warp per coefficient row.
 template <typename T>
 __global__ void __launch_bounds__(128) k_ref_to_bb(const double* __restrict__ ref, T* __restrict__ out,
                                                    const int* __restrict__ perm, const int* __restrict__ ptr,
                                                    const int* __restrict__ col, const double* __restrict__ val,
-                                                   int64_t E, int np, Lay l) {
+                                                   int64_t E, int np, Lay l, int64_t first, int64_t end) {
   __shared__ double x[35 * (LW + 1)];
-  const int64_t tile = blockIdx.x, e0 = tile * LW;
+  const int64_t tile = first / LW + blockIdx.x, e0 = tile * LW;
   const int q = blockIdx.y, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < np * LW; i += blockDim.x) {
     const int e = i / np, n = i - e * np;
     x[perm[n] * (LW + 1) + e] = e0 + e < E ? ref[q * E * np + (e0 + e) * np + n] : 0.0;
   }
   __syncthreads();
+  if (e0 + lane < first || (e0 + lane >= end && end < E)) return;
   T* o = out + tile * l.tw + q * l.sq + lane * l.se;
   for (int r = threadIdx.x >> 5; r < np; r += blockDim.x >> 5) {
     double s = 0.0;
@@ -173,14 +174,14 @@ int bb_setup_basis(dg_ctx* c) {
   return e == cudaSuccess ? DG_OK : DG_ERR_CUDA;
 }
 
-cudaError_t bb_from_ref(dg_ctx* c, const double* ref, void* out) {
-  const dim3 grid((unsigned)(c->Epad / LW), c->nv);
+cudaError_t bb_from_ref(dg_ctx* c, const double* ref, void* out, int64_t e0, int64_t e1) {
+  const dim3 grid((unsigned)(((e1 == c->E ? c->Epad : e1) + LW - 1) / LW - e0 / LW), c->nv);
   const int *p = c->bb_int + c->bb_iptr[1], *k = c->bb_int + c->bb_icol[1];
   const double* v = c->bb_dbl + c->bb_ival[1];
   if (c->prec == DG_FP32)
-    k_ref_to_bb<float><<<grid, 128, 0, c->stream>>>(ref, (float*)out, c->d_perm, p, k, v, c->E, c->np, lay(c));
+    k_ref_to_bb<float><<<grid, 128, 0, c->stream>>>(ref, (float*)out, c->d_perm, p, k, v, c->E, c->np, lay(c), e0, e1);
   else
-    k_ref_to_bb<double><<<grid, 128, 0, c->stream>>>(ref, (double*)out, c->d_perm, p, k, v, c->E, c->np, lay(c));
+    k_ref_to_bb<double><<<grid, 128, 0, c->stream>>>(ref, (double*)out, c->d_perm, p, k, v, c->E, c->np, lay(c), e0, e1);
   return cudaGetLastError();
 }
 

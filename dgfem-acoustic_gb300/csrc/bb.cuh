@@ -14,8 +14,9 @@ int64_t bb_slot(const dg_ctx* c, int64_t e, int n);
 int64_t bb_var_stride(const dg_ctx* c);
 // Basis tables (c->bb_V, bb_Vinv and their device copies).
 int bb_setup_basis(dg_ctx* c);
-// reference layout [4][E*np] (c->d_ref or another device array) -> tiles, every lane of the padding cleared; and back
-cudaError_t bb_from_ref(dg_ctx* c, const double* ref, void* out);
+// reference layout [4][E*np] (c->d_ref or another device array) -> tiles, elements e0 to e1 - 1 (up to E: every
+// lane of the padding cleared); and back
+cudaError_t bb_from_ref(dg_ctx* c, const double* ref, void* out, int64_t e0, int64_t e1);
 cudaError_t bb_to_ref(dg_ctx* c, const void* in, double* ref);
 // Hard overwrite of the pressure at source nodes, for elements' coefficients.
 cudaError_t bb_inject(dg_ctx* c);

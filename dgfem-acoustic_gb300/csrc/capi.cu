@@ -35,16 +35,19 @@ inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 // auxiliary kernels
 // ---------------------------------------------------------------------------
 
-// reference layout [4][E*np] (double, mesh local node order) -> internal
+// reference layout [4][E*np] (double, mesh local node order) -> internal,
+// elements e0 to e1 - 1
 template <typename T>
-__global__ void k_ref_to_int(const double* ref, T* out, const int* perm, int64_t E, int np, int nv, int64_t stride) {
+__global__ void k_ref_to_int(const double* ref, T* out, const int* perm, int64_t E, int np, int nv, int64_t stride,
+                             int64_t e0, int64_t e1) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= (int64_t)nv * E * np) return;
-  int q = (int)(i / (E * np));
-  int64_t r = i - (int64_t)q * E * np;
+  const int64_t m = (e1 - e0) * np;
+  if (i >= nv * m) return;
+  int q = (int)(i / m);
+  int64_t r = e0 * np + i - q * m;
   int64_t e = r / np;
   int n = (int)(r - e * np);
-  out[q * stride + e * np + perm[n]] = (T)ref[i];
+  out[q * stride + e * np + perm[n]] = (T)ref[q * E * np + r];
 }
 
 template <typename T>
@@ -729,13 +732,16 @@ cudaError_t int_to_ref(dg_ctx* c, const void* in, double* ref) {
   return cudaGetLastError();
 }
 
-cudaError_t ref_to_int(dg_ctx* c, const double* ref, void* out) {
-  if (c->bb) return bb_from_ref(c, ref, out);
-  const int64_t m = (int64_t)c->nv * c->E * c->np, stride = c->Epad * c->np;
+// Elements e0 to e1 - 1; the others keep what they have.
+cudaError_t ref_to_int(dg_ctx* c, const double* ref, void* out, int64_t e0, int64_t e1) {
+  if (c->bb) return bb_from_ref(c, ref, out, e0, e1);
+  const int64_t m = c->nv * (e1 - e0) * c->np, stride = c->Epad * c->np;
   if (c->prec == DG_FP32)
-    k_ref_to_int<float><<<nblk(m, 256), 256, 0, c->stream>>>(ref, (float*)out, c->d_perm, c->E, c->np, c->nv, stride);
+    k_ref_to_int<float><<<nblk(m, 256), 256, 0, c->stream>>>(ref, (float*)out, c->d_perm, c->E, c->np, c->nv, stride, e0,
+                                                             e1);
   else
-    k_ref_to_int<double><<<nblk(m, 256), 256, 0, c->stream>>>(ref, (double*)out, c->d_perm, c->E, c->np, c->nv, stride);
+    k_ref_to_int<double><<<nblk(m, 256), 256, 0, c->stream>>>(ref, (double*)out, c->d_perm, c->E, c->np, c->nv, stride,
+                                                              e0, e1);
   return cudaGetLastError();
 }
 
@@ -755,16 +761,22 @@ double* mapped(const double* p, int64_t n) {
   return (double*)a.devicePointer;
 }
 
-// A host array in the reference layout -> out, and in -> a host array (on
-// c->stream).
-int host_to_int(dg_ctx* c, const double* u, void* out) {
-  const int64_t n = 4 * c->E * c->np;
+// A host array in the reference layout -> out (elements e0 to e1 - 1 of it), and
+// in -> a host array (on c->stream).
+int host_to_int(dg_ctx* c, const double* u, void* out, int64_t e0, int64_t e1) {
+  const int64_t N = c->E * c->np, n = 4 * N;
   const double* ref = mapped(u, n);
   if (!ref) {
-    CK(c, cudaMemcpyAsync(c->d_ref, u, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    if (e1 - e0 == c->E) {
+      CK(c, cudaMemcpyAsync(c->d_ref, u, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    } else {
+      for (int64_t q = 0; q < c->nv; ++q)
+        CK(c, cudaMemcpyAsync(c->d_ref + q * N + e0 * c->np, u + q * N + e0 * c->np, (e1 - e0) * c->np * sizeof(double),
+                              cudaMemcpyHostToDevice, c->stream));
+    }
     ref = c->d_ref;
   }
-  CK(c, ref_to_int(c, ref, out));
+  CK(c, ref_to_int(c, ref, out, e0, e1));
   return DG_OK;
 }
 int int_to_host(dg_ctx* c, const void* in, double* u) {
@@ -786,7 +798,7 @@ int apply_layout(dg_ctx* c) {
     CK(c, int_to_ref(c, x, c->d_ref));
     if (!want) CK(c, cudaMemsetAsync(x, 0, nb, c->stream));
     c->bb = want;
-    CK(c, ref_to_int(c, c->d_ref, x));
+    CK(c, ref_to_int(c, c->d_ref, x, 0, c->E));
   }
   // what the other layout left in the work arrays is no state
   for (void* x : {c->acc, c->y0, c->y1, c->kbuf}) CK(c, cudaMemsetAsync(x, 0, nb, c->stream));
@@ -1006,6 +1018,7 @@ dgk::StageArgs<double> stage_args_f64(dg_ctx* c, int stage, const double* y_in, 
   return ::stage_args<double>(c, stage, y_in, y_out, nullptr, dt);
 }
 int ensure_out_cap(dg_ctx* c, int64_t n) { return ::ensure_out_cap(c, n); }
+int set_state_elems(dg_ctx* c, const double* u, int64_t e0, int64_t e1);
 int create_ctx(const dg_mesh_desc* mesh, const dg_phys* phys, int precision, int device, const double* elem_v0,
                const double* elem_scale, dg_ctx** out, std::string* err);
 
@@ -1268,6 +1281,25 @@ int dgc::create_ctx(const dg_mesh_desc* mesh, const dg_phys* phys, int precision
   return DG_OK;
 }
 
+int dgc::set_state_elems(dg_ctx* c, const double* u, int64_t e0, int64_t e1) {
+  if (c->dim == 2)
+    for (int64_t i = (3 * c->E + e0) * c->np; i < (3 * c->E + e1) * c->np; ++i)
+      if (u[i] != 0.0) return fail(c, DG_ERR_ARG, "2-D state must have vz = 0");
+  // the padding elements past E take part in every stage (their geometry is
+  // zero, so a finite state stays zero there); they are cleared so that a
+  // non-finite state of an earlier run cannot stay behind in them
+  if (c->Epad > c->E && !c->bb && e1 == c->E) {
+    const size_t w = c->prec == DG_FP32 ? 4 : 8;
+    for (int q = 0; q < c->nv; ++q)
+      CK(c, cudaMemsetAsync((char*)c->u + ((size_t)q * c->Epad + c->E) * c->np * w, 0,
+                            (size_t)(c->Epad - c->E) * c->np * w, c->stream));
+  }
+  const int rc = host_to_int(c, u, c->u, e0, e1);
+  if (rc) return rc;
+  CK(c, cudaStreamSynchronize(c->stream));
+  return DG_OK;
+}
+
 extern "C" {
 
 int dg_destroy(dg_ctx* c) {
@@ -1294,23 +1326,7 @@ int dg_get_info(const dg_ctx* c, dg_info_t* info) {
 
 int dg_set_state(dg_ctx* c, const double* u) {
   if (!c || !u) return DG_ERR_ARG;
-  const int64_t n = 4 * c->E * c->np;
-  if (c->dim == 2)
-    for (int64_t i = 3 * c->E * c->np; i < n; ++i)
-      if (u[i] != 0.0) return fail(c, DG_ERR_ARG, "2-D state must have vz = 0");
-  // the padding elements past E take part in every stage (their geometry is
-  // zero, so a finite state stays zero there); they are cleared so that a
-  // non-finite state of an earlier run cannot stay behind in them
-  if (c->Epad > c->E && !c->bb) {
-    const size_t w = c->prec == DG_FP32 ? 4 : 8;
-    for (int q = 0; q < c->nv; ++q)
-      CK(c, cudaMemsetAsync((char*)c->u + ((size_t)q * c->Epad + c->E) * c->np * w, 0,
-                            (size_t)(c->Epad - c->E) * c->np * w, c->stream));
-  }
-  const int rc = host_to_int(c, u, c->u);
-  if (rc) return rc;
-  CK(c, cudaStreamSynchronize(c->stream));
-  return DG_OK;
+  return dgc::set_state_elems(c, u, 0, c->E);
 }
 
 int dg_get_state(dg_ctx* c, double* u) {
@@ -1454,7 +1470,7 @@ int dg_set_step_index(dg_ctx* c, int64_t step) {
 
 int dg_rhs(dg_ctx* c, const double* u, double dt, double* k) {
   if (!c || !u || !k) return DG_ERR_ARG;
-  int rc = host_to_int(c, u, c->y1);
+  int rc = host_to_int(c, u, c->y1, 0, c->E);
   if (rc) return rc;
   CK(c, launch_stage(c, 0, c->y1, nullptr, c->kbuf, dt));
   rc = int_to_host(c, c->kbuf, k);

@@ -52,3 +52,32 @@ def test_a_longer_run_after_a_shorter_one(pkg, prec, fused):
         assert rel_l2(B.get_state(k), S.get_state()) <= tol, k
         S.close()
     B.close()
+
+
+@pytest.mark.parametrize("variant", ["", "-1"])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("which", [(2,), (0, 4), (0, 2, 4)])
+def test_state_of_some_instances_after_a_run(pkg, monkeypatch, which, prec, variant):
+    if variant:
+        monkeypatch.setenv("DGFEM_STAGE_VARIANT", variant)
+    B, meshes = _batch(pkg, prec)
+    A, _ = _batch(pkg, prec)
+    for k, m in enumerate(meshes):
+        u = smooth_state(m, seed=k)
+        A.set_state(k, u)
+        B.set_state(k, u)
+    A.run(5)
+    B.run(5)
+    want = [A.get_state(k) for k in range(A.n)]
+    for k in which:
+        B.set_state(k, smooth_state(meshes[k], seed=10 + k))
+    got = [B.get_state(k) for k in range(B.n)]
+    tol = 4e-14 if prec == "fp64" else 2e-6  # of a change of basis, as in test_gpu_host_arrays.py
+    for k in range(B.n):
+        if k in which:
+            u = smooth_state(meshes[k], seed=10 + k)
+            assert np.max(np.abs(got[k] - u)) <= tol * np.max(np.abs(u)), k
+        else:
+            np.testing.assert_array_equal(got[k], want[k])
+    A.close()
+    B.close()
