@@ -750,6 +750,7 @@ cudaError_t ref_to_int(dg_ctx* c, const double* ref, void* out, int64_t e0, int6
 // rate (193 to 210 GB/s, as the copy engine), in place of a copy before or after
 // (254,016 tetrahedra of order 4: 2.1 -> 1.5 ms, the link's 1.47 ms).
 double* mapped(const double* p, int64_t n) {
+  if ((uintptr_t)p % alignof(double)) return nullptr;  // (a copy takes any address, a kernel's loads do not)
   cudaPointerAttributes a{}, b{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, p + n - 1) != cudaSuccess) {
     cudaGetLastError();
