@@ -2,6 +2,8 @@
 // state I/O in the reference layout, sources, observers, the per-step CUDA
 // graph (source injection -> four fused RK4 stages -> residual and observer
 // reductions) and benchmarking.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -748,17 +750,34 @@ cudaError_t ref_to_int(dg_ctx* c, const double* ref, void* out, int64_t e0, int6
 // Device address of n values of page-locked host memory at p, or null: the
 // conversion kernels then read or write them over the link themselves, at its
 // rate (193 to 210 GB/s, as the copy engine), in place of a copy before or after
-// (254,016 tetrahedra of order 4: 2.1 -> 1.5 ms, the link's 1.47 ms).
+// (254,016 tetrahedra of order 4: 2.1 -> 1.5 ms, the link's 1.47 ms). One
+// allocation or registration has to hold them all: with unified addresses the
+// ends of two with pageable memory between them are as far apart as the values.
 double* mapped(const double* p, int64_t n) {
   if ((uintptr_t)p % alignof(double)) return nullptr;  // (a copy takes any address, a kernel's loads do not)
-  cudaPointerAttributes a{}, b{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, p + n - 1) != cudaSuccess) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
-      (const double*)b.devicePointer - (const double*)a.devicePointer != n - 1)
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+  using Get = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const Get get = []() -> Get {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) == cudaSuccess &&
+        found == cudaDriverEntryPointSuccess)
+      return (Get)f;
+    cudaGetLastError();
     return nullptr;
+  }();
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  if (!get || get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) != CUDA_SUCCESS ||
+      get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS)
+    return nullptr;
+  const CUdeviceptr d = (CUdeviceptr)a.devicePointer;
+  if (d < start || d - start > size || (uint64_t)n > (size - (d - start)) / sizeof(double)) return nullptr;
   return (double*)a.devicePointer;
 }
 

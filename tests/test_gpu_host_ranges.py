@@ -34,3 +34,42 @@ def test_page_locked_array_off_the_values_alignment(pkg, off, variant):
     S.get_state(out=odd)
     assert np.array_equal(odd, want)
     S.close()
+
+
+def test_two_registrations_with_pageable_memory_between(pkg):
+    """Such an array is refused, as a copy refuses it; one registration of all of it is taken."""
+    torch = pytest.importorskip("torch")
+    rt, page = torch.cuda.cudart(), 65536
+    S, u = _solver(pkg, counts=30)
+    S.set_state(u)
+    want = S.get_state()
+    k = S.rhs(u, 1e-4)
+    raw = np.empty(u.nbytes + 2 * page, np.uint8)
+    start = -raw.ctypes.data % page
+    arr = raw[start:start + u.nbytes].view(np.float64).reshape(u.shape)
+    arr[:] = u
+    ptr, last = arr.ctypes.data, (u.nbytes - 1) // page * page
+    assert last >= 4 * page
+    for p, n in ((ptr, page), (ptr + last, u.nbytes - last)):
+        assert int(rt.cudaHostRegister(p, n, 0)) == 0
+    try:
+        with pytest.raises(pkg.gpu.SolverError, match="DG_ERR_CUDA"):
+            S.set_state(arr)
+        with pytest.raises(pkg.gpu.SolverError, match="DG_ERR_CUDA"):
+            S.rhs(arr, 1e-4)
+        with pytest.raises(pkg.gpu.SolverError, match="DG_ERR_CUDA"):
+            S.get_state(out=arr)
+    finally:
+        for p in (ptr, ptr + last):
+            assert int(rt.cudaHostUnregister(p)) == 0
+    assert np.array_equal(arr, u) and np.array_equal(S.get_state(), want)
+    assert int(rt.cudaHostRegister(raw.ctypes.data, raw.nbytes, 0)) == 0
+    try:
+        S.set_state(np.zeros_like(u))
+        S.set_state(arr)
+        assert np.array_equal(S.rhs(arr, 1e-4), k)
+        S.get_state(out=arr)
+        assert np.array_equal(arr, want)
+    finally:
+        assert int(rt.cudaHostUnregister(raw.ctypes.data)) == 0
+    S.close()
