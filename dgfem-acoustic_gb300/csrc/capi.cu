@@ -1445,7 +1445,11 @@ int dg_set_observers(dg_ctx* c, int n_obs, const int64_t* offsets, const int64_t
   if (!c || n_obs < 0 || (n_obs > 0 && !offsets)) return DG_ERR_ARG;
   if (n_obs > 0 && offsets[n_obs] > 0 && (!dofs || !weights))
     return fail(c, DG_ERR_ARG, "dg_set_observers: dofs or weights is null");
-  const int64_t total = n_obs > 0 ? offsets[n_obs] : 0, ndof = c->E * c->np;
+  const int64_t total = n_obs > 0 ? std::max<int64_t>(offsets[n_obs], 0) : 0, ndof = c->E * c->np;
+  // (a range that ends where or before it starts holds nothing)
+  for (int o = 0; o < n_obs; ++o)
+    if (offsets[o] < offsets[o + 1] && (offsets[o] < 0 || offsets[o + 1] > total))
+      return fail(c, DG_ERR_ARG, "observer offsets out of range");
   std::vector<int64_t> hd(total);
   for (int64_t k = 0; k < total; ++k) {
     int64_t d = dofs[k];
