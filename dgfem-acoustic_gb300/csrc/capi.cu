@@ -482,10 +482,14 @@ int ensure_out_cap(dg_ctx* c, int64_t n) {
   if (c->d_res) cudaFree(c->d_res);
   if (c->d_obs) cudaFree(c->d_obs);
   c->d_res = nullptr, c->d_obs = nullptr;
-  CK(c, cudaMalloc(&c->d_res, cap * 5 * sizeof(double)));
-  CK(c, cudaMalloc(&c->d_obs, cap * std::max(1, c->n_obs) * 4 * sizeof(double)));
-  c->out_cap = cap;
+  // no room until both are there: a shorter run after a failure allocates again
+  c->out_cap = 0;
   drop_graphs(c);
+  cudaError_t e = cudaMalloc(&c->d_res, cap * 5 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&c->d_obs, cap * std::max(1, c->n_obs) * 4 * sizeof(double));
+  if (e != cudaSuccess) cudaGetLastError();
+  CK(c, e);
+  c->out_cap = cap;
   return DG_OK;
 }
 
