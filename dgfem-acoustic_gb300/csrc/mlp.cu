@@ -403,18 +403,26 @@ int max_width(const dg_mlp* m) {
 
 int ensure_cap(dg_mlp* m, int64_t n) {
   if (n <= m->cap) return DG_OK;
+  m->cap = 0;  // until all are there: fewer rows after a failure allocate again
   for (float* q : m->X) cudaFree(q);
   for (float* q : m->Z) cudaFree(q);
   cudaFree(m->dA), cudaFree(m->dB);
+  m->dA = m->dB = nullptr;
   m->X.assign(m->w.size(), nullptr);
   m->Z.assign(m->w.size(), nullptr);
   const int L = (int)m->w.size() - 1;
+  cudaError_t e = cudaSuccess;
+  auto get = [&](float** p, int width) {
+    if (e == cudaSuccess) e = cudaMalloc(p, n * width * sizeof(float));
+  };
   for (int l = 0; l <= L; ++l) {
-    MCK(m, cudaMalloc(&m->X[l], n * m->w[l] * sizeof(float)));
-    if (l >= 1) MCK(m, cudaMalloc(&m->Z[l], n * m->w[l] * sizeof(float)));
+    get(&m->X[l], m->w[l]);
+    if (l >= 1) get(&m->Z[l], m->w[l]);
   }
-  MCK(m, cudaMalloc(&m->dA, n * max_width(m) * sizeof(float)));
-  MCK(m, cudaMalloc(&m->dB, n * max_width(m) * sizeof(float)));
+  get(&m->dA, max_width(m));
+  get(&m->dB, max_width(m));
+  if (e != cudaSuccess) cudaGetLastError();
+  MCK(m, e);
   for (int l = 0; l <= L; ++l) m->net.X[l] = m->X[l], m->net.Z[l] = m->Z[l];
   m->cap = n;
   return DG_OK;
@@ -425,7 +433,9 @@ int ensure_targets(dg_mlp* m, int64_t n) {
   if (n <= m->bcap) return DG_OK;
   cudaFree(m->by);
   m->by = nullptr, m->bcap = 0;
-  MCK(m, cudaMalloc(&m->by, n * m->w.back() * sizeof(float)));
+  const cudaError_t e = cudaMalloc(&m->by, n * m->w.back() * sizeof(float));
+  if (e != cudaSuccess) cudaGetLastError();
+  MCK(m, e);
   m->bcap = n;
   return DG_OK;
 }
@@ -823,8 +833,11 @@ int dg_mlp_set_data(dg_mlp* m, const float* x, const float* t, int64_t n) {
   const int L = (int)m->w.size() - 1;
   cudaFree(m->tx), cudaFree(m->ty);
   m->tx = m->ty = nullptr;
-  MCK(m, cudaMalloc(&m->tx, n * m->w[0] * sizeof(float)));
-  MCK(m, cudaMalloc(&m->ty, n * m->w[L] * sizeof(float)));
+  m->n_data = 0;
+  cudaError_t e = cudaMalloc(&m->tx, n * m->w[0] * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&m->ty, n * m->w[L] * sizeof(float));
+  if (e != cudaSuccess) cudaGetLastError();
+  MCK(m, e);
   MCK(m, cudaMemcpyAsync(m->tx, x, n * m->w[0] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
   MCK(m, cudaMemcpyAsync(m->ty, t, n * m->w[L] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
   MCK(m, cudaStreamSynchronize(m->stream));

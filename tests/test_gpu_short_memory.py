@@ -34,3 +34,28 @@ def test_run_after_one_whose_results_do_not_fit(pkg, prec, variant):
         for a, b in zip(run(), want):
             np.testing.assert_array_equal(a, b)
     S.close()
+
+
+@pytest.mark.parametrize("tc", [False, True])
+def test_network_calls_after_one_whose_rows_do_not_fit(pkg, tc):
+    net = pkg.gpu.Network([6, 40, 24, 5])
+    rng = np.random.default_rng(0)
+    net.set_params(rng.normal(0, 0.3, net.n_params).astype(np.float32))
+    net.set_tensor_cores(tc)
+    x = rng.uniform(-1, 1, (64, 6)).astype(np.float32)
+    t = rng.normal(size=(64, 5)).astype(np.float32)
+    y, (g, loss) = net.forward(x), net.gradient(x, t)
+    L, n = pkg.gpu._mlp_lib(), C.c_int64(1 << 38)  # 6 TB of inputs: refused before any array is read
+    f = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))  # noqa: E731
+    assert L.dg_mlp_forward(net.h, f(x), n, f(y.copy())) == 2
+    np.testing.assert_array_equal(net.forward(x), y)
+    assert L.dg_mlp_gradient(net.h, f(x), f(t), n, f(g.copy()), None) == 2
+    again, loss2 = net.gradient(x, t)
+    assert loss2 == loss
+    np.testing.assert_array_equal(again, g)
+    net.set_data(x, t)
+    assert L.dg_mlp_set_data(net.h, f(x), f(t), n) == 2
+    with pytest.raises(pkg.gpu.SolverError, match="DG_ERR_ARG"):  # no training rows any more
+        net.train(1, 16, 1e-3, 1e-3)
+    net.set_data(x, t)
+    assert np.isfinite(net.train(1, 16, 1e-3, 1e-3)).all()
