@@ -206,15 +206,14 @@ def algorithmic_bytes_per_step(E, dofs, dim, w, variant=-1):
     """Algorithmic HBM bytes of one RK4 step's four stage launches: 18 state
     words per DOF (stage 1: u in, accumulator and next input out; stages
     2-3: input, u, accumulator in, accumulator and next input out; stage 4:
-    input, u, accumulator and residual snapshot in, u out), 14 for the FP32
-    Bernstein-basis kernels (variants 64 and up), which keep the stage inputs
-    and no accumulator (2, 3, 3 and 6), plus the element's geometry record and
+    input, u, accumulator and residual snapshot in, u out), plus the element's
+    geometry record (variants 64 and up: the Bernstein-basis kernels' own) and
     integer face record read once per stage."""
     if variant >= 64:
-        words, recf, reci = 14 if w == 4 else 18, bernstein_record_words(dim), 2 * (dim + 1)
+        recf, reci = bernstein_record_words(dim), 2 * (dim + 1)
     else:
-        words, recf, reci = 18, geometry_record_words(dim, w), ((2 * (dim + 1)) + 3) // 4 * 4
-    return words * dofs * w + 4 * E * (recf * w + reci * 4)
+        recf, reci = geometry_record_words(dim, w), ((2 * (dim + 1)) + 3) // 4 * 4
+    return 18 * dofs * w + 4 * E * (recf * w + reci * 4)
 
 
 def measured_peak_gbs():
@@ -409,7 +408,7 @@ def ensemble_summary(args, full=False):
     def alg_bytes(subset):
         d = sum(i["mesh"]["elem_nodes"].size * 3 for i in subset)
         e = sum(i["mesh"]["elem_nodes"].shape[0] for i in subset)
-        return d, 14 * d * 4 + 4 * e * rec_bytes  # (algorithmic_bytes_per_step)
+        return d, 18 * d * 4 + 4 * e * rec_bytes  # (algorithmic_bytes_per_step)
 
     _, all_bytes = alg_bytes(insts)
     # plain path: every 32nd instance on its own, same steps

@@ -221,8 +221,8 @@ int build_fused_graph(dg_batch* b) {
       m.g[k].ntiles = 0;
       if (b->slot_group[k] < 0) continue;
       dg_ctx* c = b->groups[b->slot_group[k]].ctx;
-      const float* in[4] = {(const float*)c->u, (const float*)c->y0, (const float*)c->y1, (const float*)c->acc};
-      float* out[4] = {(float*)c->y0, (float*)c->y1, (float*)c->acc, nullptr};
+      const float* in[4] = {(const float*)c->u, (const float*)c->y0, (const float*)c->y1, (const float*)c->y0};
+      float* out[4] = {(float*)c->y0, (float*)c->y1, (float*)c->y0, nullptr};
       // every instance's own dt sits in its elements' step scale
       m.g[k] = dgc::stage_args_f32(c, st, in[st - 1], out[st - 1], 1.0);
       m.g[k].ntiles = (int)(c->Epad / dgk::stage_multi_elems_per_tile(k + 2));

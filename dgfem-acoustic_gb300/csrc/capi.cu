@@ -304,7 +304,6 @@ dgk::StageArgs<T> stage_args(dg_ctx* c, int stage, const T* y_in, T* y_out, T* k
   a.y_out = y_out;
   a.u = (T*)c->u;
   a.acc = (T*)c->acc;
-  a.y2 = (const T*)c->y0, a.y3 = (const T*)c->y1;
   a.snap = (const T*)c->snap;
   a.k_out = k_out;
   a.partials = c->partials;
@@ -441,10 +440,8 @@ cudaError_t enqueue_step(dg_ctx* c, int kind, double dt, cudaEvent_t* ev, bool c
   const bool pdl = c->bb && !ev, pdl_stage = pdl && c->Epad / 32 <= c->num_sms;
   int nparts = c->variant >= 0 ? c->grid2 : c->grid;
   if (kind == 0) {
-    // no accumulator: its array holds the last stage's input
-    const bool keep = c->bb && c->prec == DG_FP32;
-    const void* in[4] = {c->u, c->y0, c->y1, keep ? c->acc : c->y0};
-    void* out[4] = {c->y0, c->y1, keep ? c->acc : c->y0, nullptr};
+    const void* in[4] = {c->u, c->y0, c->y1, c->y0};
+    void* out[4] = {c->y0, c->y1, c->y0, nullptr};
     for (int s = 0; s < 4; ++s) {
       if (ev) cudaEventRecord(ev[2 * s], c->stream);
       c->pdl = pdl_stage && (s > 0 || (chain && follows));
@@ -973,14 +970,14 @@ int select_variant(dg_ctx* c, int want) {
   float best = 1e30f;
   int best_v = -1;
   // the four stages of an RK step (their operand mixes differ); stage 4
-  // updates another buffer in place of the state, which stays untouched
+  // updates a stage buffer in place of the state, which stays untouched
   auto rk_stages = [&]() {
     cudaError_t err = cudaSuccess;
     for (int st = 1; st <= 3 && err == cudaSuccess; ++st) err = launch_stage(c, st, c->y0, c->y1, nullptr, 1e-30);
     if (err == cudaSuccess) {
       void* u = c->u;
-      c->u = c->kbuf;
-      err = launch_stage(c, 4, c->acc, nullptr, nullptr, 1e-30);
+      c->u = c->y1;
+      err = launch_stage(c, 4, c->y0, nullptr, nullptr, 1e-30);
       c->u = u;
     }
     return err;

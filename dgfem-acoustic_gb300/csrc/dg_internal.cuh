@@ -129,7 +129,6 @@ struct StageArgs {
   T* y_out;        // next stage input (stages 1-3)
   T* u;            // state at step start (updated in stage 4)
   T* acc;          // RK accumulator
-  const T *y2, *y3;  // inputs of stages 2 and 3 (FP32 Bernstein-basis kernels, stage 4)
   const T* snap;   // residual reference (stage 4)
   T* k_out;        // stage 0: dt*L(y_in)
   double* partials;  // [gridDim][5] residual partial sums (stage 4)

@@ -158,7 +158,7 @@ struct BBCfg {
   __host__ __device__ static constexpr int first_word(int tid, int role) { return Q4 ? tid : role * NP * LW + (tid & 31); }
   static constexpr int oGV = NF * (D + 1), oG = oGV + D, oS = oG + D * D, GW = oS + 1;  // geometry words
   static constexpr int GI = 2 * NF;             // neighbour, code
-  static constexpr int CH = sizeof(T) == 8 ? 6 : 7;  // coefficients whose RK operands are in flight together
+  static constexpr int CH = sizeof(T) == 8 ? 6 : P == 4 ? 10 : 7;  // coefficients whose RK operands are in flight together
   static constexpr uint32_t YB = TW * sizeof(T), GB = GW * LW * sizeof(T), IB = GI * LW * 4;
   static constexpr size_t oBar = 0;                                     // NBUF mbarriers
   static constexpr size_t oFm = 64;                                     // int [NF][16]: element word offset of a face node
@@ -395,11 +395,10 @@ struct BBRes {
 // combined with dt*L and stored; in stages 4 and 5 out becomes the residual's
 // difference.
 //
-// FP64 keeps the classical accumulator k1 + 2 k2 + 2 k3. FP32, bound by memory,
-// has none: the inputs of stages 2 to 4 stay, and the step ends with
-//   u + ((y2 - u) + 2 (y3 - u) + (y4 - u)) / 3 + dt k4 / 6,
-// 14 state words moved per step where the accumulator takes 18. The differences
-// are exact to the roundings of y2 .. y4.
+// The accumulator k1 + 2 k2 + 2 k3 has an array of its own. (The stages' inputs
+// hold the same sum, and an FP32 step that forms it from them moves 14 state words
+// in place of 18, but only to the spacing of the state: where a step changes the
+// state by about that, the sum was off by up to two thirds of it.)
 template <class C, class Free>
 struct BBGlobalEnv {
   using T = typename C::T;
@@ -407,16 +406,16 @@ struct BBGlobalEnv {
   // the trace's loads come first: their latency overlaps the volume term
   static constexpr bool kTraceLast = false;
   // FP32: this thread's part of the stage input stays in shared memory until the
-  // update (not with one buffer, which the next tile enters at the barrier)
+  // update, where it is u (not with one buffer, which the next tile enters at the
+  // barrier)
   static constexpr bool OWN = sizeof(T) == 4 && C::NBUF == 2;
   const StageArgs<T>& a;
   int64_t base;      // this thread's first coefficient in the arrays
   const T* own;      // the same in the tile's stage input
   Free free_inputs;  // called by every thread once the stage input is no longer read
-  // FP32: u of all coefficients before the lift, the other operands of stage 4
-  // in groups
+  // FP32: u of all coefficients before the lift, the other operands in groups
   static constexpr int NU = sizeof(T) == 4 ? NP : CH;
-  T x0[NU], x1[CH], x2[CH], x3[CH];
+  T x0[NU], x1[CH], x2[CH];
   __device__ __forceinline__ BBGlobalEnv(const StageArgs<T>& a_, int64_t b, const T* y, Free f)
       : a(a_), base(b), own(OWN ? y : a_.y_in + b), free_inputs(f) {}
   // Values at the neighbour's face nodes: node m has coefficient (w byte m) of
@@ -457,17 +456,23 @@ struct BBGlobalEnv {
     const int stage = a.stage;
     if (stage == 0) return;
     if constexpr (sizeof(T) == 4) {
-      if (stage >= 2 && n0 == 0) {
+      // (stages 1 and 5: the stage input is u)
+      if (n0 == 0 && !(OWN && (stage == 1 || stage == 5))) {
 #pragma unroll
         for (int n = 0; n < NP; ++n) x0[n] = a.u[base + n * SN];
       }
-      if (OWN ? stage >= 4 : stage == 1 || stage == 4) operands(n0, x3, OWN ? a.snap + base : own);
-      if (stage == 4) operands(n0, x1, a.y2 + base), operands(n0, x2, a.y3 + base);
     } else {
       operands(n0, x0, a.u + base);
-      if (stage >= 2 && stage <= 4) operands(n0, x1, a.acc + base);
-      if (stage >= 4) operands(n0, x2, a.snap + base);
     }
+    if (stage >= 2 && stage <= 4) operands(n0, x1, a.acc + base);
+    if (stage >= 4) operands(n0, x2, a.snap + base);
+  }
+  // u of coefficient n0 + i
+  __device__ __forceinline__ T u0(int n0, int i) const {
+    if constexpr (sizeof(T) == 4)
+      return OWN && (a.stage == 1 || a.stage == 5) ? own[(n0 + i) * SN] : x0[n0 + i];
+    else
+      return x0[i];
   }
   __device__ __forceinline__ void update(int n0, T dte, T (&out)[NP]) {
     const int stage = a.stage;
@@ -479,54 +484,32 @@ struct BBGlobalEnv {
         if (n0 + i < NP) ko[(n0 + i) * SN] = dte * out[n0 + i];
       return;
     }
-    if constexpr (sizeof(T) == 4) {
-      if (stage <= 3) {
-        const T c = stage == 3 ? dte : (T)0.5 * dte;
+    T* ac = a.acc + base;
+    if (stage == 1) {
 #pragma unroll
-        for (int i = 0; i < CH; ++i)
-          if (n0 + i < NP)
-            yo[(n0 + i) * SN] = (stage > 1 ? x0[n0 + i] : OWN ? own[(n0 + i) * SN] : x3[i]) + c * out[n0 + i];
-      } else {
-        T* un_ = stage == 4 ? a.u + base : yo;
-        const T* sn = a.snap + base;
-        const T c = dte * (T)(1.0 / 6.0);
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) {
+          ac[(n0 + i) * SN] = dte * out[n0 + i];
+          yo[(n0 + i) * SN] = u0(n0, i) + ((T)0.5 * dte) * out[n0 + i];
+        }
+    } else if (stage <= 3) {
+      const T c = stage == 3 ? dte : (T)0.5 * dte, c2 = (T)2 * dte;
 #pragma unroll
-        for (int i = 0; i < CH; ++i)
-          if (n0 + i < NP) {
-            const T u = x0[n0 + i], y4 = OWN ? own[(n0 + i) * SN] : x3[i];
-            const T un = stage == 4 ? u + (((x1[i] - u) + (y4 - u) + (T)2 * (x2[i] - u)) * (T)(1.0 / 3.0) + c * out[n0 + i])
-                                    : u + dte * out[n0 + i];
-            un_[(n0 + i) * SN] = un;
-            out[n0 + i] = (OWN ? x3[i] : sn[(n0 + i) * SN]) - un;
-          }
-      }
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) {
+          ac[(n0 + i) * SN] = x1[i] + c2 * out[n0 + i];
+          yo[(n0 + i) * SN] = u0(n0, i) + c * out[n0 + i];
+        }
     } else {
-      T* ac = a.acc + base;
-      if (stage == 1) {
+      T* un_ = stage == 4 ? a.u + base : yo;
 #pragma unroll
-        for (int i = 0; i < CH; ++i)
-          if (n0 + i < NP) {
-            ac[(n0 + i) * SN] = dte * out[n0 + i];
-            yo[(n0 + i) * SN] = x0[i] + ((T)0.5 * dte) * out[n0 + i];
-          }
-      } else if (stage <= 3) {
-        const T c = stage == 3 ? dte : (T)0.5 * dte, c2 = (T)2 * dte;
-#pragma unroll
-        for (int i = 0; i < CH; ++i)
-          if (n0 + i < NP) {
-            ac[(n0 + i) * SN] = x1[i] + c2 * out[n0 + i];
-            yo[(n0 + i) * SN] = x0[i] + c * out[n0 + i];
-          }
-      } else {
-        T* un_ = stage == 4 ? a.u + base : yo;
-#pragma unroll
-        for (int i = 0; i < CH; ++i)
-          if (n0 + i < NP) {
-            const T un = stage == 4 ? x0[i] + (x1[i] + dte * out[n0 + i]) * (T)(1.0 / 6.0) : x0[i] + dte * out[n0 + i];
-            un_[(n0 + i) * SN] = un;
-            out[n0 + i] = x2[i] - un;
-          }
-      }
+      for (int i = 0; i < CH; ++i)
+        if (n0 + i < NP) {
+          const T u = u0(n0, i);
+          const T un = stage == 4 ? u + (x1[i] + dte * out[n0 + i]) * (T)(1.0 / 6.0) : u + dte * out[n0 + i];
+          un_[(n0 + i) * SN] = un;
+          out[n0 + i] = x2[i] - un;
+        }
     }
   }
 };
@@ -536,11 +519,7 @@ template <class C, typename T>
 __device__ __forceinline__ void prefetch_operands(const StageArgs<T>& a, int64_t tile) {
   if (a.stage == 0) return;
   if (a.u != a.y_in) prefetch_l2(a.u + tile * C::TW, C::YB);
-  if constexpr (sizeof(T) == 8) {
-    if (a.stage >= 2 && a.stage <= 4) prefetch_l2(a.acc + tile * C::TW, C::YB);
-  } else {
-    if (a.stage == 4) prefetch_l2(a.y2 + tile * C::TW, C::YB), prefetch_l2(a.y3 + tile * C::TW, C::YB);
-  }
+  if (a.stage >= 2 && a.stage <= 4) prefetch_l2(a.acc + tile * C::TW, C::YB);
   if (a.stage >= 4) prefetch_l2(a.snap + tile * C::TW, C::YB);
 }
 
