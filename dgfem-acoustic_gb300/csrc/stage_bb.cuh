@@ -811,12 +811,15 @@ struct FxSum {
 // units of 2^U: the volume term is -elevation(t) (bb_volume without the
 // elevation). bad: an infinity or NaN among the inputs.
 //
-// In fixed point too: the state's coefficients take 57 bits below the largest
-// exponent among those of the element, the metric 58, so that sums of nine
-// products of coefficient differences stay below 2^63. A multiply-add takes an
+// In fixed point too: a variable's coefficients take 57 bits below the largest
+// exponent among its own in the element, a metric column 58, so that sums of nine
+// products of coefficient differences stay below 2^63. (One scale for all three
+// velocity components, and one for the whole metric, let the component along the
+// long sides of a thin element drown the one across it: 4.9e-15 in place of 4e-16
+// in the pressure's right-hand side at 1000 : 1.) A multiply-add takes an
 // SM sub-partition 64 cycles in FP64 and some 10 here, a conversion some 30. us
-// per step: 24,576 tetrahedra of order 3 374 -> 339, 48,000 of order 2 352 -> 310,
-// 48,000 of order 1 155 -> 146, 7,722 of order 2 67 -> 64.
+// per step: 24,576 tetrahedra of order 3 374 -> 327, 48,000 of order 2 352 -> 292,
+// 48,000 of order 1 155 -> 142, 7,722 of order 2 67 -> 62.
 template <class C>
 __device__ __forceinline__ void fx_gradient(const double* y, const double* g, int q, double rhoc2, double inv_rho0,
                                             long long (&t)[bb_np(C::D, C::P - 1)], int& U, bool& bad) {
@@ -854,30 +857,37 @@ __device__ __forceinline__ void fx_gradient(const double* y, const double* g, in
   add(y + q * NP * LW, Ey, G);
 #pragma unroll
   for (int b = 0; b < NB; ++b) t[b] = sum[b].get(), sum[b] = FxSum();
-  // the velocity's divergence, or the pressure's derivative
+  // the velocity's divergence, or the pressure's derivative: every component at
+  // the scale of its own values and of its own metric column
   const int nv = q == 0 ? D : 1;
   const double scale = q == 0 ? rhoc2 : inv_rho0;
   auto metric = [&](int v, int r) { return scale * g[(C::oG + r * D + (q == 0 ? v : q - 1)) * LW]; };
-  int mo = 0;
-  m = 0;
+  const int U1 = fx_unit(Ey, Ev);
+  U = U1;
+  bad = max(Ey, Ev) == 0x7ff;
+  int Eo[3] = {}, Eg[3] = {};
+#pragma unroll
+  for (int v = 0; v < D; ++v)
+    if (v < nv) {
+      m = 0;
+#pragma unroll
+      for (int r = 0; r < D; ++r) m = max(m, fx_size(metric(v, r)));
+      Eo[v] = fx_group(top(y + (q == 0 ? 1 + v : 0) * NP * LW, 0)), Eg[v] = fx_group(m);
+      U = max(U, fx_unit(Eo[v], Eg[v]));
+      bad |= max(Eo[v], Eg[v]) == 0x7ff;
+    }
+#pragma unroll
+  for (int b = 0; b < NB; ++b) t[b] = fx_shift(t[b], U - U1);
 #pragma unroll 1
   for (int v = 0; v < nv; ++v) {
-    mo = top(y + (q == 0 ? 1 + v : 0) * NP * LW, mo);
+    const int eo = v == 0 ? Eo[0] : v == 1 ? Eo[1] : Eo[2], eg = v == 0 ? Eg[0] : v == 1 ? Eg[1] : Eg[2];
+    const int d = U - fx_unit(eo, eg);
 #pragma unroll
-    for (int r = 0; r < D; ++r) m = max(m, fx_size(metric(v, r)));
+    for (int r = 0; r < D; ++r) G[r] = fx_digits<5>(metric(v, r), eg);
+    add(y + (q == 0 ? 1 + v : 0) * NP * LW, eo, G);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) t[b] += fx_shift(sum[b].get(), d), sum[b] = FxSum();
   }
-  const int Eo = fx_group(mo), Eg = fx_group(m);
-#pragma unroll 1
-  for (int v = 0; v < nv; ++v) {
-#pragma unroll
-    for (int r = 0; r < D; ++r) G[r] = fx_digits<5>(metric(v, r), Eg);
-    add(y + (q == 0 ? 1 + v : 0) * NP * LW, Eo, G);
-  }
-  const int U1 = fx_unit(Ey, Ev), U2 = fx_unit(Eo, Eg);
-  U = max(U1, U2);
-  bad = max(max(Ey, Ev), max(Eo, Eg)) == 0x7ff;
-#pragma unroll
-  for (int b = 0; b < NB; ++b) t[b] = fx_shift(t[b], U - U1) + fx_shift(sum[b].get(), U - U2);
 }
 
 // One tile of an FP64 state (see above): bb_tile with fluxes and gradient in
