@@ -25,10 +25,10 @@ cudaError_t bb_cell_means(dg_ctx* c, double* out, bool soa);
 // Many RK4 steps in one launch (persist.cu). Whether the context is in FP64 and
 // its tiles fit on the GPU at once; device lists and buffers of a run (false where memory for them is
 // short); n_steps steps on c->stream with residuals and observers to the
-// context's result buffers; release.
+// context's result buffers (launched: steps whose launch succeeded); release.
 bool persist_fits(const dg_ctx* c);
 bool persist_ready(dg_ctx* c);
-cudaError_t persist_run(dg_ctx* c, int64_t n_steps, double dt);
+cudaError_t persist_run(dg_ctx* c, int64_t n_steps, double dt, int64_t* launched);
 void persist_free(dg_ctx* c);
 dgk::StageArgs<double> stage_args_f64(dg_ctx* c, int stage, const double* y_in, double* y_out, double dt);
 }  // namespace dgc

@@ -535,9 +535,18 @@ int run_steps(dg_ctx* c, int kind, int64_t n_steps, double dt, double* residuals
   // a single step in the many-steps kernel takes up to 12 us more than its graph,
   // each further one 5 to 20 us less (3-D order 2, 1,080 elements: 92 against 81
   // us for one, 525 against 576 for ten)
+  bool graphs = true;
   if (kind == 0 && n_steps >= 4 && dgk::is_persist_variant(c->variant) && dgc::persist_ready(c)) {
-    CK(c, dgc::persist_run(c, n_steps, dt));
-  } else {
+    int64_t done = 0;
+    const cudaError_t e = dgc::persist_run(c, n_steps, dt, &done);
+    // a process with a share of the SMs only may not start it: the graphs then
+    graphs = e == cudaErrorCooperativeLaunchTooLarge && done == 0;
+    if (graphs)
+      cudaGetLastError();
+    else
+      CK(c, e);
+  }
+  if (graphs) {
     const int64_t many = n_steps / kGraphSteps, rest = n_steps % kGraphSteps;
     if (many > 0) rc = build_graph(c, kind, dt, kGraphSteps);
     if (!rc && rest > 0) rc = build_graph(c, kind, dt, 1);

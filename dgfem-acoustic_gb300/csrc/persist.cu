@@ -162,7 +162,7 @@ bool persist_ready(dg_ctx* c) {
   return true;
 }
 
-cudaError_t persist_run(dg_ctx* c, int64_t n_steps, double dt) {
+cudaError_t persist_run(dg_ctx* c, int64_t n_steps, double dt, int64_t* launched) {
   dg_ctx::Persist& d = c->persist;
   const int nt = (int)(c->Epad / 32);
   const int64_t words = (int64_t)nt * c->nv * c->np * 32;
@@ -189,6 +189,7 @@ cudaError_t persist_run(dg_ctx* c, int64_t n_steps, double dt) {
     d.seq += 4 * (uint32_t)p.steps;
     if (e == cudaSuccess) e = dgk::launch_persist(c->dim, c->order, p, nt, c->d_err, c->stream);
     if (e != cudaSuccess) return e;
+    *launched = done + p.steps;
     dgk::k_persist_sums<<<dim3(p.steps, 1 + c->n_obs), dgk::kSumThreads, 0, c->stream>>>(
         d.partials, nt, c->nv, inv_count, c->c0sq, c->d_res + done * 5, d.gsum, d.groups, d.obs_first, d.obs_grp,
         d.obs_w, c->d_obs + done * c->n_obs * 4, c->n_obs);
