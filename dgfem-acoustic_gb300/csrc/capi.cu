@@ -569,7 +569,7 @@ int run_steps(dg_ctx* c, int kind, int64_t n_steps, double dt, double* residuals
     // flag is cleared so that the context stays usable
     CK(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    return fail(c, DG_ERR_TIMEOUT, "a bounded device wait gave up (TMA copy did not complete)");
+    return fail(c, DG_ERR_TIMEOUT, "a bounded device wait gave up (a copy, tensor-core work or a neighbouring tile did not arrive)");
   }
   for (double v : res)
     if (!std::isfinite(v)) return fail(c, DG_ERR_NONFINITE, "non-finite values in the state (residual is NaN/Inf)");

@@ -377,7 +377,7 @@ struct dg_mlp {
   unsigned* ticket = nullptr;
   int num_sms = 0;
   int tc = 0;             // GEMMs on the tensor cores (k_gemm_tc), else k_gemm
-  int* d_err = nullptr;   // set by a tensor-core GEMM whose wait gave up
+  int* d_err = nullptr;   // set by a pass whose wait for weights or a GEMM whose wait for its MMAs gave up
   std::string err;
 };
 
@@ -462,7 +462,7 @@ int gemm(dg_mlp* m, int M, int N, int K, const float* A, int64_t sam, int64_t sa
 }
 
 // After a stream synchronisation: DG_ERR_TIMEOUT (and the flag cleared) when
-// a tensor-core GEMM gave up waiting for its MMAs.
+// a fused pass or a tensor-core GEMM gave up waiting.
 int check_gemm_waits(dg_mlp* m) {
   int h = 0;
   MCK(m, cudaMemcpyAsync(&h, m->d_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
@@ -470,7 +470,7 @@ int check_gemm_waits(dg_mlp* m) {
   if (h == 0) return DG_OK;
   MCK(m, cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream));
   MCK(m, cudaStreamSynchronize(m->stream));
-  return fail(m, DG_ERR_TIMEOUT, "dg_mlp: a tensor-core GEMM timed out waiting for its MMAs");
+  return fail(m, DG_ERR_TIMEOUT, "dg_mlp: a bounded device wait gave up (weights of a fused pass, or a GEMM's MMAs)");
 }
 
 constexpr size_t mlpf_max_smem = 227 * 1024;

@@ -1,7 +1,7 @@
-// Fused passes of the surrogate network (mlp.cu) on the CUDA cores: the whole
-// forward pass in one launch, the whole chain of input gradients in one, all
-// weight and bias gradients and the loss in one, and the optimiser step with
-// the refresh of every weight copy in one.
+// Fused passes of the surrogate network (mlp.cu), products on mma.sync with FP32
+// activations split into three BF16 values: the whole forward pass in one launch,
+// the whole chain of input gradients in one, all weight and bias gradients and the
+// loss in one, and the optimiser step with the refresh of every weight copy in one.
 //
 // A block takes R rows of the batch through every layer with the
 // activations in shared memory; the layers' BF16 weights, laid out in the
