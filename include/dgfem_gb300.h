@@ -38,7 +38,8 @@
  * stream and all its device memory; a context is not thread-safe, distinct
  * contexts may be used concurrently. Device memory is allocated in dg_create,
  * dg_set_sources, dg_set_observers and on the first dg_run that needs more
- * per-step output room.
+ * per-step output room, or (kernel_variant 80 and up) lists of sources and
+ * observers that have changed.
  */
 #ifndef DGFEM_GB300_H
 #define DGFEM_GB300_H
@@ -103,6 +104,17 @@ int dg_destroy(dg_ctx* ctx);
 const char* dg_last_error(const dg_ctx* ctx);
 int dg_get_info(const dg_ctx* ctx, dg_info_t* info);
 
+/* The state in the reference layout. The Bernstein-basis kernels (kernel_variant
+ * 64 and up in dg_get_info, the default on straight-sided triangles and
+ * tetrahedra) hold it as Bernstein coefficients in the context's precision: what
+ * dg_get_state returns after dg_set_state differs from what was set by up to m
+ * roundings of the largest value of that variable in the element, m = 1, 3, 10, 35
+ * at orders 1 to 4 (23 in 2-D at order 4; smooth states about one), where the other
+ * kernels return it as set (FP64) or rounded to FP32. So does a run that is resumed
+ * from a saved state differ from one in one piece, and the overwrite of source
+ * nodes holds to such roundings, which it also leaves on the element's other nodes.
+ * An infinity or NaN at a node spreads to other nodes of the element. In FP64
+ * these kernels take values below 2^-1011 of a flux or derivative as zero. */
 int dg_set_state(dg_ctx* ctx, const double* u);
 int dg_get_state(dg_ctx* ctx, double* u);
 
@@ -175,9 +187,11 @@ int dg_vtu_writer_stats(const dg_vtu_writer* w, int64_t* files_written, int* com
  * coefficients: a change to or from them converts state and snapshot, to
  * rounding; 80 + k: variant 64 + k, with dg_run calls of four or more steps in
  * one cooperative launch per 64 steps (FP64 contexts whose tiles of 32 elements
- * all fit on the GPU at once; there what a selection by timing ends with).
- * Returns
- * DG_ERR_ARG for a variant that does not exist for this element type or
+ * all fit on the GPU at once; there what a selection ends with, without timing it;
+ * such a launch starts when all its tiles' SMs are free, so beside other streams'
+ * long kernels 64 + k can be the better choice). On straight-sided triangles and
+ * tetrahedra the variants below 64 run only when they are asked for by number.
+ * Returns DG_ERR_ARG for a variant that does not exist for this element type or
  * precision. */
 int dg_tune(dg_ctx* ctx, int variant);
 
