@@ -1236,10 +1236,7 @@ int dgc::create_ctx(const dg_mesh_desc* mesh, const dg_phys* phys, int precision
   if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_perm, c->np * sizeof(int));
   if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_perm, c->perm_c2i.data(), c->np * sizeof(int), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = dgc::dev_alloc(c, (void**)&c->d_ref, 4 * c->E * c->np * sizeof(double));
-  // what a stage leaves in L2 is worth turning round for (stage_bb.cuh)
-  int l2 = 0;
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device);
-  c->turns = precision == DG_FP32 && (int64_t)c->nv * c->Epad * c->np * 4 <= l2;
+  c->turns = precision == DG_FP32;  // (stage_bb.cuh)
   c->max_grid = std::max(c->grid, 2 * c->num_sms);
   for (int v = 0; v < 8; ++v) {
     dgk::Stage2Info si = stage2_info(c, v);

@@ -1281,10 +1281,11 @@ __global__ void __launch_bounds__(BBCfg<T, D, P, NBUF, MINB>::NT, MINB) stage_bb
     fence_mbar_init();
   }
   // Alternate stages may go through the tiles in opposite directions, so that what
-  // the stage before touched last is still in L2. For FP32 states of up to an L2:
-  // 196,608 tetrahedra of order 3 (63 MB) 284 -> 275 us per step, 614,400 triangles
-  // of order 2 (44 MB) 168 -> 166; 254,016 tetrahedra of order 4 (142 MB) 703 ->
-  // 709, and FP64 kernels, which do not wait for memory, 0.5 % slower.
+  // the stage before touched last is still in L2. FP32 kernels do, us per step:
+  // 196,608 tetrahedra of order 3 (a state of 63 MB) 294 -> 280, 614,400 triangles
+  // of order 2 (44 MB) 174 -> 163, 254,016 tetrahedra of order 4 (142 MB) 698 -> 683,
+  // 889,056 (498 MB) 2662 -> 2642; 196,608 of order 1, all of whose arrays fit in L2,
+  // 77.3 -> 78.4. FP64 kernels, which do not wait for memory, were 0.5 % slower.
   auto tile_at = [&](int i) { return a.reverse ? a.ntiles - 1 - i : i; };
   // what no kernel before this one writes is fetched while they drain
   if (tid == 0 && (int)blockIdx.x < a.ntiles) issue_geometry(tile_at(blockIdx.x), 0);
