@@ -917,7 +917,7 @@ void tune_cache_store(const std::string& key, int v) {
 }
 
 // Where all tiles of an FP64 mesh fit on the GPU at once, runs take the many-steps
-// kernel, which was the faster one on every such mesh (1.06 to 1.45 times, see
+// kernel, which was the faster one on every such mesh (1.05 to 1.45 times, see
 // stage_persist.cuh), and only the other launches the Bernstein-basis kernel
 // selected.
 void take_persistent(dg_ctx* c) {

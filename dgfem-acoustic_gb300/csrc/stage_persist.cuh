@@ -26,8 +26,8 @@
 // FP64, us per step with one launch per stage -> here, up to one tile per SM and
 // at the resident limit: 2-D order 1 21 -> 14, 64 -> 53 (8 tiles per SM); order 2
 // 30 -> 22, 68 -> 50 (5); order 3 42 -> 33, 97 -> 79 (5); order 4 58 -> 47, 114 ->
-// 99 (4); 3-D order 1 32 -> 25, 89 -> 68 (5); order 2 56 -> 49, 111 -> 91 (3);
-// order 3 104 -> 97, 151 -> 131 (2).
+// 99 (4); 3-D order 1 34 -> 24, 83 -> 62 (5); order 2 55 -> 49, 97 -> 88 (3);
+// order 3 100 -> 95 (1).
 #pragma once
 #include <cstdint>
 
@@ -320,7 +320,7 @@ struct StagePersist {
       cudaGetLastError();
       return 0;
     }
-    return nb;
+    return nb < MINB ? nb : MINB;
   }
   static cudaError_t launch(const PersistArgs& p, int grid, int* err, cudaStream_t s) {
     void* args[2] = {const_cast<PersistArgs*>(&p), &err};
