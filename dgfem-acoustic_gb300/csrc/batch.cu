@@ -453,8 +453,8 @@ int dg_batch_create(int n, const dg_mesh_desc* meshes, const dg_phys* phys, cons
   // One launch per stage only by choice (DGFEM_BATCH_FUSED=1 or
   // dg_batch_set_fused(b, 1)): it runs every order at the registers and shared
   // memory of the largest, and all orders wait for one another at every stage.
-  // us per step, one launch -> branches: 2 instances (0.12M unknowns) 39 -> 17,
-  // 16 (2.3M) 102 -> 38, 48 (28M) 450 -> 309.
+  // us per step, one launch -> branches: 2 instances (0.12M unknowns) 39 -> 18,
+  // 16 (2.3M) 100 -> 40, 48 (28M) 450 -> 353.
   const char* ev = std::getenv("DGFEM_BATCH_FUSED");
   b->fused = b->fused_ok && ev && std::strcmp(ev, "1") == 0;
   if (group_layouts(b) != DG_OK) return bail(DG_ERR_CUDA, b->err);

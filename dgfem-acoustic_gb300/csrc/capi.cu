@@ -532,9 +532,9 @@ int run_steps(dg_ctx* c, int kind, int64_t n_steps, double dt, double* residuals
   if (n_steps == 0) return DG_OK;
   int rc = ensure_out_cap(c, n_steps);
   if (rc) return rc;
-  // a single step in the many-steps kernel takes up to 12 us more than its graph,
-  // each further one 5 to 20 us less (3-D order 2, 1,080 elements: 92 against 81
-  // us for one, 525 against 576 for ten)
+  // a single step in the many-steps kernel takes as long as its graph or up to 2 us
+  // more, each further one 2 to 20 us less (3-D order 2, 1,080 elements: 81 against
+  // 82 us for one, 513 against 553 for ten)
   bool graphs = true;
   if (kind == 0 && n_steps >= 4 && dgk::is_persist_variant(c->variant) && dgc::persist_ready(c)) {
     int64_t done = 0;
@@ -917,7 +917,7 @@ void tune_cache_store(const std::string& key, int v) {
 }
 
 // Where all tiles of an FP64 mesh fit on the GPU at once, runs take the many-steps
-// kernel, which was the faster one on every such mesh (1.05 to 1.45 times, see
+// kernel, which was the faster one on every such mesh (1.05 to 1.5 times, see
 // stage_persist.cuh), and only the other launches the Bernstein-basis kernel
 // selected.
 void take_persistent(dg_ctx* c) {
@@ -955,8 +955,8 @@ int select_variant(dg_ctx* c, int want) {
   if (bb_mesh(c)) {
     // on straight-sided triangles and tetrahedra the Bernstein-basis kernels
     // were the fastest at every order and precision (196,608 tetrahedra of
-    // order 3, FP32: 0.27 ms per step against 0.61 for the best other; 24,576
-    // in FP64: 0.34 against 2.24), so only they are timed
+    // order 3, FP32: 0.28 ms per step against 0.61 for the best other; 24,576
+    // in FP64: 0.33 against 2.24), so only they are timed
     offer(dgk::kBBVariant, 16, true);
   } else {
     cands.push_back(-1);

@@ -13,8 +13,9 @@
 // run the fused passes of mlp_fused.cuh: one launch for the forward pass, one for
 // the chain of input gradients, one for all weight gradients and the loss, one for
 // the optimiser step with every weight copy. Measured against one GEMM per layer (GB300, the
-// 6-256-256-256-256-512 network): forward of 2000 rows on the device 95 -> 29
-// us, a training step of 256 rows 680 -> 79 us.
+// 6-256-256-256-256-512 network): forward of 2000 rows on the device, one pass
+// after another, 95 -> 27 us (30 with L2 flushed; passes of several networks on
+// their own streams overlap, 19 each), a training step of 256 rows 680 -> 64 us.
 // Other networks, and dg_mlp_set_tensor_cores, use per-layer kernels: one GEMM
 // serves the three products of a layer, Z = X W^T (forward), dX = dZ W (input
 // gradient) and dW = dZ^T X (weight gradient), on the CUDA cores (k_gemm: 64 x
@@ -490,7 +491,8 @@ bool pass_fits(int ka, int kb, bool bwd) {
 // with the least time over its waves of tiles. A wave of the surrogate's tiles
 // takes 13, 22 and 38 us (8, 16 and 32 rows: the latency of the weight stream's
 // chunks, then the matrix instructions); 2000 rows: 31, 27 and 41 us in all,
-// 3648: 43, 48 and 41, 20,000: 228, 203 and 193.
+// 3648: 43, 48 and 41, 20,000: 228, 203 and 193. (Networks of other widths are
+// weighed with the same ratios, which were not measured for them.)
 int pick_groups(const dg_mlp* m, int64_t n, int ka, int kb, bool bwd) {
   int best = 1;
   double best_cost = 1e300;

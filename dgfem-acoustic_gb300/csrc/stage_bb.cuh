@@ -25,9 +25,9 @@
 // the memory floor. FP64 runs at 2 operations per clock and SM on GB300 and
 // bounds its stages by their count, which the fixed-point sums (bb_tile_fx,
 // fx_gradient) quarter. Measured per RK4 step against the nodal kernels' best:
-// 196,608 tetrahedra of order 3, FP32, 0.61 -> 0.27 ms (floor 0.15); 131,712 of
-// order 4, FP32, 0.61 -> 0.34 (0.17); 24,576 of order 3, FP64, 2.24 -> 0.34
-// (0.05); 125,000 triangles of order 4, FP32, 0.14 -> 0.085 (0.054).
+// 196,608 tetrahedra of order 3, FP32, 0.61 -> 0.28 ms (floor 0.19); 131,712 of
+// order 4, FP32, 0.61 -> 0.36 (0.21); 24,576 of order 3, FP64, 2.24 -> 0.33
+// (0.05); 125,000 triangles of order 4, FP32, 0.14 -> 0.083 (0.067).
 //
 // Layout: arrays of tiles of 32 elements, [tile][variable][coefficient][32]:
 // a warp's lanes are the tile's elements, every load and store of a
@@ -150,8 +150,8 @@ struct BBCfg {
   // [tile][coefficient][32][4], else one plane each, [tile][variable][coefficient][32]
   static constexpr bool Q4 = sizeof(T) == 4 && D == 3;
   // packed FP32 arithmetic for two variables in the fluxes and two metric columns
-  // in the volume term: 131,712 tetrahedra of order 4 361 -> 344 us per step, whose
-  // instructions bound them; at order 3 its register pairs cost more (271 -> 276)
+  // in the volume term: 131,712 tetrahedra of order 4 373 -> 360 us per step; at
+  // order 3 its register pairs cost more (1.8 %)
   static constexpr bool PACK2 = Q4 && P == 4;
   static constexpr int SQ = Q4 ? 1 : NP * LW, SN = Q4 ? 4 * LW : LW, SE = Q4 ? 4 : 1;  // word strides
   // word in the tile of the first coefficient that a thread owns in the update

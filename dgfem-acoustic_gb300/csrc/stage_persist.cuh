@@ -24,9 +24,9 @@
 // by one launch after the steps (k_persist_sums).
 //
 // FP64, us per step with one launch per stage -> here, up to one tile per SM and
-// at the resident limit: 2-D order 1 21 -> 14, 64 -> 53 (8 tiles per SM); order 2
-// 30 -> 22, 68 -> 50 (5); order 3 42 -> 33, 97 -> 79 (5); order 4 58 -> 47, 114 ->
-// 99 (4); 3-D order 1 34 -> 24, 83 -> 62 (5); order 2 55 -> 49, 97 -> 88 (3);
+// at the resident limit: 2-D order 1 20 -> 14, 64 -> 53 (8 tiles per SM); order 2
+// 29 -> 22, 67 -> 50 (5); order 3 41 -> 33, 96 -> 76 (5); order 4 57 -> 47, 116 ->
+// 98 (4); 3-D order 1 34 -> 24, 83 -> 62 (5); order 2 55 -> 49, 97 -> 88 (3);
 // order 3 100 -> 95 (1).
 #pragma once
 #include <cstdint>
