@@ -23,10 +23,11 @@ cudaError_t bb_inject(dg_ctx* c);
 // Element means into out: AoS [E][5] (p, rho, v) or SoA (p [E], rho [E], v [E][3]).
 cudaError_t bb_cell_means(dg_ctx* c, double* out, bool soa);
 // Many RK4 steps in one launch (persist.cu). Whether the context is in FP64 and
-// its tiles fit on the GPU at once; device lists and buffers of a run (false where memory for them is
+// its tiles fit on the GPU at once; whether it is the faster way then; device lists and buffers of a run (false where memory for them is
 // short); n_steps steps on c->stream with residuals and observers to the
 // context's result buffers (launched: steps whose launch succeeded); release.
 bool persist_fits(const dg_ctx* c);
+bool persist_pays(const dg_ctx* c);
 bool persist_ready(dg_ctx* c);
 cudaError_t persist_run(dg_ctx* c, int64_t n_steps, double dt, int64_t* launched);
 void persist_free(dg_ctx* c);

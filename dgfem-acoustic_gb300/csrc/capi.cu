@@ -536,7 +536,7 @@ int run_steps(dg_ctx* c, int kind, int64_t n_steps, double dt, double* residuals
   // more, each further one 2 to 20 us less (3-D order 2, 1,080 elements: 81 against
   // 82 us for one, 513 against 553 for ten)
   bool graphs = true;
-  if (kind == 0 && n_steps >= 4 && dgk::is_persist_variant(c->variant) && dgc::persist_ready(c)) {
+  if (kind == 0 && n_steps >= 4 && dgk::is_persist_variant(c->variant) && dgc::persist_pays(c) && dgc::persist_ready(c)) {
     int64_t done = 0;
     const cudaError_t e = dgc::persist_run(c, n_steps, dt, &done);
     // a process with a share of the SMs only may not start it: the graphs then
@@ -917,7 +917,7 @@ void tune_cache_store(const std::string& key, int v) {
 }
 
 // Where all tiles of an FP64 mesh fit on the GPU at once, runs take the many-steps
-// kernel, which was the faster one on every such mesh (1.05 to 1.5 times, see
+// kernel where it is the faster one (1.05 to 1.5 times, persist_pays; see
 // stage_persist.cuh), and only the other launches the Bernstein-basis kernel
 // selected.
 void take_persistent(dg_ctx* c) {

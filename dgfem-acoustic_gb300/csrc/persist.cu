@@ -61,6 +61,11 @@ bool persist_fits(const dg_ctx* c) {
   return c->prec == DG_FP64 && c->Epad / 32 <= (int64_t)dgk::persist_info(c->dim, c->order).blocks_per_sm * c->num_sms;
 }
 
+// At order 3 in 3-D the two tiles that an SM holds hold each other up. us per step
+// against one launch per stage: 95 / 100 up to a tile per SM, 118 / 124 at 1.1, 129 /
+// 125 at 1.2, 144 / 127 at 1.5, 166 / 128 at 1.8. The others pay at every size.
+bool persist_pays(const dg_ctx* c) { return !(c->dim == 3 && c->order == 3) || c->Epad / 32 <= c->num_sms; }
+
 namespace {
 
 void free_lists(dg_ctx* c) {

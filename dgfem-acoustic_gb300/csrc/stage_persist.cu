@@ -3,15 +3,12 @@
 
 namespace dgk {
 
-// per (dim, order): blocks per SM that the register budget allows for and that are
-// used. 3-D, order 3, takes one although two are resident: beyond a tile per SM the
-// tiles that share one hold each other up (1.5 tiles per SM 144 us per step against
-// 127 with one launch per stage, 1.8 tiles 166 against 128; up to one 95 against
-// 100). 3-D, order 4: 191 us per step against 190, on any number of tiles that fit;
-// not built.
+// per (dim, order): blocks per SM that the register budget allows for. (3-D, order
+// 4: 191 us per step against 190 with one launch per stage, on any number of
+// tiles that fit; not built.)
 #define DGK_PERSIST(X) \
   X(2, 1, 8) X(2, 2, 6) X(2, 3, 5) X(2, 4, 4) \
-  X(3, 1, 5) X(3, 2, 3) X(3, 3, 1)
+  X(3, 1, 5) X(3, 2, 3) X(3, 3, 2)
 
 cudaError_t launch_persist(int dim, int order, const PersistArgs& p, int grid, int* err, cudaStream_t s) {
 #define DGK_P_LAUNCH(DD, PP, MB) \

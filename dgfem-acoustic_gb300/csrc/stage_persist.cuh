@@ -27,7 +27,7 @@
 // at the resident limit: 2-D order 1 20 -> 14, 64 -> 53 (8 tiles per SM); order 2
 // 29 -> 22, 67 -> 50 (5); order 3 41 -> 33, 96 -> 76 (5); order 4 57 -> 47, 116 ->
 // 98 (4); 3-D order 1 34 -> 24, 83 -> 62 (5); order 2 55 -> 49, 97 -> 88 (3);
-// order 3 100 -> 95 (1).
+// order 3 100 -> 95, and beyond one tile per SM slower, 128 -> 166 (persist_pays).
 #pragma once
 #include <cstdint>
 
@@ -320,7 +320,7 @@ struct StagePersist {
       cudaGetLastError();
       return 0;
     }
-    return nb < MINB ? nb : MINB;
+    return nb;
   }
   static cudaError_t launch(const PersistArgs& p, int grid, int* err, cudaStream_t s) {
     void* args[2] = {const_cast<PersistArgs*>(&p), &err};

@@ -188,6 +188,7 @@ int dg_vtu_writer_stats(const dg_vtu_writer* w, int64_t* files_written, int* com
  * rounding; 80 + k: variant 64 + k, with dg_run calls of four or more steps in
  * one cooperative launch per 64 steps (FP64 contexts whose tiles of 32 elements
  * all fit on the GPU at once; there what a selection ends with, without timing it;
+ * at order 3 in 3-D with more tiles than SMs dg_run keeps 64 + k's launches;
  * such a launch starts when all its tiles' SMs are free, so beside other streams'
  * long kernels 64 + k can be the better choice). On straight-sided triangles and
  * tetrahedra the variants below 64 run only when they are asked for by number.
